@@ -10,6 +10,7 @@
 // between calls (grow-only, per device) instead of allocating and freeing
 // every buffer on every call.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -378,6 +379,59 @@ PbStatus pb_dose_adjoint_ordered(const PbGrid *grid, const PbBeam *beams, int n_
                           order_dev);
 }
 
+PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                       const float *spot_boxes, int *forward_out, int *adjoint_out)
+{
+    PbStatus s = check_grid(grid);
+    if (s != PB_OK) return s;
+    if (!beams || n_beams <= 0 || n_beams > PB_MAX_BEAMS || !spot_boxes || !forward_out ||
+        !adjoint_out)
+        return set_error(PB_ERR_INVALID, "NULL argument or beam count");
+    tile_split(*grid, beams, n_beams, spot_boxes, forward_out, adjoint_out);
+    return PB_OK;
+}
+
+static PbStatus check_split(const PbGrid &g, int split)
+{
+    if (split != 1 && split != 2 && split != 4)
+        return set_error(PB_ERR_INVALID, "split must be 1, 2 or 4");
+    if (tile_order_count(g) * split > INT_MAX)
+        return set_error(PB_ERR_INVALID, "too many tiles to split");
+    return PB_OK;
+}
+
+PbStatus pb_dose_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                       const float *wet_dev, const PbLayer *layers_dev,
+                       const float *spot_geo_dev, const float *mu_dev, float scale,
+                       float *dose_dev, const int *order_dev, int split, void *stream)
+{
+    PbStatus s = check_beams(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev);
+    if (s == PB_OK) s = check_split(*grid, split);
+    if (s != PB_OK) return s;
+    if (!dose_dev) return set_error(PB_ERR_INVALID, "dose is NULL");
+    if (!mu_dev) {
+        for (int b = 0; b < n_beams; ++b)
+            if (beams[b].n_layers) return set_error(PB_ERR_INVALID, "mu is NULL");
+    }
+    return launch_dose(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev, mu_dev, scale,
+                       dose_dev, nullptr, static_cast<cudaStream_t>(stream), -1, order_dev,
+                       split);
+}
+
+PbStatus pb_dose_adjoint_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                               const float *wet_dev, const PbLayer *layers_dev,
+                               const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
+                               float *grad_dev, const int *order_dev, int split, void *stream)
+{
+    PbStatus s = check_beams(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev);
+    if (s == PB_OK) s = check_split(*grid, split);
+    if (s != PB_OK) return s;
+    if (!dobj_dose_dev || !grad_dev) return set_error(PB_ERR_INVALID, "NULL argument");
+    return launch_adjoint(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev,
+                          dobj_dose_dev, scale, grad_dev, static_cast<cudaStream_t>(stream), -1,
+                          order_dev, split);
+}
+
 PbStatus pb_dose_adjoint(const PbGrid *grid, const PbBeam *beams, int n_beams,
                          const float *wet_dev, const PbLayer *layers_dev,
                          const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
@@ -717,6 +771,16 @@ PbStatus pb_proton_spot_host(int gpu_id, double vsadx, double vsady, const float
         B.dvp_len = dvp_len;
         PB_TRY(launch_layer_bounds(&B, 1, static_cast<PbLayer *>(D.buf[kBufLayers].p),
                                    static_cast<const float *>(D.buf[kBufGeo].p), st));
+        // how many blocks share a tile (pb_tile_split)
+        float box[4] = {INFINITY, -INFINITY, INFINITY, -INFINITY};
+        for (int i = 0; i < n_spots; ++i) {
+            box[0] = std::min(box[0], spots[i].x);
+            box[1] = std::max(box[1], spots[i].x);
+            box[2] = std::min(box[2], spots[i].y);
+            box[3] = std::max(box[3], spots[i].y);
+        }
+        int split = 1, split_adj = 1;
+        tile_split(g, &B, 1, box, &split, &split_adj);
         // the tiles in the order of their estimated work (pb_tile_order)
         PB_TRY(launch_tile_order(g, &B, 1, static_cast<const float *>(D.buf[kBufWet].p),
                                  static_cast<const PbLayer *>(D.buf[kBufLayers].p),
@@ -726,7 +790,7 @@ PbStatus pb_proton_spot_host(int gpu_id, double vsadx, double vsady, const float
                            static_cast<const PbLayer *>(D.buf[kBufLayers].p),
                            static_cast<const float *>(D.buf[kBufGeo].p),
                            static_cast<const float *>(D.buf[kBufMu].p), 1.0f, d_dose, nullptr,
-                           st, -1, static_cast<const int *>(D.buf[kBufOrder].p)));
+                           st, -1, static_cast<const int *>(D.buf[kBufOrder].p), split));
     }
     PB_TRY(check_cuda(cudaMemcpyAsync(dose_out, d_dose, vb, cudaMemcpyDeviceToHost, st),
                       "D2H dose"));

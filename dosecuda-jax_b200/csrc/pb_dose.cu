@@ -141,30 +141,76 @@ __device__ __forceinline__ LayerK layer_consts(float r80, const float *cabc, con
 // Every operation is an explicitly rounded intrinsic, so that no
 // instantiation of the tile code contracts them differently: all kernel
 // shapes give the same bits.
-template <class Row>
-__device__ __forceinline__ void layer_params(float wet_mm, float dist, const LayerK &K,
-                                             const Row &s_dep, const Row &s_sig,
-                                             const Row &s_idd, int lut_len, float &pf,
-                                             float &hf, float &ps2, float &hs2)
+// A depth's place in a LUT row: the guessed bracket's entries lo - 1 and lo
+// (clamped to the row), loaded without a branch so that the loads of several
+// voxels are in flight together.
+struct LutAt {
+    int lo;                      // guessed first row with depth >= wet_mm
+    float da, db, sa, sb, ia, ib;
+};
+
+// The first row whose depth is >= wet_mm, guessed from the first depth and the
+// first step.
+__device__ __forceinline__ int lut_guess(float wet_mm, const LayerK &K, int lut_len)
 {
     const float gs = ceilf(__fmul_rn(__fsub_rn(wet_mm, K.d0), K.inv_step));
-    int lo = gs > 0.0f ? (gs < (float)lut_len ? (int)gs : lut_len) : 0;
-    if (wet_mm != wet_mm) lo = lut_len;   // NaN compares false: the search ends high
-    while (lo > 0 && s_dep[lo - 1] >= wet_mm) --lo;
-    while (lo < lut_len && s_dep[lo] < wet_mm) ++lo;
-    float idd, sms;
-    if (lo == lut_len) {
-        idd = s_idd[lo - 1];
-        sms = s_sig[lo - 1];
-    } else if (lo == 0) {
-        idd = s_idd[0];
-        sms = s_sig[0];
-    } else {
-        const float f = __fdividef(__fsub_rn(wet_mm, s_dep[lo - 1]),
-                                   __fsub_rn(s_dep[lo], s_dep[lo - 1]));
-        idd = __fmaf_rn(__fsub_rn(s_idd[lo], s_idd[lo - 1]), f, s_idd[lo - 1]);
-        sms = __fmaf_rn(__fsub_rn(s_sig[lo], s_sig[lo - 1]), f, s_sig[lo - 1]);
+    return gs > 0.0f ? (gs < (float)lut_len ? (int)gs : lut_len) : 0;
+}
+
+template <class Row>
+__device__ __forceinline__ LutAt lut_load(float wet_mm, const LayerK &K, const Row &s_dep,
+                                          const Row &s_sig, const Row &s_idd, int lut_len)
+{
+    LutAt L;
+    L.lo = lut_guess(wet_mm, K, lut_len);
+    if (wet_mm != wet_mm) L.lo = lut_len;   // NaN compares false: the search ends high
+    const int a = max(L.lo - 1, 0), b = min(L.lo, lut_len - 1);
+    L.da = s_dep[a];
+    L.db = s_dep[b];
+    L.sa = s_sig[a];
+    L.sb = s_sig[b];
+    L.ia = s_idd[a];
+    L.ib = s_idd[b];
+    return L;
+}
+
+// The row's IDD and sigma at wet_mm.  A guess that is not the lower-bound row
+// (a table without a uniform step) is moved until it is, as lut_load's caller
+// would have searched it.
+template <class Row>
+__device__ __forceinline__ void lut_eval(LutAt L, float wet_mm, const Row &s_dep,
+                                         const Row &s_sig, const Row &s_idd, int lut_len,
+                                         float &idd, float &sms)
+{
+    int lo = L.lo;
+    if ((lo > 0 && L.da >= wet_mm) || (lo < lut_len && L.db < wet_mm)) {
+        while (lo > 0 && s_dep[lo - 1] >= wet_mm) --lo;
+        while (lo < lut_len && s_dep[lo] < wet_mm) ++lo;
+        const int a = max(lo - 1, 0), b = min(lo, lut_len - 1);
+        L.da = s_dep[a];
+        L.db = s_dep[b];
+        L.sa = s_sig[a];
+        L.sb = s_sig[b];
+        L.ia = s_idd[a];
+        L.ib = s_idd[b];
     }
+    if (lo == lut_len) {
+        idd = L.ia;
+        sms = L.sa;
+    } else if (lo == 0) {
+        idd = L.ib;
+        sms = L.sb;
+    } else {
+        const float f = __fdividef(__fsub_rn(wet_mm, L.da), __fsub_rn(L.db, L.da));
+        idd = __fmaf_rn(__fsub_rn(L.ib, L.ia), f, L.ia);
+        sms = __fmaf_rn(__fsub_rn(L.sb, L.sa), f, L.sa);
+    }
+}
+
+__device__ __forceinline__ void layer_gauss(float wet_mm, float dist, const LayerK &K, float idd,
+                                            float sms, float &pf, float &hf, float &ps2,
+                                            float &hs2)
+{
     const float d = __fadd_rn(__fsub_rn(dist, wet_mm), K.off);
     const float st = __fadd_rn(__fmaf_rn(__fmaf_rn(K.ca, d, K.cb), d, K.cc), sms);
     const float w = fminf(fmaxf(wet_mm, 0.1f), __fsub_rn(K.r80, 0.1f));
@@ -186,6 +232,18 @@ __device__ __forceinline__ void layer_params(float wet_mm, float dist, const Lay
     hf = __fmul_rn(__fmul_rn(wh, iddn), rh);
     ps2 = st2 != 0.0f ? __fmul_rn(-0.5f * kLog2e, rp) : -INFINITY;
     hs2 = sht2 != 0.0f ? __fmul_rn(-0.5f * kLog2e, rh) : -INFINITY;
+}
+
+template <class Row>
+__device__ __forceinline__ void layer_params(float wet_mm, float dist, const LayerK &K,
+                                             const Row &s_dep, const Row &s_sig,
+                                             const Row &s_idd, int lut_len, float &pf,
+                                             float &hf, float &ps2, float &hs2)
+{
+    float idd, sms;
+    lut_eval(lut_load(wet_mm, K, s_dep, s_sig, s_idd, lut_len), wet_mm, s_dep, s_sig, s_idd,
+             lut_len, idd, sms);
+    layer_gauss(wet_mm, dist, K, idd, sms, pf, hf, ps2, hs2);
 }
 
 // Squared distance (times 1/|t|^2) from the spot's axis to the tile's BEV
@@ -369,20 +427,30 @@ __device__ __forceinline__ bool layer_sig2(const PbLayer &L, const TileBounds &t
     return true;
 }
 
+// nb receives a lower bound of the tile's nhs (cull_class), 0 where there is
+// none.
 __device__ __forceinline__ bool layer_skip(const PbLayer &L, const TileBounds &tb,
-                                           const PbBeam &B, float cut)
+                                           const PbBeam &B, float cut, float &nb)
 {
+    nb = 0.0f;
     if (!L.bound_ok) return false;
+    float it2, sig2;
+    if (!layer_sig2(L, tb, B, cut, it2, sig2)) return false;
+    nb = (0.5f * kLog2e) / sig2;
     float pxl, pxh, pyl, pyh;
     layer_box(L, tb, pxl, pxh, pyl, pyh);
     const float dx = fmaxf(0.0f, fmaxf(tb.x0 - pxh, pxl - tb.x1));
     const float dy = fmaxf(0.0f, fmaxf(tb.y0 - pyh, pyl - tb.y1));
     const float r2 = dx * dx + dy * dy;
     if (!(r2 > 0.0f)) return false;
-    float it2, sig2;
-    if (!layer_sig2(L, tb, B, cut, it2, sig2)) return false;
-    const float e = r2 * it2 * ((0.5f * kLog2e) / sig2);
-    return e >= kCullLog2;
+    return r2 * it2 * nb >= kCullLog2;
+}
+
+__device__ __forceinline__ bool layer_skip(const PbLayer &L, const TileBounds &tb,
+                                           const PbBeam &B, float cut)
+{
+    float nb;
+    return layer_skip(L, tb, B, cut, nb);
 }
 
 // Voxels of this block's tile owned by this thread: (li, lj, lk + step*q),
@@ -1057,9 +1125,27 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
 // evaluates every voxel with two fused multiply-adds.  The per-voxel work
 // is the exponent (one multiply), the SFU's ex2 and the accumulation, so
 // the spot loops are bound by the SFU's exp2 rate rather than shared with
-// the FMA pipe.  The LUT rows are read through the read-only data cache
-// (no staging barrier).  Decisions (layer selection, the per-layer range
-// cut, the spot cull) are those of the 8^3 tiles above.
+// the FMA pipe.  Decisions (layer selection, the per-layer range cut, the spot
+// cull) are those of the 8^3 tiles above.
+//
+// What bounds it: exp2.  A loop of the halo group alone reaches 84 % of the
+// measured exp2 peak, both terms 89 %; the rest of the launch is set-up, so
+// that is kept off the threads:
+//   - per beam, the tile's box comes from its eight corner voxels (one warp)
+//     and only the depths from every voxel;
+//   - one lane per layer tests it and leaves the kept layers' constants in
+//     shared memory (the 128 threads had each formed them again);
+//   - per kept layer the spots' cull values are formed first, and a layer
+//     whose spots all lie beyond the bound of the tile's widest halo (a fifth
+//     of the kept ones: the corners of the spots' box hold none) is left out
+//     before the per-voxel work;
+//   - the LUT intervals of the tile's depths are staged in shared memory with
+//     their differences, one interval per thread, so a voxel takes two shared
+//     loads instead of six global ones and a search.
+// Measured, launches with no spot in reach: 413 -> 281 us on the 4-beam
+// 256x256x160 plan; forward 5.65 -> 5.55 ms, adjoint 6.26 -> 6.05 ms; on the
+// 120^3 cube with 1,210 spots the forward 228 -> 193 us (141 us with each tile
+// shared by two blocks, tile_split).
 //
 // Shapes (template TY, TZ, KCULL): tiles of 8x8x8 (64 threads), 8x8x4 and
 // 8x4x8 (32 threads), 8x16x8 and 8x8x16 (128 threads); KCULL spots culled
@@ -1067,6 +1153,11 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
 // cull differently, or add a layer's spots in another order, and agree to
 // rounding.
 
+// Spots the forward evaluates side by side, both terms and halo only (up to
+// this many less one are added with weight 0 to fill the last group).  4-beam
+// 256x256x160 plan / 512x512x200 plan of 59,840 spots, forward alone: 4 spots
+// 5.65 / 100.8 ms, 5 5.58 / 99.7, 6 5.55 / 98.8, 7 5.74 / 102.3, 8 5.79 / 102.7.
+constexpr int kGroupBoth = 6, kGroupHalo = 6;
 constexpr int kLine = 8;
 
 // Line-tile record of one surviving spot: (-x, -y, x/VSADX, -y/VSADY),
@@ -1076,25 +1167,80 @@ struct LineSpot {
     float4 a, b, c;
 };
 
+// What the block reads of a kept (tile, layer) pair, written once by the lane
+// that selects the layer.
+constexpr int kLayerChunk = 32;   // layers selected at a time, one per lane of a warp
+struct LineLayer {
+    LayerK K;
+    float cut;             // 1.1 R80
+    float nb;              // lower bound of the tile's nhs (layer_skip), 0: none
+    int s0, n_spots;       // first spot in the plan's arrays, spots
+    int energy_id;
+    int lut0, n_lut;       // LUT intervals of the tile's depths, 0: not staged
+};
+
+// Interval lo of a LUT row, between its entries lo - 1 and lo, as a thread
+// stages it in shared memory for its block: first depth, reciprocal width,
+// and IDD and sigma with their differences across the interval.
+struct LutStage {
+    float4 a;              // depth, 1 / width, IDD, IDD difference
+    float2 b;              // sigma, sigma difference
+};
+
 // Per-voxel state that changes once per layer lives here rather than in
 // registers (thread t's voxel q at [q][t]), so that the spot loops keep
 // only their own values live.
-template <int NT, int KCULL, bool BEAM_OUT = false, bool DOSE = true>
+template <int NT, int KCULL, bool BEAM_OUT = false, bool DOSE = true, int SPLIT = 1>
 struct LineShared {
     static constexpr int kWarps = NT / 32;
-    LineSpot spot[NT * KCULL + 8];
-    float gsum[NT * KCULL + 8];      // adjoint: per-slot gradient partials
+    static constexpr int kStage = NT;   // most LUT intervals staged
+    union {
+        LineSpot spot[NT * KCULL + (DOSE ? 16 : 8)];   // and the last groups' padding
+        LutStage lut[kStage];        // before the layer's spots are compacted
+        float2 lut_at[kLine][NT];    // or IDD and sigma per voxel, from rows not staged
+    };
+    int lut_bad;                     // the layer whose staged row is not uniform
+    float gsum[DOSE ? 1 : NT * KCULL + 8];   // adjoint: per-slot gradient partials
     float w[kLine][NT];              // the beam's 10*WET per voxel (INF: not valid)
     float d[kLine][NT];              // distance to the source per voxel
     float tot[2][kLine][DOSE ? NT : 1];   // dose: compensated sum over layers and beams
     float pfh[2][kLine][DOSE ? NT : 1];   // dose: the layer's prefactors Pf, Hf
+    // joint tiles: a layer's dose per voxel, for the cluster's other blocks
+    float ld[SPLIT > 1 ? 2 : 1][kLine][DOSE && SPLIT > 1 ? NT : 1];
     float bsum[BEAM_OUT ? 2 : 1][kLine][BEAM_OUT ? NT : 1];   // each beam's own sum
+    TileBounds tb;                   // the tile's box and depth range for the beam
+    float4 step;                     // head-frame step per voxel along x: x, y, and of the
+                                     // divergence factors
     float red[kWarps][kRedSlots];
     int wcount[KCULL][kWarps];
     int wcount_h[KCULL][kWarps];
-    int lcount[kWarps];
-    int lsel[NT];
+    int nsel;                        // the chunk's kept layers
+    LineLayer layer[kLayerChunk];
 };
+
+// Marks a voxel that a layer does not reach, where a layer's dose per voxel is
+// handed on: a NaN that no FP32 instruction returns (theirs is 0x7fffffff).
+constexpr int kNoDose = -1;
+
+// Barrier over the blocks of a cluster; writes to shared memory before it are
+// seen by the cluster's other blocks after it.
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// The value at this block's shared-memory address `p` in the shared memory of
+// the cluster's block `rank`.
+__device__ __forceinline__ float cluster_load(const float *p, int rank)
+{
+    const unsigned own = (unsigned)__cvta_generic_to_shared(p);
+    unsigned a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
 
 // Offsets q - 3.5 of a line's voxel pair (2p, 2p + 1) from the line's centre
 // (exact in FP32).
@@ -1118,7 +1264,72 @@ __device__ __forceinline__ void line_spot(const LineSpot &r, float Xc, float Yc,
     B1 = __fmaf_rn(ax, r.c.x, __fmaf_rn(ay, r.c.y, __fmul_rn(az, r.c.z)));
 }
 
-template <int TY, int TZ, int KCULL, bool BEAM_OUT, int MODE = kModeDose>
+// Head-frame geometry of one line of a beam: the step per voxel along x and
+// the line's centre, with the divergence factors' step and centre.
+struct LineGeom {
+    float dX, dY, dZ, dgx, dgy, Xc, Yc, Zc, gxc, gyc;
+};
+
+__device__ __forceinline__ LineGeom line_geom(const PbGrid &g, const PbBeam &B, int i0, int j,
+                                              int k)
+{
+    LineGeom G;
+    image_to_head(B.geom, g.spacing, 0.0f, 0.0f, G.dX, G.dY, G.dZ);
+    G.dgx = -__fdiv_rn(G.dZ, B.geom.vsadx);
+    G.dgy = -__fdiv_rn(G.dZ, B.geom.vsady);
+    float px, py, pz, X0, Y0, Z0;
+    vox_mm(B.geom, g.spacing, i0, j, k, px, py, pz);
+    image_to_head(B.geom, px, py, pz, X0, Y0, Z0);
+    G.Xc = __fmaf_rn(3.5f, G.dX, X0);
+    G.Yc = __fmaf_rn(3.5f, G.dY, Y0);
+    G.Zc = __fmaf_rn(3.5f, G.dZ, Z0);
+    G.gxc = __fsub_rn(1.0f, __fdiv_rn(G.Zc, B.geom.vsadx));
+    G.gyc = __fsub_rn(1.0f, __fdiv_rn(G.Zc, B.geom.vsady));
+    return G;
+}
+
+// A line tile's box (TileBounds without the depths) from its eight corner
+// voxels, one per lane of each group of eight lanes.  The head-frame
+// coordinates and the divergence factors are affine in the voxel's indexes,
+// so their extremes over the tile are at its corners; the distance to the
+// source is convex, so its greatest value is at a corner too, and its least
+// is bounded from below by that of the box's nearest point.
+__device__ __forceinline__ TileBounds corner_bounds(const PbGrid &g, const PbBeam &B, int i0,
+                                                    int j0, int k0, int nj, int nk, int lane,
+                                                    float4 &step)
+{
+    const int j = (lane & 2) ? min(j0 + nj, g.ny) - 1 : j0;
+    const int k = (lane & 4) ? min(k0 + nk, g.nz) - 1 : k0;
+    const float o = (lane & 1) ? line_off(min(kLine, g.nx - i0) - 1) : line_off(0);
+    const LineGeom G = line_geom(g, B, i0, j, k);
+    step = make_float4(G.dX, G.dY, G.dgx, G.dgy);
+    const float GX = __fmaf_rn(o, G.dgx, G.gxc), GY = __fmaf_rn(o, G.dgy, G.gyc);
+    const float X = __fmaf_rn(o, G.dX, G.Xc), Y = __fmaf_rn(o, G.dY, G.Yc);
+    const float Z = __fmaf_rn(o, G.dZ, G.Zc);
+    float v[9] = {X, X, Y, Y, GX, GX, GY, GY, Z};   // even: min, odd: max; Z: max
+    float d1 = source_distance(B, X, Y, Z);
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const float u = __shfl_xor_sync(0xffffffffu, v[m], s);
+            v[m] = (m & 1) ? fmaxf(v[m], u) : fminf(v[m], u);
+        }
+        v[8] = fmaxf(v[8], __shfl_xor_sync(0xffffffffu, v[8], s));
+        d1 = fmaxf(d1, __shfl_xor_sync(0xffffffffu, d1, s));
+    }
+    TileBounds tb;
+    tb.x0 = v[0]; tb.x1 = v[1]; tb.y0 = v[2]; tb.y1 = v[3];
+    tb.gx0 = v[4]; tb.gx1 = v[5]; tb.gy0 = v[6]; tb.gy1 = v[7];
+    const float sad = 0.5f * (B.geom.vsadx + B.geom.vsady);
+    const float nx = fmaxf(0.0f, fmaxf(v[0], -v[1])), ny = fmaxf(0.0f, fmaxf(v[2], -v[3]));
+    const float nz = fmaxf(0.0f, sad - v[8]);
+    tb.d0 = 0.99999f * sqrtf(nx * nx + ny * ny + nz * nz);
+    tb.d1 = d1;
+    return tb;
+}
+
+template <int TY, int TZ, int KCULL, bool BEAM_OUT, int MODE = kModeDose, int SPLIT = 1>
 __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int tz,
                                           const float *__restrict__ wet,
                                           const PbLayer *__restrict__ layers,
@@ -1127,10 +1338,11 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                           float *__restrict__ dose,
                                           float *__restrict__ beam_dose,
                                           LineShared<TY * TZ, KCULL, BEAM_OUT,
-                                                     MODE == kModeDose> &sh,
+                                                     MODE == kModeDose, SPLIT> &sh,
                                           unsigned long long *count = nullptr,
                                           const float *__restrict__ wfield = nullptr,
-                                          float *__restrict__ grad = nullptr)
+                                          float *__restrict__ grad = nullptr, int rank = 0,
+                                          int ranks = 1)
 {
     constexpr int NT = TY * TZ;
     constexpr int kWarps = NT / 32;
@@ -1140,6 +1352,9 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
     static_assert(MODE == kModeDose || MODE == kModeCount || MODE == kModeAdjoint,
                   "line tiles: dose, count or weight adjoint");
     constexpr int kCap = NT * KCULL;
+    // end of the halo-only spots: the forward's filled-up groups need the room
+    constexpr int kTop = MODE == kModeDose ? kCap + 16 : kCap;
+    static_assert(kGroupBoth + kGroupHalo - 2 <= 16, "padding of both classes");
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
 
@@ -1149,6 +1364,7 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
     const int64_t vbase = i0 + (int64_t)A.g.nx * (j + (int64_t)A.g.ny * k);
     const int64_t V = (int64_t)A.g.nx * A.g.ny * A.g.nz;
     unsigned long long n_ex2 = 0, n_eval = 0;
+    if (t == 0) sh.lut_bad = 0;   // before the first barrier
 
     if constexpr (MODE == kModeDose) {
 #pragma unroll
@@ -1178,122 +1394,186 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
 
     for (int b = 0; b < A.n_beams; ++b) {
         const PbBeam &B = A.beams[b];
-        // line geometry: head-frame centre and step per voxel along x
-        float dX, dY, dZ;
-        image_to_head(B.geom, A.g.spacing, 0.0f, 0.0f, dX, dY, dZ);
-        const float dgx = -__fdiv_rn(dZ, B.geom.vsadx), dgy = -__fdiv_rn(dZ, B.geom.vsady);
-        float Xc, Yc, Zc;
+        float Xc, Yc, gxc, gyc;   // the line's centre and its divergence factors
         {
-            float px, py, pz, X0, Y0, Z0;
-            vox_mm(B.geom, A.g.spacing, i0, j, k, px, py, pz);
-            image_to_head(B.geom, px, py, pz, X0, Y0, Z0);
-            Xc = __fmaf_rn(3.5f, dX, X0);
-            Yc = __fmaf_rn(3.5f, dY, Y0);
-            Zc = __fmaf_rn(3.5f, dZ, Z0);
+            const LineGeom G = line_geom(A.g, B, i0, j, k);
+            Xc = G.Xc;
+            Yc = G.Yc;
+            gxc = G.gxc;
+            gyc = G.gyc;
         }
-        const float gxc = __fsub_rn(1.0f, __fdiv_rn(Zc, B.geom.vsadx));
-        const float gyc = __fsub_rn(1.0f, __fdiv_rn(Zc, B.geom.vsady));
-        TileBounds tb;
         {
-            // the beam's depth and source distance per voxel into shared
-            // memory; the tile's box over its valid voxels
-            float v[12] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY,
-                           INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
+            float w0 = INFINITY, w1 = -INFINITY;
 #pragma unroll
             for (int q = 0; q < kLine; ++q) {
-                const float o = line_off(q);
-                float w = INFINITY, dd = 0.0f;
+                float w = INFINITY;
                 if (q < nvalid) {
-                    const float X = __fmaf_rn(o, dX, Xc), Y = __fmaf_rn(o, dY, Yc);
-                    const float Z = __fmaf_rn(o, dZ, Zc);
                     w = __fmul_rn(__ldg(wet + b * V + vbase + q), 10.0f);
-                    dd = source_distance(B, X, Y, Z);
-                    const float GX = __fmaf_rn(o, dgx, gxc), GY = __fmaf_rn(o, dgy, gyc);
-                    v[0] = fminf(v[0], X);  v[1] = fmaxf(v[1], X);
-                    v[2] = fminf(v[2], Y);  v[3] = fmaxf(v[3], Y);
-                    v[4] = fminf(v[4], GX); v[5] = fmaxf(v[5], GX);
-                    v[6] = fminf(v[6], GY); v[7] = fmaxf(v[7], GY);
-                    v[8] = fminf(v[8], dd); v[9] = fmaxf(v[9], dd);
                     // the least depth over voxels that can be active; a NaN
                     // depth is never skipped
                     if (!ADJ || wv[q] != 0.0f) {
-                        v[10] = fminf(v[10], w == w ? w : -INFINITY);
-                        v[11] = fmaxf(v[11], w == w ? w : INFINITY);
+                        w0 = fminf(w0, w == w ? w : -INFINITY);
+                        w1 = fmaxf(w1, w == w ? w : INFINITY);
                     }
                 }
                 sh.w[q][t] = w;
-                sh.d[q][t] = dd;
             }
-#pragma unroll
-            for (int m = 0; m < 12; ++m) v[m] = (m & 1) ? warp_max(v[m]) : warp_min(v[m]);
+            w0 = warp_min(w0);
+            w1 = warp_max(w1);
             if (lane == 0) {
-#pragma unroll
-                for (int m = 0; m < 12; ++m) sh.red[warp][m] = v[m];
+                sh.red[warp][0] = w0;
+                sh.red[warp][1] = w1;
             }
             __syncthreads();
-            float r[12];
-#pragma unroll
-            for (int m = 0; m < 12; ++m) r[m] = sh.red[0][m];
-            for (int w = 1; w < kWarps; ++w) {
-#pragma unroll
-                for (int m = 0; m < 12; ++m)
-                    r[m] = (m & 1) ? fmaxf(r[m], sh.red[w][m]) : fminf(r[m], sh.red[w][m]);
-            }
-            tb.x0 = r[0]; tb.x1 = r[1]; tb.y0 = r[2]; tb.y1 = r[3];
-            tb.gx0 = r[4]; tb.gx1 = r[5]; tb.gy0 = r[6]; tb.gy1 = r[7];
-            tb.d0 = r[8]; tb.d1 = r[9]; tb.w0 = r[10]; tb.w1 = r[11];
         }
+        bool have_d = false;   // sh.d is filled for this beam
         if constexpr (BEAM_OUT) {
 #pragma unroll
             for (int q = 0; q < kLine; ++q) sh.bsum[0][q][t] = sh.bsum[1][q][t] = 0.0f;
         }
 
-        for (int l0 = 0; l0 < B.n_layers; l0 += NT) {
-            __syncthreads();   // the previous chunk's list and the bounds have been read
-            bool keep = false;
-            {
-                const int l = l0 + t;
-                if (l < B.n_layers) {
-                    const PbLayer L = layers[B.layer_start + l];
-                    const float cut = __fmul_rn(1.1f, L.r80);
-                    keep = L.n_spots > 0 && tb.w0 <= cut && !layer_skip(L, tb, B, cut);
+        for (int l0 = 0; l0 < B.n_layers; l0 += kLayerChunk) {
+            if (l0 > 0) __syncthreads();   // the previous chunk's records have been read
+            if (warp == 0) {
+                // one lane per layer: the tile's box and depth range, the
+                // layers that can reach it and their constants.  Kept in
+                // shared memory, since the spot loops need every register.
+                float4 step;
+                TileBounds tb = corner_bounds(A.g, B, i0, ty * TY, tz * TZ, TY, TZ, lane, step);
+                tb.w0 = sh.red[0][0];
+                tb.w1 = sh.red[0][1];
+                for (int w = 1; w < kWarps; ++w) {
+                    tb.w0 = fminf(tb.w0, sh.red[w][0]);
+                    tb.w1 = fmaxf(tb.w1, sh.red[w][1]);
+                }
+                if (lane == 0) {
+                    sh.tb = tb;
+                    sh.step = step;
+                }
+                LineLayer Y;
+                bool keep = false;
+                if (l0 + lane < B.n_layers) {
+                    const PbLayer L = layers[B.layer_start + l0 + lane];
+                    Y.cut = __fmul_rn(1.1f, L.r80);
+                    Y.s0 = B.spot_start + L.spot_start;
+                    Y.n_spots = L.n_spots;
+                    Y.energy_id = L.energy_id;
+                    keep = L.n_spots > 0 && tb.w0 <= Y.cut && !layer_skip(L, tb, B, Y.cut, Y.nb);
+                    if (keep) {
+                        Y.K = layer_consts(L.r80,
+                                           B.dvp_dev + (size_t)B.dvp_len * L.energy_id + 2,
+                                           RowG{B.depths_dev + (size_t)L.energy_id * B.lut_len},
+                                           B.lut_len);
+                        // the row's intervals over the tile's depths, staged
+                        // where the guess of lut_load is the interval itself:
+                        // a table from 0 in steps of a power of two (each
+                        // entry is checked when it is staged)
+                        Y.lut0 = lut_guess(tb.w0, Y.K, B.lut_len);
+                        Y.n_lut = lut_guess(fminf(tb.w1, Y.cut), Y.K, B.lut_len) - Y.lut0 + 1;
+                        if (!(Y.K.d0 == 0.0f && Y.K.inv_step > 0.0f &&
+                              (__float_as_int(Y.K.inv_step) & 0x7fffff) == 0 &&
+                              tb.w0 > -INFINITY && Y.n_lut <= sh.kStage))
+                            Y.n_lut = 0;
+                    }
+                }
+                const unsigned lm = __ballot_sync(0xffffffffu, keep);
+                if (keep) sh.layer[__popc(lm & ((1u << lane) - 1u))] = Y;
+                if (lane == 0) sh.nsel = __popc(lm);
+            }
+            __syncthreads();
+            const int nsel = sh.nsel;
+            if (nsel > 0 && !have_d) {
+                // source distance per voxel, each thread its own line's
+                have_d = true;
+                const LineGeom G = line_geom(A.g, B, i0, j, k);
+#pragma unroll
+                for (int q = 0; q < kLine; ++q) {
+                    const float o = line_off(q);
+                    sh.d[q][t] = q < nvalid ? source_distance(B, __fmaf_rn(o, G.dX, G.Xc),
+                                                              __fmaf_rn(o, G.dY, G.Yc),
+                                                              __fmaf_rn(o, G.dZ, G.Zc))
+                                            : 0.0f;
                 }
             }
-            const unsigned lm = __ballot_sync(0xffffffffu, keep);
-            if (lane == 0) sh.lcount[warp] = __popc(lm);
-            __syncthreads();
-            int nsel = 0, lpos = 0;
-            for (int w = 0; w < kWarps; ++w) {
-                if (w == warp) lpos = nsel + __popc(lm & ((1u << lane) - 1u));
-                nsel += sh.lcount[w];
-            }
-            if (keep) sh.lsel[lpos] = l0 + t;
-            __syncthreads();
-            for (int li = 0; li < nsel; ++li) {
-                // every kept layer has spots, so each runs at least one
+            int round = 0;
+            for (int l1 = 0; l1 < nsel; l1 += ranks, ++round) {
+              const int li = l1 + rank;
+              bool live = li < nsel;
+              const int layer_id = (b << 20) + l0 + li + 1;   // not 0
+              const LineLayer &Y = sh.layer[live ? li : 0];
+              const int s0 = Y.s0, n_spots = live ? Y.n_spots : 0;
+              // the cull values and weights of a round's spots, loaded ahead
+              // of the per-voxel work that they do not depend on
+              float ev[KCULL], mv[KCULL];
+              auto load_round = [&](int base) {
+#pragma unroll
+                for (int c = 0; c < KCULL; ++c) {
+                    const int si = base + c * NT + t;
+                    ev[c] = mv[c] = 0.0f;
+                    if (si < n_spots) {
+                        const float4 g0 = __ldg(geo + 2 * (int64_t)(s0 + si));
+                        if constexpr (MODE == kModeDose) mv[c] = __ldg(mu + s0 + si);
+                        ev[c] = cull_r2(g0.x, g0.y, g0.z, sh.tb);
+                    }
+                }
+              };
+              if (live) {
+                load_round(0);
+                if (t < Y.n_lut) {
+                    const int lo = Y.lut0 + t, a = max(lo - 1, 0), c = min(lo, B.lut_len - 1);
+                    const size_t ro = (size_t)Y.energy_id * B.lut_len;
+                    const float da = __ldg(B.depths_dev + ro + a);
+                    const float dc = __ldg(B.depths_dev + ro + c);
+                    const float ia = __ldg(B.idds_dev + ro + a), ic = __ldg(B.idds_dev + ro + c);
+                    const float sa = __ldg(B.sigmas_dev + ro + a);
+                    const float sc = __ldg(B.sigmas_dev + ro + c);
+                    const bool inner = lo > 0 && lo < B.lut_len;
+                    if (da * Y.K.inv_step != (float)a || dc * Y.K.inv_step != (float)c)
+                        sh.lut_bad = layer_id;
+                    LutStage r;
+                    r.a = make_float4(da, inner ? Y.K.inv_step : 0.0f, ia,
+                                      inner ? __fsub_rn(ic, ia) : 0.0f);
+                    r.b = make_float2(sa, inner ? __fsub_rn(sc, sa) : 0.0f);
+                    sh.lut[t] = r;
+                }
+                // a layer of one round none of whose spots can pass, with
+                // the bound of the tile's widest halo, is left out
+                bool near = !(Y.nb > 0.0f && n_spots <= kCap);
+#pragma unroll
+                for (int c = 0; c < KCULL; ++c)
+                    near |= c * NT + t < n_spots && !(ev[c] * Y.nb >= kCullLog2);
+                live = __syncthreads_or(near);
+                if constexpr (MODE == kModeDose && SPLIT > 1) {
+                    if (ranks > 1 && !live) {
+#pragma unroll
+                        for (int q = 0; q < kLine; ++q)
+                            sh.ld[round & 1][q][t] = __int_as_float(kNoDose);
+                    }
+                }
+              }
+              if (live) {
+                // every layer taken has spots, so it runs at least one
                 // compaction round, whose barriers separate this layer's
                 // block_max2 from the next one's
-                const PbLayer L = layers[B.layer_start + sh.lsel[li]];
-                const float cut = __fmul_rn(1.1f, L.r80);
-                const size_t ro = (size_t)L.energy_id * B.lut_len;
+                const float cut = Y.cut;
+                const size_t ro = (size_t)Y.energy_id * B.lut_len;
                 const RowG dep{B.depths_dev + ro}, sig{B.sigmas_dev + ro}, idd{B.idds_dev + ro};
-                const LayerK K =
-                    layer_consts(L.r80, B.dvp_dev + (size_t)B.dvp_len * L.energy_id + 2, dep,
-                                 B.lut_len);
+                const LayerK &K = Y.K;
                 float pf[kLine], hf[kLine];
                 float2 PS[kLine / 2], HS[kLine / 2];   // voxel pairs (q, q + 1)
                 bool act[kLine];
                 float hmax = -INFINITY, pmax = -INFINITY;
                 // every voxel's parameters without branching (inactive
-                // voxels take a harmless depth and are masked afterwards)
+                // voxels take a harmless depth and are masked afterwards);
+                const bool staged = Y.n_lut > 0 && sh.lut_bad != layer_id;
 #pragma unroll
                 for (int q = 0; q < kLine; ++q) {
-                    const float w = sh.w[q][t];
-                    act[q] = !(w > cut) && q < nvalid;
+                    act[q] = !(sh.w[q][t] > cut) && q < nvalid;
                     if constexpr (ADJ) act[q] = act[q] && wv[q] != 0.0f;
+                }
+                auto voxel = [&](int q, float w, float id, float sm) {
                     float ps2, hs2;
-                    layer_params(act[q] ? w : 0.0f, sh.d[q][t], K, dep, sig, idd, B.lut_len,
-                                 pf[q], hf[q], ps2, hs2);
+                    layer_gauss(w, sh.d[q][t], K, id, sm, pf[q], hf[q], ps2, hs2);
                     if (act[q]) {
                         hmax = fmaxf(hmax, hs2);
                         pmax = fmaxf(pmax, ps2);
@@ -1311,6 +1591,32 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                         sh.pfh[0][q][t] = pf[q];
                         sh.pfh[1][q][t] = hf[q];
                     }
+                };
+                if (!staged) {
+#pragma unroll 1
+                    for (int q = 0; q < kLine; ++q) {
+                        const float w0 = sh.w[q][t];
+                        const float w = w0 > cut ? 0.0f : w0;
+                        float2 v;
+                        lut_eval(lut_load(w, K, dep, sig, idd, B.lut_len), w, dep, sig, idd,
+                                 B.lut_len, v.x, v.y);
+                        sh.lut_at[q][t] = v;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < kLine; ++q) {
+                    const float w = act[q] ? sh.w[q][t] : 0.0f;
+                    float2 v;
+                    if (staged) {
+                        const int e = (int)ceilf(__fmul_rn(w, K.inv_step)) - Y.lut0;
+                        const LutStage r = sh.lut[min(max(e, 0), Y.n_lut - 1)];
+                        const float f = __fmul_rn(__fsub_rn(w, r.a.x), r.a.y);
+                        v.x = __fmaf_rn(r.a.w, f, r.a.z);
+                        v.y = __fmaf_rn(r.b.y, f, r.b.x);
+                    } else {
+                        v = sh.lut_at[q][t];
+                    }
+                    voxel(q, w, v.x, v.y);
                 }
                 float nhs, nps;
                 block_max2<NT>(hmax, pmax, sh.red, nhs, nps);
@@ -1330,19 +1636,17 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                     }
                 }
 
-                const int s0 = B.spot_start + L.spot_start;
-                for (int base = 0; base < L.n_spots; base += kCap) {
+                for (int base = 0; base < n_spots; base += kCap) {
                     int cls[KCULL];
                     float4 ga[KCULL], gb[KCULL];
                     unsigned m2[KCULL], m1[KCULL];
 #pragma unroll
                     for (int c = 0; c < KCULL; ++c) {
                         const int si = base + c * NT + t;
-                        cls[c] = 0;
-                        if (si < L.n_spots) {
+                        cls[c] = si < n_spots ? cull_class(ev[c], nhs, nps) : 0;
+                        if (cls[c]) {
                             ga[c] = __ldg(geo + 2 * (int64_t)(s0 + si));
-                            cls[c] = cull_class(cull_r2(ga[c].x, ga[c].y, ga[c].z, tb), nhs, nps);
-                            if (cls[c]) gb[c] = __ldg(geo + 2 * (int64_t)(s0 + si) + 1);
+                            gb[c] = __ldg(geo + 2 * (int64_t)(s0 + si) + 1);
                         }
                         m2[c] = __ballot_sync(0xffffffffu, cls[c] == 2);
                         m1[c] = __ballot_sync(0xffffffffu, cls[c] == 1);
@@ -1352,6 +1656,7 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                         }
                     }
                     __syncthreads();
+                    const float4 stp = sh.step;
                     int n2 = 0, n1 = 0;
                     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
@@ -1369,13 +1674,13 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                             const int si = s0 + base + c * NT + t;
                             // the dose keeps the spot's weight, the adjoint its index
                             const float wgt =
-                                MODE == kModeDose ? __ldg(mu + si) : __int_as_float(si);
+                                MODE == kModeDose ? mv[c] : __int_as_float(si);
                             const float nx = -ga[c].x, ny = -ga[c].y, txs = ga[c].w;
                             const float nty = -gb[c].x, it2 = ga[c].z;
                             // the spot's step of each component per voxel along x
-                            const float sx = __fmaf_rn(nx, dgx, dX);
-                            const float sy = __fmaf_rn(ny, dgy, dY);
-                            const float sz = __fmaf_rn(txs, dY, __fmul_rn(nty, dX));
+                            const float sx = __fmaf_rn(nx, stp.z, stp.x);
+                            const float sy = __fmaf_rn(ny, stp.w, stp.y);
+                            const float sz = __fmaf_rn(txs, stp.y, __fmul_rn(nty, stp.x));
                             const float c2 = __fmul_rn(
                                 it2, __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, __fmul_rn(sz, sz))));
                             const float k2 = __fmul_rn(2.0f, it2);
@@ -1384,10 +1689,25 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                             r.b = make_float4(-gb[c].y, it2, c2, wgt);
                             r.c = make_float4(__fmul_rn(k2, sx), __fmul_rn(k2, sy),
                                               __fmul_rn(k2, sz), 0.0f);
-                            sh.spot[cls[c] == 2 ? pos2 : kCap - 1 - pos1] = r;
+                            sh.spot[cls[c] == 2 ? pos2 : kTop - 1 - pos1] = r;
                         }
                     }
+                    if constexpr (MODE == kModeDose) {
+                        // weight 0 and an axis distance above 0 everywhere
+                        // on the line
+                        LineSpot r;
+                        r.a = r.c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        r.b = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+                        if (t < kGroupBoth - 1 &&
+                            n2 + t < (n2 + kGroupBoth - 1) / kGroupBoth * kGroupBoth)
+                            sh.spot[n2 + t] = r;
+                        if (t < kGroupHalo - 1 &&
+                            n1 + t < (n1 + kGroupHalo - 1) / kGroupHalo * kGroupHalo)
+                            sh.spot[kTop - 1 - n1 - t] = r;
+                    }
                     __syncthreads();
+                    // the next round's, while this one's spots are evaluated
+                    if (base + kCap < n_spots) load_round(base + kCap);
                     if constexpr (COUNT) {
                         n_ex2 += (unsigned long long)(kLine * NT) * (2 * n2 + n1);
                         n_eval += (unsigned long long)(kLine * NT) * (n2 + n1);
@@ -1450,46 +1770,59 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                             sh.gsum[sl] = 0.0f;
                         }
                     } else {
-                        // both terms (unrolled by 4: the per-beam forward
-                        // 6.37 against 6.49 ms, the plain one unchanged)
-#pragma unroll 4
-                        for (int c = 0; c < n2; ++c) {
-                            const LineSpot r = sh.spot[c];
-                            float S0, B1;
-                            line_spot(r, Xc, Yc, gxc, gyc, S0, B1);
-                            const float2 s0 = f2(S0), b1 = f2(B1), c2 = f2(r.b.z), w = f2(r.b.w);
+                        // groups of kGroup spots, evaluated side by side;
+                        // the class's last group is filled up with spots of
+                        // weight 0
+                        auto group = [&](auto two, auto size, const int c0) {
+                            constexpr int kGroup = decltype(size)::value;
+                            float S0[kGroup], B1[kGroup], C2[kGroup], W[kGroup];
+#pragma unroll
+                            for (int u = 0; u < kGroup; ++u) {
+                                const LineSpot r = sh.spot[c0 + u];
+                                line_spot(r, Xc, Yc, gxc, gyc, S0[u], B1[u]);
+                                C2[u] = r.b.z;
+                                W[u] = r.b.w;
+                            }
 #pragma unroll
                             for (int p = 0; p < kLine / 2; ++p) {
                                 const float2 o = line_off2(p);
-                                const float2 S = __ffma2_rn(__ffma2_rn(c2, o, b1), o, s0);
-                                AP[p] = __ffma2_rn(w, ex2x2(__fmul2_rn(PS[p], S)), AP[p]);
-                                AH[p] = __ffma2_rn(w, ex2x2(__fmul2_rn(HS[p], S)), AH[p]);
-                            }
-                        }
-                        // halo only (unrolled by 4: 6.04 against 6.12 ms)
-#pragma unroll 4
-                        for (int c = kCap - n1; c < kCap; ++c) {
-                            const LineSpot r = sh.spot[c];
-                            float S0, B1;
-                            line_spot(r, Xc, Yc, gxc, gyc, S0, B1);
-                            const float2 s0 = f2(S0), b1 = f2(B1), c2 = f2(r.b.z), w = f2(r.b.w);
 #pragma unroll
-                            for (int p = 0; p < kLine / 2; ++p) {
-                                const float2 o = line_off2(p);
-                                const float2 S = __ffma2_rn(__ffma2_rn(c2, o, b1), o, s0);
-                                AH[p] = __ffma2_rn(w, ex2x2(__fmul2_rn(HS[p], S)), AH[p]);
+                                for (int u = 0; u < kGroup; ++u) {
+                                    const float2 S = __ffma2_rn(
+                                        __ffma2_rn(f2(C2[u]), o, f2(B1[u])), o, f2(S0[u]));
+                                    if constexpr (decltype(two)::value)
+                                        AP[p] = __ffma2_rn(f2(W[u]), ex2x2(__fmul2_rn(PS[p], S)),
+                                                           AP[p]);
+                                    AH[p] = __ffma2_rn(f2(W[u]), ex2x2(__fmul2_rn(HS[p], S)),
+                                                       AH[p]);
+                                }
                             }
-                        }
+                        };
+                        using Both = std::integral_constant<int, kGroupBoth>;
+                        using Halo = std::integral_constant<int, kGroupHalo>;
+#pragma unroll 1
+                        for (int c = 0; c < n2; c += kGroupBoth)
+                            group(std::true_type{}, Both{}, c);
+#pragma unroll 1
+                        for (int c = kTop - (n1 + kGroupHalo - 1) / kGroupHalo * kGroupHalo;
+                             c < kTop; c += kGroupHalo)
+                            group(std::false_type{}, Halo{}, c);
                     }
                     __syncthreads();
                 }
                 if constexpr (MODE == kModeDose) {
 #pragma unroll
                     for (int q = 0; q < kLine; ++q) {
-                        if (act[q]) {
+                        const bool act_q = q < nvalid && !(sh.w[q][t] > Y.cut);
+                        float ld = __int_as_float(kNoDose);
+                        if (act_q) {
                             const float ap = (q & 1) ? AP[q >> 1].y : AP[q >> 1].x;
                             const float ah = (q & 1) ? AH[q >> 1].y : AH[q >> 1].x;
-                            const float ld = fmaf(sh.pfh[0][q][t], ap, sh.pfh[1][q][t] * ah);
+                            ld = fmaf(sh.pfh[0][q][t], ap, sh.pfh[1][q][t] * ah);
+                        }
+                        if (SPLIT > 1 && ranks > 1) {
+                            sh.ld[round & 1][q][t] = ld;
+                        } else if (act_q) {
                             if constexpr (BEAM_OUT) {
                                 float bs = sh.bsum[0][q][t], bc = sh.bsum[1][q][t];
                                 neumaier(bs, bc, ld);
@@ -1503,6 +1836,29 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                         }
                     }
                 }
+              }
+              if constexpr (MODE == kModeDose && SPLIT > 1) {
+                if (ranks > 1) {
+                    // the round's layers, in order, into the voxels this
+                    // block owns.  The next round writes the other buffer,
+                    // and the one after it starts behind the next barrier,
+                    // which every reader of this buffer has passed by then.
+                    cluster_barrier();
+                    constexpr int kOwn = kLine / SPLIT;
+                    const int nr = min(ranks, nsel - l1);
+#pragma unroll
+                    for (int m = 0; m < kOwn; ++m) {
+                        const int q = rank * kOwn + m;
+                        float ts = sh.tot[0][q][t], tc = sh.tot[1][q][t];
+                        for (int r = 0; r < nr; ++r) {
+                            const float ld = cluster_load(&sh.ld[round & 1][q][t], r);
+                            if (__float_as_int(ld) != kNoDose) neumaier(ts, tc, ld);
+                        }
+                        sh.tot[0][q][t] = ts;
+                        sh.tot[1][q][t] = tc;
+                    }
+                }
+              }
             }
         }
         if (BEAM_OUT) {
@@ -1519,22 +1875,25 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
             atomicAdd(count + 1, n_eval);
         }
     } else if constexpr (MODE == kModeDose) {
+        const int own = SPLIT > 1 && ranks > 1 ? kLine / SPLIT : kLine;
 #pragma unroll
         for (int q = 0; q < kLine; ++q)
-            if (q < nvalid) dose[vbase + q] = (sh.tot[0][q][t] + sh.tot[1][q][t]) * A.scale;
+            if (q < nvalid && (SPLIT == 1 || q / own == rank))
+                dose[vbase + q] = (sh.tot[0][q][t] + sh.tot[1][q][t]) * A.scale;
+        // no block leaves while another may still read its shared memory
+        if (SPLIT > 1 && ranks > 1) cluster_barrier();
     }
 }
 
 // Resident blocks per SM the line-tile kernels are compiled for (their
-// register budget): 20 of 32 threads, 10 of 64, 5 of 128.  The kernels with
-// more live state per thread (the per-beam forward's extra sums, the
-// adjoint's weighted prefactors and spot groups) take 4 of 128 threads (128
-// registers): on the 4-beam 256x256x160 plan the adjoint went from 6.65 to
-// 6.43 ms and the per-beam forward from 6.78 to 6.47 ms, while the plain
-// forward is faster at 5 (6.12 against 6.25 ms).
-template <int NT, bool HEAVY = false> constexpr int line_min_blocks()
+// register budget): 4 of 128 threads and 8 of 64 (128 registers a thread), 20
+// of 32.  The groups of kGroupHalo spots need the registers more than the
+// kernel needs a fifth block: on the 4-beam 256x256x160 plan the forward took
+// 5.85 ms at 5 blocks (96 registers) against 5.55 ms, the 120^3 water cube
+// 225 against 193 us.
+template <int NT> constexpr int line_min_blocks()
 {
-    return NT == 32 ? 20 : (NT == 64 ? 10 : (HEAVY ? 4 : 5));
+    return NT == 32 ? 20 : (NT == 64 ? 8 : 4);
 }
 
 #ifndef PB_TILE_ORDER
@@ -1595,7 +1954,7 @@ __device__ __forceinline__ bool line_tile_coords(const PlanArgs &A, long long ti
 }
 
 template <int TY, int TZ, int KCULL, bool BEAM_OUT>
-__global__ void __launch_bounds__(TY * TZ, line_min_blocks<TY * TZ, BEAM_OUT>())
+__global__ void __launch_bounds__(TY * TZ, line_min_blocks<TY * TZ>())
 k_dose_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
             const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
             const float *__restrict__ mu, float *__restrict__ dose,
@@ -1605,6 +1964,25 @@ k_dose_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
     int tx, ty, tz;
     if (!line_tile_coords<TY, TZ>(A, blockIdx.x, tx, ty, tz)) return;
     line_tile<TY, TZ, KCULL, BEAM_OUT>(A, tx, ty, tz, wet, layers, geo, mu, dose, beam_dose, sh);
+}
+
+// The forward with each tile taken by a cluster of SPLIT blocks, which share
+// the tile's layers (block r every SPLIT-th kept layer) and add the layers'
+// doses in order, so that the dose is k_dose_line's bit for bit.
+template <int TY, int TZ, int KCULL, int SPLIT>
+__global__ void __cluster_dims__(SPLIT, 1, 1)
+__launch_bounds__(TY * TZ, line_min_blocks<TY * TZ>())
+k_dose_line_split(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
+                  const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
+                  const float *__restrict__ mu, float *__restrict__ dose)
+{
+    __shared__ LineShared<TY * TZ, KCULL, false, true, SPLIT> sh;
+    int tx, ty, tz;
+    // the same tile, and the same answer, in every block of the cluster
+    if (!line_tile_coords<TY, TZ>(A, blockIdx.x / SPLIT, tx, ty, tz)) return;
+    line_tile<TY, TZ, KCULL, false, kModeDose, SPLIT>(A, tx, ty, tz, wet, layers, geo, mu, dose,
+                                                      nullptr, sh, nullptr, nullptr, nullptr,
+                                                      (int)(blockIdx.x % SPLIT), SPLIT);
 }
 
 // Forward kernel variants the autotuner chooses from.  Two families:
@@ -1660,17 +2038,18 @@ k_dose_count_line(const __grid_constant__ PlanArgs A, const float *__restrict__ 
                                                               count, wfield);
 }
 
-__global__ void __launch_bounds__(kLineTY * kLineTZ, line_min_blocks<kLineTY * kLineTZ, true>())
+__global__ void __launch_bounds__(kLineTY * kLineTZ, line_min_blocks<kLineTY * kLineTZ>())
 k_adjoint_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
                const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
-               const float *__restrict__ wfield, float *__restrict__ grad)
+               const float *__restrict__ wfield, float *__restrict__ grad, int split)
 {
     __shared__ LineShared<kLineTY * kLineTZ, kLineCull, false, false> sh;
+    // each tile by `split` blocks, block r taking every split-th kept layer
     int tx, ty, tz;
-    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x, tx, ty, tz)) return;
-    line_tile<kLineTY, kLineTZ, kLineCull, false, kModeAdjoint>(A, tx, ty, tz, wet, layers, geo,
-                                                                nullptr, nullptr, nullptr, sh,
-                                                                nullptr, wfield, grad);
+    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / split, tx, ty, tz)) return;
+    line_tile<kLineTY, kLineTZ, kLineCull, false, kModeAdjoint>(
+        A, tx, ty, tz, wet, layers, geo, nullptr, nullptr, nullptr, sh, nullptr, wfield, grad,
+        (int)(blockIdx.x % split), split);
 }
 
 // ------------------------------------------------------------ tile order
@@ -1739,49 +2118,25 @@ k_tile_cost(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
     float c = 0.0f;
     for (int b = 0; b < A.n_beams; ++b) {
         const PbBeam &B = A.beams[b];
-        float dX, dY, dZ;
-        image_to_head(B.geom, A.g.spacing, 0.0f, 0.0f, dX, dY, dZ);
-        const float dgx = -__fdiv_rn(dZ, B.geom.vsadx), dgy = -__fdiv_rn(dZ, B.geom.vsady);
-        float v[12] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY,
-                       INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
+        float4 step;
+        TileBounds tb = corner_bounds(A.g, B, i0, ty * TY, tz * TZ, TY, TZ, lane, step);
+        float w0 = INFINITY, w1 = -INFINITY;
 #pragma unroll
         for (int m = 0; m < kLinesPerLane; ++m) {
             const int ln = lane + 32 * m;
             const int j = ty * TY + ln % TY, k = tz * TZ + ln / TY;
             const int nvalid = (j < A.g.ny && k < A.g.nz) ? min(kLine, A.g.nx - i0) : 0;
-            if (nvalid <= 0) continue;
-            const int64_t vbase = i0 + (int64_t)A.g.nx * (j + (int64_t)A.g.ny * k);
-            float px, py, pz, X0, Y0, Z0;
-            vox_mm(B.geom, A.g.spacing, i0, j, k, px, py, pz);
-            image_to_head(B.geom, px, py, pz, X0, Y0, Z0);
-            const float Xc = __fmaf_rn(3.5f, dX, X0), Yc = __fmaf_rn(3.5f, dY, Y0);
-            const float Zc = __fmaf_rn(3.5f, dZ, Z0);
-            const float gxc = __fsub_rn(1.0f, __fdiv_rn(Zc, B.geom.vsadx));
-            const float gyc = __fsub_rn(1.0f, __fdiv_rn(Zc, B.geom.vsady));
+            const float *p = wet + b * V + i0 + (int64_t)A.g.nx * (j + (int64_t)A.g.ny * k);
 #pragma unroll
             for (int q = 0; q < kLine; ++q) {
                 if (q >= nvalid) continue;
-                const float o = line_off(q);
-                const float X = __fmaf_rn(o, dX, Xc), Y = __fmaf_rn(o, dY, Yc);
-                const float Z = __fmaf_rn(o, dZ, Zc);
-                const float w = __fmul_rn(__ldg(wet + b * V + vbase + q), 10.0f);
-                const float dd = source_distance(B, X, Y, Z);
-                const float GX = __fmaf_rn(o, dgx, gxc), GY = __fmaf_rn(o, dgy, gyc);
-                v[0] = fminf(v[0], X);  v[1] = fmaxf(v[1], X);
-                v[2] = fminf(v[2], Y);  v[3] = fmaxf(v[3], Y);
-                v[4] = fminf(v[4], GX); v[5] = fmaxf(v[5], GX);
-                v[6] = fminf(v[6], GY); v[7] = fmaxf(v[7], GY);
-                v[8] = fminf(v[8], dd); v[9] = fmaxf(v[9], dd);
-                v[10] = fminf(v[10], w == w ? w : -INFINITY);
-                v[11] = fmaxf(v[11], w == w ? w : INFINITY);
+                const float w = __fmul_rn(__ldg(p + q), 10.0f);
+                w0 = fminf(w0, w == w ? w : -INFINITY);
+                w1 = fmaxf(w1, w == w ? w : INFINITY);
             }
         }
-#pragma unroll
-        for (int m = 0; m < 12; ++m) v[m] = (m & 1) ? warp_max(v[m]) : warp_min(v[m]);
-        TileBounds tb;
-        tb.x0 = v[0]; tb.x1 = v[1]; tb.y0 = v[2]; tb.y1 = v[3];
-        tb.gx0 = v[4]; tb.gx1 = v[5]; tb.gy0 = v[6]; tb.gy1 = v[7];
-        tb.d0 = v[8]; tb.d1 = v[9]; tb.w0 = v[10]; tb.w1 = v[11];
+        tb.w0 = warp_min(w0);
+        tb.w1 = warp_max(w1);
         for (int l = lane; l < B.n_layers; l += 32)
             c += layer_pair_cost(layers[B.layer_start + l], tb, B);
     }
@@ -2229,7 +2584,7 @@ static void launch_line_t(const PlanArgs &A, const float *wet, const PbLayer *la
 PbStatus launch_dose(const PbGrid &g, const PbBeam *beams, int n_beams,
                      const float *wet, const PbLayer *layers, const float *geo,
                      const float *mu, float scale, float *dose, float *beam_dose,
-                     cudaStream_t st, int variant, const int *order)
+                     cudaStream_t st, int variant, const int *order, int split)
 {
     PlanArgs A;
     fill_args(A, g, beams, n_beams, scale);
@@ -2253,7 +2608,16 @@ PbStatus launch_dose(const PbGrid &g, const PbBeam *beams, int n_beams,
     case 1: launch_line_t<8, 8, 4>(A, wet, layers, g4, mu, dose, st); break;
     case 2: launch_line_t<8, 4, 4>(A, wet, layers, g4, mu, dose, st); break;
     case 3: launch_line_t<4, 8, 4>(A, wet, layers, g4, mu, dose, st); break;
-    case 4: launch_line_t<16, 8, 2>(A, wet, layers, g4, mu, dose, st); break;
+    case 4:
+        if (split == 4)
+            k_dose_line_split<16, 8, 2, 4><<<line_tiles(g, 16, 8) * 4, 128, 0, st>>>(
+                A, wet, layers, g4, mu, dose);
+        else if (split == 2)
+            k_dose_line_split<16, 8, 2, 2><<<line_tiles(g, 16, 8) * 2, 128, 0, st>>>(
+                A, wet, layers, g4, mu, dose);
+        else
+            launch_line_t<16, 8, 2>(A, wet, layers, g4, mu, dose, st);
+        break;
     case 5: launch_line_t<8, 16, 2>(A, wet, layers, g4, mu, dose, st); break;
     case 6: launch_dose_t<128, 4, 1>(A, tiles, wet, layers, g4, mu, dose, st); break;
     case 7: launch_dose_t<128, 4, 2>(A, tiles, wet, layers, g4, mu, dose, st); break;
@@ -2318,7 +2682,7 @@ int dose_variant_threads(int variant)
 PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
                         const float *wet, const PbLayer *layers, const float *geo,
                         const float *w, float scale, float *grad, cudaStream_t st,
-                        int variant, const int *order)
+                        int variant, const int *order, int split)
 {
     PlanArgs A;
     fill_args(A, g, beams, n_beams, scale);
@@ -2334,8 +2698,8 @@ PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
     const int64_t tiles = (int64_t)A.tiles_x * A.tiles_y * A.tiles_z;
     const float4 *g4 = reinterpret_cast<const float4 *>(geo);
     if (variant_line(variant)) {
-        k_adjoint_line<<<line_tiles(g, kLineTY, kLineTZ), kLineTY * kLineTZ, 0, st>>>(
-            A, wet, layers, g4, w, grad);
+        k_adjoint_line<<<line_tiles(g, kLineTY, kLineTZ) * split, kLineTY * kLineTZ, 0, st>>>(
+            A, wet, layers, g4, w, grad, split);
         return check_launch("k_adjoint_line");
     }
     k_adjoint_tile<<<(unsigned)tiles, 128, 0, st>>>(A, wet, layers, g4, w, grad);
@@ -2403,6 +2767,62 @@ void tile_order_tile(int *voxels)
     voxels[0] = kLine;
     voxels[1] = kLineTY;
     voxels[2] = kLineTZ;
+}
+
+// Blocks per tile.  A tile that the beams reach keeps its block busy for tens
+// of microseconds (a warp per scheduler, one layer after the other), so a plan
+// with fewer such tiles than the GPU has places for blocks (148 SMs x 4) ends
+// on that latency while SMs idle; sharing each tile's layers among 2 or 4
+// blocks then shortens it, at the price of setting the tile up in each.  The
+// lines measured (microseconds, forward / adjoint, 1, 2 and 4 blocks):
+//     96 tiles reached   56, 40, 34 / 64, 39, 35
+//    455                417, 289, 235 / 549, 336, 229
+//    540                190, 149, 183 / 244, 157, 165
+//    561                787, 521, 504 / 951, 571, 493
+//    702                365, 345, 362 / 350, 239, 165
+//   1232                269, 284, 353 / 295, 284, 334
+//   1412                306, 324, 384 / 346, 344, 384
+// The adjoint has no exchange between the blocks and skips tiles where its
+// field is zero, so it gains up to a larger count.  The tiles reached are
+// estimated from the beams' spot boxes: a tile counts when its centre lies
+// within 60 mm (where the widest halo falls below 2^-24) and half a tile's
+// width of a beam's box of spot axes.
+constexpr int kSplitMaxTiles = 4096;   // larger grids are not looked at
+
+void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                int *forward, int *adjoint)
+{
+    *forward = *adjoint = 1;
+    const int ntx = (g.nx + kLine - 1) / kLine, nty = (g.ny + kLineTY - 1) / kLineTY;
+    const int ntz = (g.nz + kLineTZ - 1) / kLineTZ;
+    if ((long long)ntx * nty * ntz > kSplitMaxTiles) return;
+    const float reach = 60.0f + 0.5f * kLine * g.spacing;
+    int active = 0;
+    for (int z = 0; z < ntz; ++z)
+        for (int y = 0; y < nty; ++y)
+            for (int x = 0; x < ntx; ++x) {
+                bool in = false;
+                for (int b = 0; b < n_beams && !in; ++b) {
+                    const PbBeamGeom &B = beams[b].geom;
+                    const float *q = spot_boxes + 4 * b;
+                    if (!(q[0] <= q[1] && q[2] <= q[3])) continue;   // no spots
+                    const float px = (kLine * (x + 0.5f) - 0.5f) * g.spacing - B.iso[0];
+                    const float py = (kLineTY * (y + 0.5f) - 0.5f) * g.spacing - B.iso[1];
+                    const float pz = (kLineTZ * (z + 0.5f) - 0.5f) * g.spacing - B.iso[2];
+                    const float xt = px * B.costa - pz * B.sinta;
+                    const float hy = px * B.sinta + pz * B.costa;
+                    const float hx = -(xt * B.cosga + py * B.singa);
+                    const float hz = py * B.cosga - xt * B.singa;
+                    const float gx = 1.0f - hz / B.vsadx, gy = 1.0f - hz / B.vsady;
+                    in = hx > fminf(q[0] * gx, q[1] * gx) - reach &&
+                         hx < fmaxf(q[0] * gx, q[1] * gx) + reach &&
+                         hy > fminf(q[2] * gy, q[3] * gy) - reach &&
+                         hy < fmaxf(q[2] * gy, q[3] * gy) + reach;
+                }
+                active += in;
+            }
+    *forward = active < 500 ? 4 : active < 900 ? 2 : 1;
+    *adjoint = active < 900 ? 4 : active < 1500 ? 2 : 1;
 }
 
 size_t tile_order_work_size(const PbGrid &g)

@@ -64,7 +64,7 @@ PbStatus launch_dose(const PbGrid &g, const PbBeam *beams, int n_beams,
                      const float *wet, const PbLayer *layers,
                      const float *geo, const float *mu, float scale,
                      float *dose, float *beam_dose, cudaStream_t st, int variant = -1,
-                     const int *order = nullptr);
+                     const int *order = nullptr, int split = 1);
 
 // variant < 0 selects the default forward shape (dose_variant_default);
 // the adjoint and the operation count use the kernel family of `variant`.
@@ -88,10 +88,13 @@ PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
                         const float *wet, const PbLayer *layers,
                         const float *geo, const float *w, float scale,
                         float *grad, cudaStream_t st, int variant = -1,
-                        const int *order = nullptr);
+                        const int *order = nullptr, int split = 1);
 long long tile_order_count(const PbGrid &g);
 void tile_order_tile(int *voxels);
 size_t tile_order_work_size(const PbGrid &g);
+// Blocks per tile for the forward and the adjoint (pb_tile_split).
+void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                int *forward, int *adjoint);
 PbStatus launch_tile_order(const PbGrid &g, const PbBeam *beams, int n_beams, const float *wet,
                            const PbLayer *layers, void *work, int *order, cudaStream_t st);
 

@@ -147,6 +147,12 @@ _SIGS = {
                              _VP, _VP, _VP, _VP]),
     "pb_dose_adjoint_ordered": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP,
                                      ctypes.c_float, _VP, _VP, _VP]),
+    "pb_tile_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, ctypes.POINTER(_I),
+                           ctypes.POINTER(_I)]),
+    "pb_dose_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _F, _VP, _VP, _I,
+                           _VP]),
+    "pb_dose_adjoint_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _F, _VP,
+                                   _VP, _I, _VP]),
     "pb_count_evaluated_adjoint": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP,
                                         ctypes.c_float, _VP, _VP]),
     "pb_measure_ex2_rate": (_I, [ctypes.POINTER(ctypes.c_double), _VP]),

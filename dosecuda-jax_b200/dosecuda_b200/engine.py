@@ -268,12 +268,26 @@ class DevicePlan:
             B.n_energies = t.n_energies
             B.lut_len = t.lut_len
             B.dvp_len = t.dvp_len
+        # blocks per tile of the plan's launches and of each beam's own
+        boxes = np.array([(g[:, 0].min(), g[:, 0].max(), g[:, 1].min(), g[:, 1].max()) if len(g)
+                          else (1.0, -1.0, 1.0, -1.0) for g in geo_blocks], np.float32)
+        self._split, self._split_adjoint = self._tile_split(0, self.n_beams, boxes)
+        self._beam_split = [self._tile_split(b, 1, boxes)[0] for b in range(self.n_beams)]
         # per-layer culling bounds (spot box, halo and MCS sigma bounds) on the device
         if self.layer_offsets[-1]:
             check(_lib.lib.pb_layer_bounds(ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
                                            ptr(self.layers), ptr(self.spot_geo),
                                            _stream(self.device)), "pb_layer_bounds")
         self.spots_loaded = True
+
+    def _tile_split(self, b0: int, n: int, boxes: np.ndarray):
+        """(forward, adjoint) blocks per tile of a launch over beams
+        b0 .. b0 + n - 1 (pb_tile_split); boxes: each beam's spot box."""
+        fwd, adj = ctypes.c_int(1), ctypes.c_int(1)
+        q = np.ascontiguousarray(boxes[b0:b0 + n])
+        check(_lib.lib.pb_tile_split(ctypes.byref(self.grid), self._beam_ptr(b0), n, ptr(q),
+                                     ctypes.byref(fwd), ctypes.byref(adj)), "pb_tile_split")
+        return fwd.value, adj.value
 
     def __del__(self):
         if not getattr(self, "_owns_textures", True):
@@ -409,12 +423,18 @@ class DevicePlan:
         bd = torch.empty((self.n_beams, self.n_vox), dtype=torch.float32,
                          device=self.device) if beam_doses else None
         order = self.tile_order()
-        check(_lib.lib.pb_dose_ordered(ctypes.byref(self.grid),
-                                       ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
-                                       ptr(self.wet), ptr(self.layers), ptr(self.spot_geo),
-                                       ptr(mu), float(scale), ptr(dose), ptr(bd), ptr(order),
-                                       _stream(self.device)), "pb_dose_ordered")
-        return (dose, bd) if beam_doses else dose
+        beams = ctypes.cast(self.beams, ctypes.c_void_p)
+        if beam_doses:
+            check(_lib.lib.pb_dose_ordered(ctypes.byref(self.grid), beams, self.n_beams,
+                                           ptr(self.wet), ptr(self.layers), ptr(self.spot_geo),
+                                           ptr(mu), float(scale), ptr(dose), ptr(bd), ptr(order),
+                                           _stream(self.device)), "pb_dose_ordered")
+            return dose, bd
+        check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), beams, self.n_beams, ptr(self.wet),
+                                     ptr(self.layers), ptr(self.spot_geo), ptr(mu), float(scale),
+                                     ptr(dose), ptr(order), self._split, _stream(self.device)),
+              "pb_dose_split")
+        return dose
 
     def beam_tile_order_parts(self, b: int, n_parts: int):
         """Beam b's tile order split into up to n_parts groups of whole z
@@ -450,10 +470,11 @@ class DevicePlan:
                                                        device=self.device)
         if dose.numel() != self.n_vox or not dose.is_contiguous():
             raise ValueError("out must be a contiguous tensor of V floats")
-        check(_lib.lib.pb_dose_ordered(ctypes.byref(self.grid), self._beam_ptr(b), 1,
-                                       ptr(self.wet[b]), ptr(self.layers), ptr(self.spot_geo),
-                                       ptr(mu), float(scale), ptr(dose), None, ptr(order),
-                                       _stream(self.device)), "pb_dose_ordered")
+        check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), self._beam_ptr(b), 1,
+                                     ptr(self.wet[b]), ptr(self.layers), ptr(self.spot_geo),
+                                     ptr(mu), float(scale), ptr(dose), ptr(order),
+                                     self._beam_split[b], _stream(self.device)),
+              "pb_dose_split")
         return dose
 
     def forward_variant(self, variant: int, mu_sorted: Optional[torch.Tensor] = None,
@@ -484,10 +505,11 @@ class DevicePlan:
                                                        device=self.device)
         if variant is None:
             order = self.tile_order()
-            check(_lib.lib.pb_dose_adjoint_ordered(
+            check(_lib.lib.pb_dose_adjoint_split(
                 ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
                 ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(w), float(scale),
-                ptr(grad), ptr(order), _stream(self.device)), "pb_dose_adjoint_ordered")
+                ptr(grad), ptr(order), self._split_adjoint, _stream(self.device)),
+                "pb_dose_adjoint_split")
         else:
             check(_lib.lib.pb_dose_adjoint_variant(
                 ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,

@@ -383,6 +383,27 @@ PbStatus pb_dose_adjoint_ordered(const PbGrid *grid, const PbBeam *beams, int n_
                                  float scale, float *grad_dev, const int *order_dev,
                                  void *stream);
 
+/* Blocks per tile for pb_dose_split and pb_dose_adjoint_split (1, 2 or 4),
+ * from how many tiles the beams reach: where those are fewer than the GPU
+ * has places for blocks, sharing a tile's layers among several blocks
+ * shortens the launch.  Host only.  spot_boxes: per beam the least and
+ * greatest spot x, then y, at the isocentre plane (mm; least > greatest for
+ * a beam without spots).  No counterpart in the reference. */
+PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                       const float *spot_boxes, int *forward_out, int *adjoint_out);
+/* pb_dose_ordered (without per-beam doses) and pb_dose_adjoint_ordered with
+ * each tile of the default shape shared by `split` blocks (1, 2 or 4).  The
+ * dose is the same bits for every split, the gradient the same to float
+ * rounding (the order of its atomic sums). */
+PbStatus pb_dose_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                       const float *wet_dev, const PbLayer *layers_dev,
+                       const float *spot_geo_dev, const float *mu_dev, float scale,
+                       float *dose_dev, const int *order_dev, int split, void *stream);
+PbStatus pb_dose_adjoint_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                               const float *wet_dev, const PbLayer *layers_dev,
+                               const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
+                               float *grad_dev, const int *order_dev, int split, void *stream);
+
 /* Adjoint of pb_dose: grad_dev[s] = scale * sum_v dobj_dose_dev[v] * K(v,s)
  * for every spot s, where K(v,s) is the dose per unit weight of spot s at
  * voxel v.  Matrix-free: footprints are recomputed.  grad_dev is
