@@ -264,6 +264,19 @@ PbStatus pb_texture_update(PbTexture tex, const float *rlsp_dev, void *stream)
     return texture_update(tex, rlsp_dev, static_cast<cudaStream_t>(stream));
 }
 
+PbStatus pb_texture_sample(PbTexture tex, const PbGrid *grid, const float *at_dev, int64_t pairs,
+                           float *unit_dev, float *cells_dev, void *stream)
+{
+    PbStatus s = check_grid(grid);
+    if (s != PB_OK) return s;
+    if (!tex || !at_dev || !unit_dev || !cells_dev || pairs < 0 || pairs > INT_MAX)
+        return set_error(PB_ERR_INVALID, "NULL argument or count");
+    if (!texture_matches(tex, *grid) || !texture_samples(tex) || !texture_cells(tex).quad)
+        return set_error(PB_ERR_INVALID, "not a texture with cell records of this grid");
+    return launch_texture_sample(texture_object(tex), texture_cells(tex), *grid, at_dev, pairs,
+                                 unit_dev, cells_dev, static_cast<cudaStream_t>(stream));
+}
+
 PbStatus pb_texture_destroy(PbTexture tex)
 {
     texture_destroy(tex);

@@ -34,9 +34,21 @@ PbStatus launch_rlsp(const float *hu, int64_t n, const double *xh,
 PbStatus check_wet_args(const float *rlsp_dev, uint64_t tex, const PbGrid *grid,
                         const PbBeamGeom *beams, int n_beams, const float *wet_dev);
 
-PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const float2 *rec,
+// Cell records of an RLSP volume (pb_wet.cu); null: none.
+struct RayCells {
+    const float4 *quad;
+    const unsigned char *dist;
+    const unsigned int *odd;
+    const float2 *cell;
+};
+
+PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &rec,
                     const PbGrid &g, const PbBeamGeom *beams, int n_beams, float *raw,
                     float *wet, int *status, cudaStream_t st);
+
+PbStatus launch_texture_sample(cudaTextureObject_t tex, const RayCells &rec, const PbGrid &g,
+                               const float *at, int64_t pairs, float *unit, float *cells,
+                               cudaStream_t st);
 
 // Batched WET pass (pb_wet.cu): one record per (plan, beam).
 // The smoothing sample table of one beam (pb_wet.cu), as the WET launch
@@ -47,7 +59,7 @@ void smooth_table_host(const PbGrid &g, const PbBeamGeom *beams, int n_beams, in
 size_t batch_wet_size();
 long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbBeamGeom *beams,
                          int n_beams, const float *rlsp, cudaTextureObject_t tex,
-                         const float2 *rec, float *raw, float *wet, long long brick_start);
+                         const RayCells &rec, float *raw, float *wet, long long brick_start);
 PbStatus launch_wet_batch(const void *items_dev, int n_items, long long n_bricks, int *status,
                           cudaStream_t st);
 
@@ -57,7 +69,7 @@ bool texture_samples(uint64_t h);   // a texture (not a records-only handle)
 PbStatus texture_update(uint64_t h, const float *rlsp, cudaStream_t st);
 bool texture_matches(uint64_t h, const PbGrid &g);
 cudaTextureObject_t texture_object(uint64_t h);
-const float2 *texture_cells(uint64_t h);
+RayCells texture_cells(uint64_t h);
 void texture_destroy(uint64_t h);
 
 PbStatus launch_dose(const PbGrid &g, const PbBeam *beams, int n_beams,

@@ -144,30 +144,40 @@ PbStatus pb_rlsp_from_hu(const float *hu_dev, int64_t n, const double *curve_hu,
  * unit's filter weights are fixed point, so samples through it differ
  * slightly from exact trilinear interpolation; the reference's WET is
  * defined by them.  Creating one allocates a CUDA array.  The handle also
- * holds per-cell records (whether each 2x2x2 block of texels is flat, and
- * how far the nearest non-flat one is) from which pb_wet adds whole runs of
- * samples through flat regions at once. */
+ * holds per-cell records (the texels of each 2x2x2 block, and how far the
+ * nearest block is whose texels differ) from which pb_wet adds whole runs of
+ * samples through flat regions at once and forms the other samples with the
+ * unit's filter (pb_texture_sample compares the two).  They take 27 bytes per
+ * voxel (19 without a texture); a grid that leaves no memory for them, or with
+ * more than 8191 voxels along an axis, is sampled through the unit alone. */
 typedef uint64_t PbTexture;
 
 PbStatus pb_texture_create(const float *rlsp_dev, const PbGrid *grid,
                            PbTexture *tex_out, void *stream);
 /* A handle with the cell records only (no texture, no CUDA array), for
- * exact-trilinear WET with the same runs through flat regions.  No
- * counterpart in the reference. */
+ * exact-trilinear WET with the same runs through flat regions and its
+ * samples from the records.  No counterpart in the reference. */
 PbStatus pb_cells_create(const float *rlsp_dev, const PbGrid *grid, PbTexture *cells_out,
                          void *stream);
 /* Refill an existing handle (either kind) from a volume of the same grid. */
 PbStatus pb_texture_update(PbTexture tex, const float *rlsp_dev, void *stream);
 PbStatus pb_texture_destroy(PbTexture tex);
+/* Check of the cell records' filter against the texture unit: samples at
+ * 2 x pairs coordinates (x, y, z each, unnormalised), through the unit into
+ * unit_dev and from the records, as pb_wet takes them, into cells_dev; 0
+ * where a coordinate is nearer than 0.003 to the grid's faces or outside.
+ * No counterpart in the reference. */
+PbStatus pb_texture_sample(PbTexture tex, const PbGrid *grid, const float *at_dev, int64_t pairs,
+                           float *unit_dev, float *cells_dev, void *stream);
 
 /* WET (cm) of every voxel for n_beams beams: the ray trace toward the
  * source (CudaClasses.cu:180-228, accumulated in FP64) followed by the
  * lateral smoothing (IMPTClasses.cu:139-202).
  *   tex from pb_texture_create: RLSP is sampled through the texture (the
  *             reference's samples); rlsp_dev is not read and may be NULL.
- *   tex from pb_cells_create, or 0: RLSP is read from rlsp_dev with exact
- *             FP32 trilinear weights (border 0); with the records, runs
- *             through flat cells are added at once.
+ *   tex from pb_cells_create, or 0: exact FP32 trilinear weights (border 0),
+ *             RLSP from rlsp_dev and, where there are records, from those of
+ *             the same volume; runs through flat cells are added at once.
  * raw_work_dev and wet_dev hold n_beams x V floats; raw_work_dev receives
  * the unsmoothed WET.  status_dev (nullable) is one device int that is
  * OR-ed with PB_ERR_RAY_CAP if a ray reaches its step cap. */

@@ -1,0 +1,138 @@
+"""The ray trace's samples from the cell records.
+
+With the texture unit's filter: compared with the unit itself over random
+coordinates, over every pair of fractions of two axes, and at the halves of the
+coordinates' 1/256 steps and of the weights, with volumes of one texel (each
+weight by itself) and of noise.  Both sum at most eight products of a weight
+(whole 256ths) and a texel in FP32: 8 roundings of the largest texel.
+
+With exact weights: the depths of a noisy volume with and without the
+records, whose samples are the same FP32 operations (sums of 4 and of 8 samples
+before FP64: 1e-6 of the largest depth)."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import cuda_available
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+DEV = torch.device("cuda", 0)
+
+
+def _samples(vol, at):
+    """(unit, cells) of the volume (nz, ny, nx) at the coordinates (n, 3)."""
+    from dosecuda_b200 import _lib
+    nz, ny, nx = vol.shape
+    g = _lib.PbGrid(nx, ny, nz, 1.0)
+    h = ctypes.c_uint64(0)
+    stream = ctypes.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)
+    v = torch.as_tensor(vol, device=DEV).contiguous()
+    _lib.check(_lib.lib.pb_texture_create(_lib.ptr(v), ctypes.byref(g), ctypes.byref(h), stream))
+    try:
+        a = torch.as_tensor(at, dtype=torch.float32, device=DEV).contiguous()
+        assert len(a) % 2 == 0
+        unit, cells = torch.empty(len(a), device=DEV), torch.empty(len(a), device=DEV)
+        _lib.check(_lib.lib.pb_texture_sample(h, ctypes.byref(g), _lib.ptr(a), len(a) // 2,
+                                              _lib.ptr(unit), _lib.ptr(cells), stream))
+        torch.cuda.synchronize()
+    finally:
+        _lib.lib.pb_texture_destroy(h)
+    return unit.cpu().numpy(), cells.cpu().numpy()
+
+
+BOUND = 8.0 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("shape", [(24, 31, 40), (1, 5, 7), (3, 2, 1)])
+def test_filter_is_the_units(shape):
+    rng = np.random.default_rng(5)
+    vol = rng.uniform(0.0, 2.0, shape).astype(np.float32)
+    n = np.array(shape[::-1], np.float64)
+    at = rng.uniform(0.0, 1.0, (1 << 18, 3)) * n
+    at[::3] = np.floor(at[::3] * 1024.0) / 1024.0   # among them the halves of 1/256
+    unit, cells = _samples(vol, at.astype(np.float32))
+    assert unit.max() > 0.5
+    assert np.abs(unit - cells).max() <= BOUND * vol.max()
+
+
+def test_weights_of_every_texel():
+    """One texel of 1: the sample is that texel's weight, a whole 256th."""
+    vol = np.zeros((8, 8, 8), np.float32)
+    vol[4, 4, 4] = 1.0
+    f = np.arange(256) / 256.0
+    rng = np.random.default_rng(2)
+    for axes in ((0, 1), (0, 2), (1, 2)):
+        for corner in range(8):
+            at = np.empty((256 * 256, 3))
+            for a in range(3):
+                part = rng.integers(0, 256) / 256.0
+                if a == axes[0]:
+                    part = np.repeat(f, 256)
+                elif a == axes[1]:
+                    part = np.tile(f, 256)
+                at[:, a] = 4.0 - ((corner >> a) & 1) + 0.5 + part
+            unit, cells = _samples(vol, at)
+            assert np.array_equal(unit, cells)
+            assert np.array_equal(unit * 256.0, np.round(unit * 256.0))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_not_a_number_and_infinite_texels(value):
+    """The unit leaves out texels of weight 0, so a volume with such a value is
+    sampled by the unit: the depths are those of the handle whose other texels
+    are finite, wherever the ray does not come near it, and no ray that passes
+    it loses a sample that the unit has."""
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_impt import IMPTPlan
+    shape = (14, 16, 18)
+    rng = np.random.default_rng(8)
+    vol = rng.uniform(0.5, 1.5, shape).astype(np.float32)
+    spots = np.array([[0.0, 0.0, 1.0, 30.0]], np.float32)
+    iso = np.array([18.0, 16.0, 14.0], np.float32)
+    dp = engine.DevicePlan(shape, 2.0, np.zeros(3, np.float32),
+                           [engine.BeamSpec(0.0, 0.0, iso, spots, IMPTPlan().beam_models[0])], DEV)
+
+    def raw(v):
+        dp.compute_wet(torch.as_tensor(v, device=DEV).reshape(-1))
+        return dp.raw_wet.clone().reshape(shape)
+    clean = raw(vol)
+    vol[7, 8, 9] = value
+    other = raw(vol)
+    far = torch.ones(shape, dtype=torch.bool, device=DEV)
+    far[5:10, :, 7:12] = False
+    assert torch.allclose(other[far], clean[far], rtol=2e-6, atol=1e-6)
+    assert not torch.equal(torch.nan_to_num(other), torch.nan_to_num(clean))
+    vol[7, 8, 9] = 1.0
+    raw(vol)
+    assert bool(torch.isfinite(dp.raw_wet).all())
+
+
+@pytest.mark.parametrize("shape,spacing,angle,couch", [
+    ((24, 30, 37), 2.5, 31.0, 12.0), ((19, 40, 33), 1.0, 0.0, 0.0), ((40, 9, 64), 3.0, 270.0, 0.0)])
+@pytest.mark.parametrize("noise", [0.0, 0.02])
+def test_exact_depths_with_and_without_records(shape, spacing, angle, couch, noise):
+    from dosecuda_b200 import _lib, engine
+    from dosecuda_b200.plan_impt import IMPTPlan
+    rng = np.random.default_rng(3)
+    rho = np.ones(shape, np.float32)
+    rho[:, : shape[1] // 3] = 0.25
+    rho += (noise * rng.standard_normal(shape)).astype(np.float32)
+    iso = 0.47 * spacing * np.array(shape[::-1], np.float32)
+    spots = np.array([[0.0, 0.0, 1.0, 30.0]], np.float32)
+    dp = engine.DevicePlan(shape, spacing, np.zeros(3, np.float32),
+                           [engine.BeamSpec(angle, couch, iso, spots, IMPTPlan().beam_models[0])],
+                           DEV)
+    v = torch.as_tensor(rho, device=DEV).reshape(-1).contiguous()
+    dp.compute_wet(v, wet_mode="exact")
+    with_records = dp.raw_wet.clone()
+    raw, wet = torch.empty_like(with_records), torch.empty_like(with_records)
+    _lib.check(_lib.lib.pb_wet(_lib.ptr(v), 0, ctypes.byref(dp.grid),
+                               ctypes.cast(dp.geoms, ctypes.c_void_p), 1, _lib.ptr(raw),
+                               _lib.ptr(wet), None,
+                               ctypes.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)))
+    assert float(raw.max()) > 1.0
+    assert float((raw - with_records).abs().max()) <= 1e-6 * float(raw.max())
