@@ -602,98 +602,6 @@ __device__ __forceinline__ float warp_sum_n(float (&v)[N], int lane, int &slot)
     return t;
 }
 
-// Spot-position derivatives of the adjoint sums.  With q = |t x ray|^2 *
-// it2 the scaled squared axis distance (axis_r2), the spot's factor at a
-// voxel is mu (Pf 2^(ps2 q) + Hf 2^(hs2 q)), so
-//   d/dxs = mu ln2 (Pf ps2 e1 + Hf hs2 e2) dq/dxs,
-// and from ax = X - xs gx, ay = Y - ys gy, cz = (xs/VSADX) Y - (ys/VSADY) X
-// - xs ys k (k = 1/VSADX - 1/VSADY), it2 = 1/(1 + xs^2/VSADX^2 + ys^2/VSADY^2):
-//   dq/dxs = 2 it2 (-ax gx + cz (Y/VSADX - ys k) - q xs/VSADX^2)
-//   dq/dys = 2 it2 (-ay gy + cz (-X/VSADY - xs k) - q ys/VSADY^2).
-// The voxel sums of wv (Pf ps2 e1 + Hf hs2 e2) ln2 times the bracket meet as
-// in the weight adjoint; the spot's factor mu * 2 * it2 is applied when they
-// go to grad_x, grad_y.  The weight gradient is formed alongside (grad may
-// be NULL).
-template <int NT, int NP, int KCAP>
-__device__ __forceinline__ void adjoint_positions(const SpotRec *s_spot, float *gsum,
-                                                  float *gsum_x, float *gsum_y, int n2, int n1,
-                                                  const PbBeam &B, const float2 *XP,
-                                                  const float2 *YP, const float2 *GXP,
-                                                  const float2 *GYP, const float2 *PS,
-                                                  const float2 *HS, const float2 *FP,
-                                                  const float2 *FH, const float2 *FPd,
-                                                  const float2 *FHd, int lane,
-                                                  const float *__restrict__ mu,
-                                                  float *__restrict__ grad,
-                                                  float *__restrict__ grad_x,
-                                                  float *__restrict__ grad_y)
-{
-    const float ivx = __fdiv_rn(1.0f, B.geom.vsadx), ivy = __fdiv_rn(1.0f, B.geom.vsady);
-    const float kap = __fsub_rn(ivx, ivy);
-    const float ivx2 = __fmul_rn(ivx, ivx), ivy2 = __fmul_rn(ivy, ivy);
-    for (int cls = 0; cls < 2; ++cls) {
-        const int lo = cls == 0 ? 0 : KCAP - n1, hi = cls == 0 ? n2 : KCAP;
-        for (int c0 = lo; c0 < hi; c0 += 8) {
-            float v[8], vx[8], vy[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const SpotRec r = s_spot[c0 + k];
-                const float xs = -r.a.x, ys = -r.a.z;
-                const float2 kx2 = f2(-__fmul_rn(xs, ivx2)), ky2 = f2(-__fmul_rn(ys, ivy2));
-                const float2 ckx = f2(-__fmul_rn(ys, kap)), cky = f2(-__fmul_rn(xs, kap));
-                float2 t = make_float2(0.0f, 0.0f), ux = t, uy = t;
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const float2 ax = __ffma2_rn(lo2(r.a), GXP[p], XP[p]);
-                    const float2 ay = __ffma2_rn(hi2(r.a), GYP[p], YP[p]);
-                    const float2 cz = __ffma2_rn(lo2(r.b), YP[p], __ffma2_rn(hi2(r.b), XP[p],
-                                                                            lo2(r.c)));
-                    const float2 S = __ffma2_rn(ax, ax, __ffma2_rn(ay, ay, __fmul2_rn(cz, cz)));
-                    const float2 qq = __fmul2_rn(S, hi2(r.c));
-                    const float2 e2 = ex2x2(__fmul2_rn(HS[p], qq));
-                    t = __ffma2_rn(FH[p], e2, t);
-                    float2 u = __fmul2_rn(FHd[p], e2);
-                    if (cls == 0) {
-                        const float2 e1 = ex2x2(__fmul2_rn(PS[p], qq));
-                        t = __ffma2_rn(FP[p], e1, t);
-                        u = __ffma2_rn(FPd[p], e1, u);
-                    }
-                    float2 bx = __ffma2_rn(cz, __ffma2_rn(YP[p], f2(ivx), ckx),
-                                           __fmul2_rn(ax, __fmul2_rn(GXP[p], f2(-1.0f))));
-                    bx = __ffma2_rn(qq, kx2, bx);
-                    float2 by = __ffma2_rn(cz, __ffma2_rn(XP[p], f2(-ivy), cky),
-                                           __fmul2_rn(ay, __fmul2_rn(GYP[p], f2(-1.0f))));
-                    by = __ffma2_rn(qq, ky2, by);
-                    ux = __ffma2_rn(u, bx, ux);
-                    uy = __ffma2_rn(u, by, uy);
-                }
-                v[k] = t.x + t.y;
-                vx[k] = ux.x + ux.y;
-                vy[k] = uy.x + uy.y;
-            }
-            int slot;
-            const float sum = warp_sum8(v, lane, slot);
-            const float sx = warp_sum8(vx, lane, slot);
-            const float sy = warp_sum8(vy, lane, slot);
-            if ((lane & 3) == 0 && c0 + slot < hi) {
-                if (sum != 0.0f) atomicAdd(&gsum[c0 + slot], sum);
-                if (sx != 0.0f) atomicAdd(&gsum_x[c0 + slot], sx);
-                if (sy != 0.0f) atomicAdd(&gsum_y[c0 + slot], sy);
-            }
-        }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < n2 + n1; c += NT) {
-        const int sl = c < n2 ? c : KCAP - n1 + (c - n2);
-        const int si = __float_as_int(s_spot[sl].d.x);
-        const float f = __fmul_rn(__fmul_rn(2.0f, s_spot[sl].c.z), __ldg(mu + si));
-        if (grad && gsum[sl] != 0.0f) atomicAdd(grad + si, gsum[sl]);
-        if (gsum_x[sl] != 0.0f) atomicAdd(grad_x + si, __fmul_rn(gsum_x[sl], f));
-        if (gsum_y[sl] != 0.0f) atomicAdd(grad_y + si, __fmul_rn(gsum_y[sl], f));
-        gsum[sl] = gsum_x[sl] = gsum_y[sl] = 0.0f;
-    }
-}
-
 // One 8x8x8 tile of one plan by one block of NT threads, VPT = 512 / NT
 // voxels per thread; spots are culled KCULL per thread per compaction round.
 //   kModeDose     the dose (BEAM_OUT: also each beam's dose)
@@ -702,9 +610,6 @@ __device__ __forceinline__ void adjoint_positions(const SpotRec *s_spot, float *
 //                 and to count[1] the spot-voxel evaluations the forward
 //                 issues (each surviving spot against the tile's 512 voxel
 //                 slots); no dose
-//   kModeAdjointPos  as kModeAdjoint (grad may be NULL), and also the
-//                 derivatives with respect to the spot's position at the
-//                 isocentre plane into grad_x, grad_y (see below)
 //   kModeAdjoint  grad[spot] += scale * sum over the tile's voxels of
 //                 wfield[v] * d dose[v] / d mu[spot], with the voxels where
 //                 wfield is 0 inactive.  Each thread evaluates its voxels
@@ -722,14 +627,10 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
                                           DoseShared<NT, KCULL> &sh,
                                           unsigned long long *count = nullptr,
                                           const float *__restrict__ wfield = nullptr,
-                                          float *__restrict__ grad = nullptr,
-                                          float *__restrict__ grad_x = nullptr,
-                                          float *__restrict__ grad_y = nullptr,
-                                          float *gsum_xy = nullptr)
+                                          float *__restrict__ grad = nullptr)
 {
-    constexpr bool POS = MODE == kModeAdjointPos;
     constexpr bool COUNT = MODE == kModeCount;
-    constexpr bool ADJ = MODE == kModeAdjoint || POS;
+    constexpr bool ADJ = MODE == kModeAdjoint;
     unsigned long long n_ex2 = 0, n_eval = 0;
     static_assert(NT * VPT == 512, "a block covers one 8x8x8 tile");
     constexpr int kVpt = VPT;
@@ -764,9 +665,6 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
         }
         if (!__syncthreads_or(anyw)) return;
         for (int c = threadIdx.x; c < kCull * kThreads + 8; c += kThreads) sh.gsum[c] = 0.0f;
-        if constexpr (POS)
-            for (int c = threadIdx.x; c < 2 * (kCull * kThreads + 8); c += kThreads)
-                gsum_xy[c] = 0.0f;
     }
     if constexpr (COUNT) {
         // counting for the adjoint: the tiles it skips are skipped here too
@@ -910,19 +808,13 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
                 block_max2<kThreads>(hmax, pmax, s_red, nhs, nps);
                 nhs = -nhs;
                 nps = -nps;
-                // adjoint: the voxels' weighted prefactors as packed pairs;
-                // for positions also times d(exponent)/dq = ln2 * ps2 (hs2)
-                float2 FP[NP], FH[NP], FPd[NP], FHd[NP];
+                // adjoint: the voxels' weighted prefactors as packed pairs
+                float2 FP[NP], FH[NP];
                 if constexpr (ADJ) {
 #pragma unroll
                     for (int p = 0; p < NP; ++p) {
                         FP[p] = make_float2(wv[2 * p] * pf[2 * p], wv[2 * p + 1] * pf[2 * p + 1]);
                         FH[p] = make_float2(wv[2 * p] * hf[2 * p], wv[2 * p + 1] * hf[2 * p + 1]);
-                        if constexpr (POS) {
-                            constexpr float kLn2 = 0.6931471805599453f;
-                            FPd[p] = __fmul2_rn(__fmul2_rn(FP[p], PS[p]), f2(kLn2));
-                            FHd[p] = __fmul2_rn(__fmul2_rn(FH[p], HS[p]), f2(kLn2));
-                        }
                     }
                 }
                 float2 AP[NP], AH[NP];
@@ -985,10 +877,6 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
                     if constexpr (COUNT) {
                         n_ex2 += 512ull * (unsigned long long)(2 * n2 + n1);
                         n_eval += 512ull * (unsigned long long)(n2 + n1);
-                    } else if constexpr (POS) {
-                        adjoint_positions<kThreads, NP, kCap>(
-                            s_spot, sh.gsum, gsum_xy, gsum_xy + kCap + 8, n2, n1, B, XP, YP,
-                            GXP, GYP, PS, HS, FP, FH, FPd, FHd, lane, mu, grad, grad_x, grad_y);
                     } else if constexpr (ADJ) {
                         // both terms: slots [0, n2); halo only: [kCap - n1, kCap);
                         // a group's slots past its class hold other records or
@@ -1190,7 +1078,8 @@ struct LutStage {
 // Per-voxel state that changes once per layer lives here rather than in
 // registers (thread t's voxel q at [q][t]), so that the spot loops keep
 // only their own values live.
-template <int NT, int KCULL, bool BEAM_OUT = false, bool DOSE = true, int SPLIT = 1>
+template <int NT, int KCULL, bool BEAM_OUT = false, bool DOSE = true, int SPLIT = 1,
+          bool POS = false>
 struct LineShared {
     static constexpr int kWarps = NT / 32;
     static constexpr int kStage = NT;   // most LUT intervals staged
@@ -1200,7 +1089,8 @@ struct LineShared {
         float2 lut_at[kLine][NT];    // or IDD and sigma per voxel, from rows not staged
     };
     int lut_bad;                     // the layer whose staged row is not uniform
-    float gsum[DOSE ? 1 : NT * KCULL + 8];   // adjoint: per-slot gradient partials
+    // adjoint: per-slot gradient partials (weight; with positions also x, y)
+    float gsum[POS ? 3 : 1][DOSE ? 1 : NT * KCULL + 8];
     float w[kLine][NT];              // the beam's 10*WET per voxel (INF: not valid)
     float d[kLine][NT];              // distance to the source per voxel
     float tot[2][kLine][DOSE ? NT : 1];   // dose: compensated sum over layers and beams
@@ -1329,6 +1219,46 @@ __device__ __forceinline__ TileBounds corner_bounds(const PbGrid &g, const PbBea
     return tb;
 }
 
+// Spot-position derivatives of a line's adjoint sums.  With S the scaled
+// squared axis distance it2 |t x ray|^2 and a voxel's factor mu (Pf 2^(ps2 S) +
+// Hf 2^(hs2 S)),
+//   d/dxs = mu ln2 (Pf ps2 e1 + Hf hs2 e2) dS/dxs,
+// and from ax = X - xs gx, ay = Y - ys gy, az = (xs/VSADX) Y - (ys/VSADY) X
+// - xs ys k (k = 1/VSADX - 1/VSADY), it2 = 1/(1 + xs^2/VSADX^2 + ys^2/VSADY^2):
+//   dS/dxs = 2 it2 (-ax gx + az (Y/VSADX - ys k) - S xs/VSADX^2)
+//   dS/dys = 2 it2 (-ay gy + az (-X/VSADY - xs k) - S ys/VSADY^2).
+// Every factor is affine in the voxel's offset q' on the line and S is a
+// quadratic, so each bracket is a quadratic too: a line needs only the moments
+// m0, m1, m2 of its voxels' factors with 1, q', q'^2, and a spot's two
+// derivatives are three products each (out by 2 it2 mu ln2, which the tile's
+// sum is multiplied with).
+__device__ __forceinline__ void line_position(const LineSpot &r, float Xc, float Yc, float gxc,
+                                              float gyc, float S0, float B1, const float4 &step,
+                                              const PbBeamGeom &G, float m0, float m1, float m2,
+                                              float &vx, float &vy)
+{
+    const float ivx = __fdividef(1.0f, G.vsadx), ivy = __fdividef(1.0f, G.vsady);
+    const float kap = __fsub_rn(ivx, ivy);
+    const float kx2 = r.a.x * (ivx * ivx), ky2 = r.a.y * (ivy * ivy);   // -xs/VSADX^2, ...
+    // the components at the line's centre and their steps along it
+    const float ax = __fmaf_rn(r.a.x, gxc, Xc), ay = __fmaf_rn(r.a.y, gyc, Yc);
+    const float az = __fmaf_rn(r.a.z, Yc, __fmaf_rn(r.a.w, Xc, r.b.x));
+    const float sx = __fmaf_rn(r.a.x, step.z, step.x), sy = __fmaf_rn(r.a.y, step.w, step.y);
+    const float sz = __fmaf_rn(r.a.z, step.y, r.a.w * step.x);
+    const float cx = __fmaf_rn(Yc, ivx, r.a.y * kap), dx = step.y * ivx;
+    const float cy = __fmaf_rn(Xc, -ivy, r.a.x * kap), dy = -step.x * ivy;
+    const float x0 = __fmaf_rn(S0, kx2, __fmaf_rn(az, cx, -ax * gxc));
+    const float x1 = __fmaf_rn(B1, kx2, __fmaf_rn(az, dx, __fmaf_rn(sz, cx,
+                                                  __fmaf_rn(-ax, step.z, -sx * gxc))));
+    const float x2 = __fmaf_rn(r.b.z, kx2, __fmaf_rn(sz, dx, -sx * step.z));
+    const float y0 = __fmaf_rn(S0, ky2, __fmaf_rn(az, cy, -ay * gyc));
+    const float y1 = __fmaf_rn(B1, ky2, __fmaf_rn(az, dy, __fmaf_rn(sz, cy,
+                                                  __fmaf_rn(-ay, step.w, -sy * gyc))));
+    const float y2 = __fmaf_rn(r.b.z, ky2, __fmaf_rn(sz, dy, -sy * step.w));
+    vx = __fmaf_rn(m0, x0, __fmaf_rn(m1, x1, m2 * x2));
+    vy = __fmaf_rn(m0, y0, __fmaf_rn(m1, y1, m2 * y2));
+}
+
 template <int TY, int TZ, int KCULL, bool BEAM_OUT, int MODE = kModeDose, int SPLIT = 1>
 __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int tz,
                                           const float *__restrict__ wet,
@@ -1338,19 +1268,20 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                           float *__restrict__ dose,
                                           float *__restrict__ beam_dose,
                                           LineShared<TY * TZ, KCULL, BEAM_OUT,
-                                                     MODE == kModeDose, SPLIT> &sh,
+                                                     MODE == kModeDose, SPLIT,
+                                                     MODE == kModeAdjointPos> &sh,
                                           unsigned long long *count = nullptr,
                                           const float *__restrict__ wfield = nullptr,
                                           float *__restrict__ grad = nullptr, int rank = 0,
-                                          int ranks = 1)
+                                          int ranks = 1, float *__restrict__ grad_x = nullptr,
+                                          float *__restrict__ grad_y = nullptr)
 {
     constexpr int NT = TY * TZ;
     constexpr int kWarps = NT / 32;
     constexpr bool COUNT = MODE == kModeCount;
-    constexpr bool ADJ = MODE == kModeAdjoint;
+    constexpr bool POS = MODE == kModeAdjointPos;
+    constexpr bool ADJ = MODE == kModeAdjoint || POS;
     static_assert(NT % 32 == 0, "whole warps");
-    static_assert(MODE == kModeDose || MODE == kModeCount || MODE == kModeAdjoint,
-                  "line tiles: dose, count or weight adjoint");
     constexpr int kCap = NT * KCULL;
     // end of the halo-only spots: the forward's filled-up groups need the room
     constexpr int kTop = MODE == kModeDose ? kCap + 16 : kCap;
@@ -1379,7 +1310,8 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
             anyw |= (wv[q] != 0.0f);
         }
         if (!__syncthreads_or(anyw)) return;
-        for (int c = t; c < kCap + 8; c += NT) sh.gsum[c] = 0.0f;
+        for (int c = t; c < kCap + 8; c += NT)
+            for (auto &sum : sh.gsum) sum[c] = 0.0f;
     }
     if constexpr (COUNT) {
         // counting for the adjoint: the tiles it skips are skipped here too
@@ -1711,6 +1643,81 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                     if constexpr (COUNT) {
                         n_ex2 += (unsigned long long)(kLine * NT) * (2 * n2 + n1);
                         n_eval += (unsigned long long)(kLine * NT) * (n2 + n1);
+                    } else if constexpr (POS) {
+                        auto group = [&](auto two, auto n, const int c0) {
+                            constexpr int N = decltype(n)::value;
+                            float v[N], vx[N], vy[N];
+#pragma unroll
+                            for (int u = 0; u < N; ++u) {
+                                const LineSpot r = sh.spot[c0 + u];
+                                float S0, B1;
+                                line_spot(r, Xc, Yc, gxc, gyc, S0, B1);
+                                const float2 s0 = f2(S0), b1 = f2(B1), c2 = f2(r.b.z);
+                                float2 acc = make_float2(0.0f, 0.0f), m0 = acc, m1 = acc, m2 = acc;
+#pragma unroll
+                                for (int p = 0; p < kLine / 2; ++p) {
+                                    const float2 o = line_off2(p);
+                                    const float2 S = __ffma2_rn(__ffma2_rn(c2, o, b1), o, s0);
+                                    const float2 h = __fmul2_rn(AH[p], ex2x2(__fmul2_rn(HS[p], S)));
+                                    acc = __fadd2_rn(acc, h);
+                                    float2 g = __fmul2_rn(HS[p], h);
+                                    if constexpr (decltype(two)::value) {
+                                        const float2 q = __fmul2_rn(AP[p],
+                                                                    ex2x2(__fmul2_rn(PS[p], S)));
+                                        acc = __fadd2_rn(acc, q);
+                                        g = __ffma2_rn(PS[p], q, g);
+                                    }
+                                    m0 = __fadd2_rn(m0, g);
+                                    m1 = __ffma2_rn(o, g, m1);
+                                    m2 = __ffma2_rn(__fmul2_rn(o, o), g, m2);
+                                }
+                                v[u] = acc.x + acc.y;
+                                line_position(r, Xc, Yc, gxc, gyc, S0, B1, sh.step, B.geom,
+                                              m0.x + m0.y, m1.x + m1.y, m2.x + m2.y, vx[u], vy[u]);
+                            }
+                            int slot;
+                            float sum[3];
+                            sum[0] = warp_sum_n<N>(v, lane, slot);
+                            sum[1] = warp_sum_n<N>(vx, lane, slot);
+                            sum[2] = warp_sum_n<N>(vy, lane, slot);
+                            if ((lane & (32 / N - 1)) == 0) {
+#pragma unroll
+                                for (int m = 0; m < 3; ++m)
+                                    if (sum[m] != 0.0f) atomicAdd(&sh.gsum[m][c0 + slot], sum[m]);
+                            }
+                        };
+                        auto groups = [&](auto two, const int lo, const int hi) {
+                            int c0 = lo;
+#pragma unroll 1
+                            for (; c0 + 8 <= hi; c0 += 8)
+                                group(two, std::integral_constant<int, 8>{}, c0);
+                            if (hi - c0 >= 4) {
+                                group(two, std::integral_constant<int, 4>{}, c0);
+                                c0 += 4;
+                            }
+                            if (hi - c0 >= 2) {
+                                group(two, std::integral_constant<int, 2>{}, c0);
+                                c0 += 2;
+                            }
+                            if (c0 < hi) group(two, std::integral_constant<int, 1>{}, c0);
+                        };
+                        groups(std::true_type{}, 0, n2);
+                        groups(std::false_type{}, kCap - n1, kCap);
+                        __syncthreads();
+                        for (int c = t; c < n2 + n1; c += NT) {
+                            const int sl = c < n2 ? c : kCap - n1 + (c - n2);
+                            const int si = __float_as_int(sh.spot[sl].b.w);
+                            // the factor that line_position leaves out
+                            constexpr float kLn2 = 0.6931471805599453f;
+                            const float f = __fmul_rn(__fmul_rn(2.0f * kLn2, sh.spot[sl].b.y),
+                                                      __ldg(mu + si));
+                            const float a = sh.gsum[0][sl];
+                            const float gx = sh.gsum[1][sl], gy = sh.gsum[2][sl];
+                            if (grad && a != 0.0f) atomicAdd(grad + si, a);
+                            if (gx != 0.0f) atomicAdd(grad_x + si, __fmul_rn(gx, f));
+                            if (gy != 0.0f) atomicAdd(grad_y + si, __fmul_rn(gy, f));
+                            sh.gsum[0][sl] = sh.gsum[1][sl] = sh.gsum[2][sl] = 0.0f;
+                        }
                     } else if constexpr (ADJ) {
                         // both terms: slots [0, n2); halo only: [kCap - n1, kCap);
                         // a group's slots past its class hold other records or
@@ -1743,7 +1750,7 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                             int slot;
                             const float sum = warp_sum_n<N>(v, lane, slot);
                             if ((lane & (32 / N - 1)) == 0 && sum != 0.0f)
-                                atomicAdd(&sh.gsum[c0 + slot], sum);
+                                atomicAdd(&sh.gsum[0][c0 + slot], sum);
                         };
                         auto groups = [&](auto two, const int lo, const int hi) {
                             int c0 = lo;
@@ -1765,9 +1772,9 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                         // each surviving spot's tile sum to its gradient
                         for (int c = t; c < n2 + n1; c += NT) {
                             const int sl = c < n2 ? c : kCap - n1 + (c - n2);
-                            const float a = sh.gsum[sl];
+                            const float a = sh.gsum[0][sl];
                             if (a != 0.0f) atomicAdd(grad + __float_as_int(sh.spot[sl].b.w), a);
-                            sh.gsum[sl] = 0.0f;
+                            sh.gsum[0][sl] = 0.0f;
                         }
                     } else {
                         // groups of kGroup spots, evaluated side by side;
@@ -2052,6 +2059,28 @@ k_adjoint_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet
         (int)(blockIdx.x % split), split);
 }
 
+// Spot-weight and spot-position gradients (grad may be NULL).  A line's eight
+// voxels give three moments per spot (line_position) where a tile of single
+// voxels evaluated both brackets at each: 1,150 -> 525 us on the 2-beam
+// 128x121x88 plan of 3,300 spots.  What bounds it is the chain of a group (FMA
+// and exp2 of eight spots, then three sums over the warp), so it takes
+// registers rather than warps: 2 blocks per SM 525 us, 3 571, 4 643 (with the
+// remainders of a class in groups of 4, 2 and 1; one by one 12 us more).
+__global__ void __launch_bounds__(kLineTY * kLineTZ, 2)
+k_adjoint_pos_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
+                   const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
+                   const float *__restrict__ mu, const float *__restrict__ wfield,
+                   float *__restrict__ grad, float *__restrict__ grad_x,
+                   float *__restrict__ grad_y, int split)
+{
+    __shared__ LineShared<kLineTY * kLineTZ, kLineCull, false, false, 1, true> sh;
+    int tx, ty, tz;
+    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / split, tx, ty, tz)) return;
+    line_tile<kLineTY, kLineTZ, kLineCull, false, kModeAdjointPos>(
+        A, tx, ty, tz, wet, layers, geo, mu, nullptr, nullptr, sh, nullptr, wfield, grad,
+        (int)(blockIdx.x % split), split, grad_x, grad_y);
+}
+
 // ------------------------------------------------------------ tile order
 //
 // The line tiles' work spans more than two orders of magnitude (tens of us
@@ -2228,21 +2257,6 @@ k_adjoint_tile(const __grid_constant__ PlanArgs A, const float *__restrict__ wet
     __shared__ DoseShared<128, 2> sh;
     dose_tile<128, 4, 2, false, kModeAdjoint>(A, blockIdx.x, wet, layers, geo, nullptr, nullptr,
                                               nullptr, sh, nullptr, wfield, grad);
-}
-
-// Spot-weight and spot-position gradients: dose_tile in kModeAdjointPos.
-__global__ void __launch_bounds__(128, dose_min_blocks<128>())
-k_adjoint_pos_tile(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
-                   const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
-                   const float *__restrict__ mu, const float *__restrict__ wfield,
-                   float *__restrict__ grad, float *__restrict__ grad_x,
-                   float *__restrict__ grad_y)
-{
-    __shared__ DoseShared<128, 2> sh;
-    __shared__ float gsum_xy[2 * (2 * 128 + 8)];
-    dose_tile<128, 4, 2, false, kModeAdjointPos>(A, blockIdx.x, wet, layers, geo, mu, nullptr,
-                                                 nullptr, sh, nullptr, wfield, grad, grad_x,
-                                                 grad_y, gsum_xy);
 }
 
 // SFU exp2 throughput: kEx2Chains independent chains x <- 2^(-x) per
@@ -2709,10 +2723,12 @@ PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
 PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_beams,
                                   const float *wet, const PbLayer *layers, const float *geo,
                                   const float *mu, const float *w, float scale, float *grad,
-                                  float *grad_x, float *grad_y, cudaStream_t st)
+                                  float *grad_x, float *grad_y, cudaStream_t st, const int *order,
+                                  int split)
 {
     PlanArgs A;
     fill_args(A, g, beams, n_beams, scale);
+    A.order = order;
     int total_spots = 0;
     for (int b = 0; b < n_beams; ++b) {
         const int e = beams[b].spot_start + beams[b].n_spots;
@@ -2723,11 +2739,9 @@ PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_be
     for (float *o : {grad, grad_x, grad_y})
         if (o && s == PB_OK) s = check_cuda(cudaMemsetAsync(o, 0, bytes, st), "cudaMemsetAsync");
     if (s != PB_OK) return s;
-    const int64_t tiles = (int64_t)A.tiles_x * A.tiles_y * A.tiles_z;
-    k_adjoint_pos_tile<<<(unsigned)tiles, 128, 0, st>>>(A, wet, layers,
-                                                        reinterpret_cast<const float4 *>(geo), mu,
-                                                        w, grad, grad_x, grad_y);
-    return check_launch("k_adjoint_pos_tile");
+    k_adjoint_pos_line<<<line_tiles(g, kLineTY, kLineTZ) * split, kLineTY * kLineTZ, 0, st>>>(
+        A, wet, layers, reinterpret_cast<const float4 *>(geo), mu, w, grad, grad_x, grad_y, split);
+    return check_launch("k_adjoint_pos_line");
 }
 
 size_t objective_work_size() { return sizeof(double) * kObjBlocks; }

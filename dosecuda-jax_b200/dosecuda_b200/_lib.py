@@ -138,6 +138,8 @@ _SIGS = {
     "pb_objective": (_I, [_VP, _VP, _VP, _I64, _VP, _VP, _VP, _VP]),
     "pb_count_pairs": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP]),
     "pb_layer_bounds": (_I, [_VP, _I, _VP, _VP, _VP]),
+    "pb_dose_adjoint_positions_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP,
+                                             _VP, _F, _VP, _VP, _VP, _VP, _I, _VP]),
     "pb_dose_adjoint_positions": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _VP,
                                        _F, _VP, _VP, _VP, _VP]),
     "pb_count_evaluated": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _VP]),

@@ -528,11 +528,12 @@ class DevicePlan:
         mu = self.mu_sorted if mu_sorted is None else mu_sorted
         n = max(self.n_spots, 1)
         g, gx, gy = (torch.empty(n, dtype=torch.float32, device=self.device) for _ in range(3))
-        check(_lib.lib.pb_dose_adjoint_positions(
+        mu, w, order = mu.contiguous(), dobj_ddose.contiguous(), self.tile_order()
+        check(_lib.lib.pb_dose_adjoint_positions_split(
             ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
-            ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu.contiguous()),
-            ptr(dobj_ddose.contiguous()), float(scale), ptr(g), ptr(gx), ptr(gy),
-            _stream(self.device)), "pb_dose_adjoint_positions")
+            ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu), ptr(w), float(scale),
+            ptr(g), ptr(gx), ptr(gy), ptr(order), self._split_adjoint, _stream(self.device)),
+            "pb_dose_adjoint_positions_split")
         return g[: self.n_spots], gx[: self.n_spots], gy[: self.n_spots]
 
     def count_pairs(self) -> int:

@@ -254,6 +254,14 @@ PbStatus pb_dose_adjoint_positions(const PbGrid *grid, const PbBeam *beams, int 
                                    const float *spot_geo_dev, const float *mu_dev,
                                    const float *dobj_dose_dev, float scale, float *grad_dev,
                                    float *grad_x_dev, float *grad_y_dev, void *stream);
+/* The same in a given tile order (pb_tile_order; NULL: none), each tile shared
+ * by `split` blocks (1, 2 or 4: pb_tile_split's for the adjoint). */
+PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                         const float *wet_dev, const PbLayer *layers_dev,
+                                         const float *spot_geo_dev, const float *mu_dev,
+                                         const float *dobj_dose_dev, float scale,
+                                         float *grad_dev, float *grad_x_dev, float *grad_y_dev,
+                                         const int *order_dev, int split, void *stream);
 
 /* ------------------------------------------------------- measurement */
 

@@ -105,3 +105,89 @@ def test_nan_and_infinite_depths_as_the_other_family():
         keep = torch.ones(dp.n_vox, dtype=torch.bool, device=DEV)
         keep[[100, 5000]] = False
         assert torch.allclose(d[keep], clean[keep], rtol=1e-6, atol=1e-6 * float(clean.max()))
+
+
+def _reference_gradients(dp, w):
+    """Weight and position gradients of sum w D in FP64 (sorted order), from
+    the physics of the dose: torch.autograd on the spots' positions."""
+    nx, ny, nz = dp.grid.nx, dp.grid.ny, dp.grid.nz
+    geo = dp.spot_geo.cpu().double().reshape(-1, 8).numpy()
+    mu = dp.mu_sorted.double()
+    x = torch.tensor(geo[:, 0], device=DEV, requires_grad=True)
+    y = torch.tensor(geo[:, 1], device=DEV, requires_grad=True)
+    m = mu.clone().requires_grad_(True)
+    k, j, i = torch.meshgrid(*(torch.arange(n, device=DEV, dtype=torch.float64)
+                               for n in (nz, ny, nx)), indexing="ij")
+    total = 0.0
+    for b in range(dp.n_beams):
+        B, G = dp.beams[b], dp.beams[b].geom
+        model = dp._spec[b].model
+        p = [a.reshape(-1) * float(dp.grid.spacing) - float(G.iso[q])
+             for q, a in enumerate((i, j, k))]
+        xt = p[0] * G.costa - p[2] * G.sinta
+        hy = p[0] * G.sinta + p[2] * G.costa
+        X, Y, Z = -(xt * G.cosga + p[1] * G.singa), hy, p[1] * G.cosga - xt * G.singa
+        wet = dp.wet[b].double() * 10.0
+        dist = torch.sqrt(X * X + Y * Y + (0.5 * (G.vsadx + G.vsady) - Z) ** 2)
+        for L in dp.layers_np[dp.layer_offsets[b]:dp.layer_offsets[b + 1]]:
+            e, first = int(L["energy_id"]), B.spot_start + int(L["spot_start"])
+            sl = slice(first, first + int(L["n_spots"]))
+            r80 = float(model.divergence_params[e, 1])
+            ca, cb, cc = (float(v) for v in model.divergence_params[e, 2:5])
+            lut = [torch.as_tensor(np.asarray(t[e], np.float64), device=DEV)
+                   for t in (model.lut_depths, model.lut_sigmas, model.lut_idds)]
+            lo = torch.searchsorted(lut[0], wet).clamp(1, len(lut[0]) - 1)
+            f = ((wet - lut[0][lo - 1]) / (lut[0][lo] - lut[0][lo - 1])).clamp(0.0, 1.0)
+            sig, idd = (t[lo - 1] + f * (t[lo] - t[lo - 1]) for t in lut[1:])
+            d = dist - wet + 0.7 * r80
+            st2 = (ca * d * d + cb * d + cc + sig) ** 2
+            c = wet.clamp(min=0.1).clamp(max=r80 - 0.1)
+            sh = 2.85 + 0.0014 * r80 * torch.log(c + 3.0) + 0.06 * c - 7.4e-5 * c * c - \
+                0.22 * r80 / (c - r80 - 5.0) ** 2
+            wh = 0.052 * torch.log(1.13 + c / (11.2 - 0.023 * r80)) + \
+                0.35 * (0.0017 * r80 * r80 - r80) / ((r80 + 3.0) ** 2 - c * c) - \
+                1.61e-9 * c * (r80 + 3.0) ** 2
+            sh, wh = sh.clamp(min=0.0), wh.clamp(0.0, 0.9)
+            sht2 = st2 + sh * sh
+            tx, ty = x[sl] / G.vsadx, y[sl] / G.vsady
+            ax = X[:, None] - x[sl] * (1.0 - Z / G.vsadx)[:, None]
+            ay = Y[:, None] - y[sl] * (1.0 - Z / G.vsady)[:, None]
+            az = tx * Y[:, None] - ty * X[:, None] - \
+                x[sl] * y[sl] * (1.0 / G.vsadx - 1.0 / G.vsady)
+            r2 = (ax * ax + ay * ay + az * az) / (1.0 + tx * tx + ty * ty)
+            unit = idd / (2.0 * np.pi)
+            kern = ((1.0 - wh) * unit / st2)[:, None] * torch.exp(-0.5 * r2 / st2[:, None]) + \
+                (wh * unit / sht2)[:, None] * torch.exp(-0.5 * r2 / sht2[:, None])
+            use = torch.where(wet <= float(np.float32(1.1) * np.float32(r80)), w.double(), 0.0)
+            total = total + (use[:, None] * kern * m[sl]).sum()
+    total.backward()
+    return m.grad, x.grad, y.grad
+
+
+@pytest.mark.parametrize("n_layers,per_layer,depth_step,shape", [
+    (1, 1, 1.0, (21, 37, 43)), (2, 7, 1.0, (8, 16, 8)), (3, 9, 0.7, (9, 17, 9)),
+    (2, 257, 1.0, (7, 15, 25)), (34, 5, 1.0, (12, 20, 17))])
+def test_position_gradients_against_64_bits(n_layers, per_layer, depth_step, shape):
+    """Every split, with and without an order, and without the weight
+    gradient.  A gradient is a sum of some 1e4 to 1e5 signed FP32 terms, each
+    with a few roundings and an exp2 of 2^-22: 1e-5 of the largest covers
+    them (the terms' own magnitudes add up to some ten times the sum)."""
+    from dosecuda_b200 import _lib
+    dp = _plan(n_layers, per_layer, depth_step, shape)
+    w = torch.randn(dp.n_vox, device=DEV, generator=torch.Generator(DEV).manual_seed(3)) + 0.5
+    ref = _reference_gradients(dp, w)
+    out = [torch.empty(dp.n_spots, device=DEV) for _ in range(3)]
+    for split in (1, 2, 4):
+        for order in (None, dp.tile_order()):
+            weight = out[0] if order is None else None
+            for o in out:
+                o.fill_(float("nan"))
+            _lib.check(_lib.lib.pb_dose_adjoint_positions_split(
+                ctypes.byref(dp.grid), ctypes.cast(dp.beams, ctypes.c_void_p), dp.n_beams,
+                _lib.ptr(dp.wet), _lib.ptr(dp.layers), _lib.ptr(dp.spot_geo),
+                _lib.ptr(dp.mu_sorted), _lib.ptr(w), 1.0, _lib.ptr(weight), _lib.ptr(out[1]),
+                _lib.ptr(out[2]), _lib.ptr(order), split,
+                ctypes.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)))
+            for q, (o, r) in enumerate(zip(out, ref)):
+                if q > 0 or weight is not None:
+                    assert float((o.double() - r).abs().max()) <= 1e-5 * float(r.abs().max())
