@@ -797,59 +797,27 @@ __device__ __forceinline__ void exact_steps(const PbBeamGeom &B, const SmoothBea
 // where the reference's FP32 position is rounded (exact_steps); the
 // chosen voxels are the reference's.  POW2: the grid spacing is a power
 // of two.
+
+// Radii 1..nr of a voxel: dr < lim and dr < 10.
+__device__ __forceinline__ int smooth_radii(float lim)
+{
+    return lim > 9.0f ? 9 : (int)ceilf(lim) - 1;
+}
+
+// One voxel near the faces: every sample is tested against the grid.
 template <bool POW2>
 __device__ __forceinline__ float smooth_voxel(const float *__restrict__ R, const PbGrid &g,
-                                              const PbBeamGeom &Bp, const SmoothBeam &T,
+                                              const PbBeamGeom &B, const SmoothBeam &T,
                                               const float *dc, const float *ds, int i, int j,
-                                              int k)
+                                              int k, float center)
 {
-    const int64_t v = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
-    const float center = R[v];
-    const float lim = __fmul_rn(center, 10.0f);
-    if (!(1.0f < lim)) return center;
-    // radii 1..nr: dr < lim and dr < 10
-    const int nr = lim > 9.0f ? 9 : (int)ceilf(lim) - 1;
-    const PbBeamGeom B = Bp;   // the rotation and isocentre in registers
+    const int nr = smooth_radii(__fmul_rn(center, 10.0f));
     float px, py, pz, hx, hy, hz;
     vox_mm(B, g.spacing, i, j, k, px, py, pz);
     image_to_head_ref(B, px, py, pz, hx, hy, hz);
     const float s = g.spacing;
     const float fi = (float)i, fj = (float)j, fk = (float)k;
     float sum = center;
-    // The radius loops run to 9 for every thread, the samples past the
-    // voxel's own count masked out: the loop counters and the table reads
-    // stay uniform across the warp, and whether a sample is flagged is a
-    // uniform branch.
-    if (i >= T.margin[0] && i <= g.nx - 1 - T.margin[0] && j >= T.margin[1] &&
-        j <= g.ny - 1 - T.margin[1] && k >= T.margin[2] && k <= g.nz - 1 - T.margin[2] &&
-        (int64_t)g.nx * g.ny * g.nz < ((int64_t)1 << 31)) {
-        // Interior: both candidates of every sample lie inside the grid
-        // (the margins), so there are no bounds tests and the indexes are
-        // 32-bit.  A sample past the voxel's count is loaded and not added,
-        // without a branch.
-        const int vi = (int)v, sy = g.nx, sz = g.nx * g.ny;
-        // The nine radii unrolled with an explicit count of 9 (the WET pass
-        // of the 4-beam 256x256x160 plan: 6.79 ms, against 7.29 ms with a
-        // bare "unroll", whose code came out larger, 7.31 ms unrolled by
-        // three and 7.36 by two); the directions stay a loop.
-        for (int dd = 0; dd < 6; ++dd) {
-            const unsigned tm = T.tmask[dd];   // the same for the whole beam
-#pragma unroll 9
-            for (int r = 0; r < 9; ++r) {
-                const int axes = (tm >> (3 * r)) & 7u;
-                int idx = vi + T.off[dd][r];
-                if (axes) {
-                    int ui = 0, uj = 0, uk = 0;
-                    exact_steps<POW2>(B, T, s, dc, ds, hx, hy, hz, fi, fj, fk, dd, r, axes, ui, uj,
-                                      uk);
-                    idx += ui + sy * uj + sz * uk;
-                }
-                const float x = __ldg(R + idx);
-                sum = r < nr ? __fadd_rn(sum, x) : sum;
-            }
-        }
-        return __fdiv_rn(sum, (float)(6 * nr + 1));
-    }
     int n = 1;
     for (int dd = 0; dd < 6; ++dd) {
         unsigned tm = T.tmask[dd];
@@ -877,26 +845,259 @@ __device__ __forceinline__ float smooth_voxel(const float *__restrict__ R, const
     return __fdiv_rn(sum, (float)n);
 }
 
-// 12 resident blocks per SM (40 registers) with a power-of-two spacing,
-// measured faster; with the division call the kernel spills at 40 and is
-// left unbounded.
+// The voxels whose every sample lies in the grid (the table's margins) and the
+// shell around them are different blocks of the launch.  Inside, a thread takes
+// kSmoothPer voxels 32 apart in memory, a warp 32 * kSmoothPer consecutive ones: a
+// sample's table entry, its test for a flagged axis and its address are formed
+// once for the four, whose loads differ by a constant, and a warp's load is one
+// run of 128 bytes.  One voxel a thread in 8x4x4 bricks, interior or not, spent
+// some 20 instructions on a sample that is not flagged (issue slots 87 % used) and
+// four L1 wavefronts on each load.  256x256x160, 4 beams along the axes (18 of 54
+// samples flagged): 2.28 -> 1.7 ms; 200x188x160, 3 oblique beams: 0.93 -> 0.46 ms.
+constexpr int kSmoothPer = 4;   // (smooth_block names the four)
+constexpr int kSmoothBlock = 128 * kSmoothPer;   // voxels of a block inside
+
+// The inner box of a grid: voxels m[a] .. n[a] - 1 - m[a] of each axis, or none;
+// the blocks of the inside (over the whole volume) and of the shell.
+struct SmoothBox {
+    int mx, my, mz;                // half of each axis where nothing is inside
+    long long inner, shell;        // blocks
+};
+
+__host__ __device__ __forceinline__ SmoothBox smooth_box(const PbGrid &g, const int *margin)
+{
+    SmoothBox X;
+    const long long V = (long long)g.nx * g.ny * g.nz;
+    const bool some = 2 * margin[0] < g.nx && 2 * margin[1] < g.ny && 2 * margin[2] < g.nz &&
+                      V < (1ll << 31);
+    X.mx = margin[0];
+    X.my = margin[1];
+    // nothing inside: the shell's end planes are the whole volume
+    X.mz = some ? margin[2] : g.nz;
+    const long long in = some ? (long long)(g.nx - 2 * X.mx) * (g.ny - 2 * X.my) *
+                                    (g.nz - 2 * X.mz) : 0;
+    X.inner = some ? (V + kSmoothBlock - 1) / kSmoothBlock : 0;
+    X.shell = (V - in + 127) / 128;
+    return X;
+}
+
+// The q-th voxel of the shell: the end planes, then of each other plane the end
+// rows and of its other rows the ends.  False past the last.
+__device__ __forceinline__ bool shell_voxel(const PbGrid &g, const SmoothBox &X, long long q,
+                                            int &i, int &j, int &k)
+{
+    const long long plane = (long long)g.nx * g.ny;
+    if (X.mz >= g.nz) {                          // all of the volume
+        if (q >= plane * g.nz) return false;
+        k = (int)(q / plane);
+        q -= plane * k;
+        j = (int)q / g.nx;
+        i = (int)q - j * g.nx;
+        return true;
+    }
+    if (q < 2 * X.mz * plane) {
+        k = (int)(q / plane);
+        q -= plane * k;
+        if (k >= X.mz) k += g.nz - 2 * X.mz;
+        j = (int)q / g.nx;
+        i = (int)q - j * g.nx;
+        return true;
+    }
+    q -= 2 * X.mz * plane;
+    const int rows = 2 * X.my * g.nx, per = rows + (g.ny - 2 * X.my) * 2 * X.mx;
+    if (per == 0) return false;
+    k = X.mz + (int)(q / per);
+    if (k >= g.nz - X.mz) return false;
+    int r = (int)(q - (long long)per * (k - X.mz));
+    if (r < rows) {
+        j = r / g.nx;
+        i = r - j * g.nx;
+        if (j >= X.my) j += g.ny - 2 * X.my;
+        return true;
+    }
+    r -= rows;
+    j = X.my + r / (2 * X.mx);
+    i = r % (2 * X.mx);
+    if (i >= X.mx) i += g.nx - 2 * X.mx;
+    return true;
+}
+
 template <bool POW2>
-__global__ void __launch_bounds__(128, POW2 ? 12 : 1)
+__device__ __forceinline__ void smooth_block(const float *__restrict__ R, const PbGrid &g,
+                                             const PbBeamGeom &Bp, const SmoothBeam &T,
+                                             const float *dc, const float *ds, long long block,
+                                             float *__restrict__ out)
+{
+    const int64_t V = (int64_t)g.nx * g.ny * g.nz;
+    const SmoothBox X = smooth_box(g, T.margin);
+    const PbBeamGeom B = Bp;   // the rotation and isocentre in registers
+    const float s = g.spacing;
+    int i, j, k;
+    if (block >= X.inner) {
+        if (!shell_voxel(g, X, (block - X.inner) * 128 + threadIdx.x, i, j, k)) return;
+        const int64_t v = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
+        const float c = R[v];
+        out[v] = 1.0f < __fmul_rn(c, 10.0f) ? smooth_voxel<POW2>(R, g, B, T, dc, ds, i, j, k, c)
+                                            : c;
+        return;
+    }
+    const int v0 = (int)block * kSmoothBlock + (threadIdx.x >> 5) * (32 * kSmoothPer) +
+                   (threadIdx.x & 31);
+    if (v0 >= V) return;
+    {
+        const unsigned row = (unsigned)v0 / (unsigned)g.nx;
+        i = (int)((unsigned)v0 - row * (unsigned)g.nx);
+        k = (int)(row / (unsigned)g.ny);
+        j = (int)(row - (unsigned)k * (unsigned)g.ny);
+    }
+    // Whether every sample of the four, at either candidate, lies in the
+    // volume's memory: then the loads need no tests.  What a voxel of the shell
+    // reads so is not used.
+    const int64_t reach = X.mx + (int64_t)g.nx * (X.my + (int64_t)g.ny * X.mz);
+    const bool whole = v0 >= reach && v0 + 32 * (kSmoothPer - 1) + reach < V;
+    float center[kSmoothPer], sum[kSmoothPer], hx[kSmoothPer], hy[kSmoothPer], hz[kSmoothPer];
+    float fi[kSmoothPer], fj[kSmoothPer], fk[kSmoothPer];
+    int nr[kSmoothPer];        // radii of each voxel, -1: not inside
+    bool inner = false;
+#pragma unroll
+    for (int m = 0; m < kSmoothPer; ++m) {
+        if (m > 0) {
+            i += 32;
+            while (i >= g.nx) {
+                i -= g.nx;
+                if (++j == g.ny) {
+                    j = 0;
+                    ++k;
+                }
+            }
+        }
+        const bool in = i >= X.mx && i < g.nx - X.mx && j >= X.my && j < g.ny - X.my &&
+                        k >= X.mz && k < g.nz - X.mz;
+        center[m] = in ? R[v0 + 32 * m] : 0.0f;
+        sum[m] = center[m];
+        const float lim = __fmul_rn(center[m], 10.0f);
+        nr[m] = !in ? -1 : 1.0f < lim ? smooth_radii(lim) : 0;
+        inner |= nr[m] > 0;
+        float px, py, pz;
+        vox_mm(B, s, i, j, k, px, py, pz);
+        image_to_head_ref(B, px, py, pz, hx[m], hy[m], hz[m]);
+        fi[m] = (float)i;
+        fj[m] = (float)j;
+        fk[m] = (float)k;
+    }
+    if (whole && inner) {
+        const float *at = R + v0;
+        const int sy = g.nx, sz = g.nx * g.ny;
+        for (int dd = 0; dd < 6; ++dd) {
+            const unsigned tm = T.tmask[dd];   // the same for the whole beam
+            if (tm == 0) {
+#pragma unroll
+                for (int r = 0; r < 9; ++r) {
+                    const float *q = at + T.off[dd][r];
+#pragma unroll
+                    for (int m = 0; m < kSmoothPer; ++m) {
+                        const float x = __ldg(q + 32 * m);
+                        sum[m] = r < nr[m] ? __fadd_rn(sum[m], x) : sum[m];
+                    }
+                }
+                continue;
+            }
+            const float c = dc[dd], sn = ds[dd];
+#pragma unroll 1
+            for (int r = 0; r < 9; ++r) {
+                const int axes = (tm >> (3 * r)) & 7u;
+                const float *q = at + T.off[dd][r];
+                float x[kSmoothPer] = {};
+                // One flagged axis, the usual case (beams along the image
+                // axes): exact_steps' operations for it alone, with what does
+                // not change over the samples in registers.  The candidate is
+                // inside the grid, so h > 0 and a quotient of h rounds up.
+                auto one_axis = [&](auto a, const int stride) {
+                    constexpr int A = decltype(a)::value;
+                    const float hh = T.hh[dd][r][A], dr = (float)(r + 1);
+#pragma unroll
+                    for (int m = 0; m < kSmoothPer; ++m) {
+                        const float xz = -__fmaf_rn(dr, c, hx[m]);
+                        float p;
+                        if constexpr (A == 1) {
+                            p = __fmaf_rn(xz, B.singa, __fmul_rn(hz[m], B.cosga));
+                        } else {
+                            const float xg = __fmaf_rn(xz, B.cosga, __fmul_rn(-hz[m], B.singa));
+                            const float zg = __fmaf_rn(dr, sn, hy[m]);
+                            p = A == 0 ? __fmaf_rn(xg, B.costa, __fmul_rn(zg, B.sinta))
+                                       : __fmaf_rn(-xg, B.sinta, __fmul_rn(zg, B.costa));
+                        }
+                        p = __fadd_rn(p, B.iso[A]);
+                        const float h = __fadd_rn(A == 0 ? fi[m] : A == 1 ? fj[m] : fk[m], hh);
+                        const float quotient = POW2 ? __fmul_rn(p, T.inv_s) : div_rn(p, s);
+                        x[m] = __ldg(q + 32 * m + (quotient >= h ? stride : 0));
+                    }
+                };
+                if (axes == 1) {
+                    one_axis(std::integral_constant<int, 0>{}, 1);
+                } else if (axes == 2) {
+                    one_axis(std::integral_constant<int, 1>{}, sy);
+                } else if (axes == 4) {
+                    one_axis(std::integral_constant<int, 2>{}, sz);
+                } else if (axes) {
+#pragma unroll 1
+                    for (int m = 0; m < kSmoothPer; ++m) {
+                        int ui = 0, uj = 0, uk = 0;
+                        auto of = [&](const float *v) {   // no indexed registers
+                            return m == 0 ? v[0] : m == 1 ? v[1] : m == 2 ? v[2] : v[3];
+                        };
+                        exact_steps<POW2>(B, T, s, dc, ds, of(hx), of(hy), of(hz), of(fi), of(fj),
+                                          of(fk), dd, r, axes, ui, uj, uk);
+                        const float w = __ldg(q + 32 * m + (ui + sy * uj + sz * uk));
+#pragma unroll
+                        for (int l = 0; l < kSmoothPer; ++l) x[l] = l == m ? w : x[l];
+                    }
+                } else {
+#pragma unroll
+                    for (int m = 0; m < kSmoothPer; ++m) x[m] = __ldg(q + 32 * m);
+                }
+#pragma unroll
+                for (int m = 0; m < kSmoothPer; ++m)
+                    sum[m] = r < nr[m] ? __fadd_rn(sum[m], x[m]) : sum[m];
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < kSmoothPer; ++m) {
+        if (nr[m] < 0) continue;
+        float r = nr[m] > 0 ? __fdiv_rn(sum[m], (float)(6 * nr[m] + 1)) : center[m];
+        if (!whole && nr[m] > 0)   // the first and last rows inside
+            r = smooth_voxel<POW2>(R, g, B, T, dc, ds, (int)fi[m], (int)fj[m], (int)fk[m],
+                                   center[m]);
+        out[v0 + 32 * m] = r;
+    }
+}
+
+// Resident blocks per SM (registers): 9 of 56; 6, 7, 8 and 10 took 6.15, 5.96, 5.84
+// and 5.90 ms for the whole WET of the 256x256x160 phantom against 5.80.
+// For the batch, whose table is in shared memory, 10: 8.03 ms for a batch of 8 plans
+// against 8.18 (6) and 8.08 (8).
+constexpr int kSmoothBlocks = 9, kSmoothBatchBlocks = 10;
+// First block of each beam.
+struct SmoothStarts {
+    int n;
+    unsigned start[PB_MAX_BEAMS];
+};
+
+template <bool POW2>
+__global__ void __launch_bounds__(128, kSmoothBlocks)
 k_smooth(const float *__restrict__ raw, PbGrid g, const __grid_constant__ BeamGeomSet bs,
-         const __grid_constant__ SmoothSet st, int zbricks, float *__restrict__ wet)
+         const __grid_constant__ SmoothSet st,
+         const __grid_constant__ SmoothStarts at, float *__restrict__ wet)
 {
     __shared__ float s_dc[6], s_ds[6];
-    const int tid = threadIdx.x + 8 * (threadIdx.y + 4 * threadIdx.z);
-    if (tid < 6) smooth_dir_dev(tid, s_dc[tid], s_ds[tid]);
+    if (threadIdx.x < 6) smooth_dir_dev(threadIdx.x, s_dc[threadIdx.x], s_ds[threadIdx.x]);
     __syncthreads();
-    const int b = blockIdx.z / zbricks;
-    const int k = (blockIdx.z - b * zbricks) * 4 + threadIdx.z;
-    const int j = blockIdx.y * 4 + threadIdx.y;
-    const int i = blockIdx.x * 8 + threadIdx.x;
-    if (i >= g.nx || j >= g.ny || k >= g.nz) return;
+    int b = 0;
+    while (b + 1 < at.n && blockIdx.x >= at.start[b + 1]) ++b;
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
-    const int64_t v = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
-    wet[b * V + v] = smooth_voxel<POW2>(raw + b * V, g, bs.b[b], st.b[b], s_dc, s_ds, i, j, k);
+    smooth_block<POW2>(raw + b * V, g, bs.b[b], st.b[b], s_dc, s_ds, blockIdx.x - at.start[b],
+                       wet + b * V);
 }
 
 // One (plan, beam) of a batched WET pass.
@@ -911,7 +1112,8 @@ struct BatchWet {
     SmoothBeam sm;              // this beam's smoothing samples
     int cap;
     int bx, by, bz;             // 8x4x4 bricks per axis
-    long long brick_start;      // first brick of this item in the launch
+    long long brick_start;      // first brick of this item in the launches
+    long long smooth_blocks;    // its blocks of the smoothing launch, no more than its bricks
 };
 
 __device__ __forceinline__ int find_wet_item(const BatchWet *__restrict__ items, int n,
@@ -959,25 +1161,26 @@ k_raytrace_batch(const BatchWet *__restrict__ items, int n_items, int *status)
     W.raw[i + (int64_t)W.g.nx * (j + (int64_t)W.g.ny * k)] = r;
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, kSmoothBatchBlocks)
 k_smooth_batch(const BatchWet *__restrict__ items, int n_items)
 {
     static_assert(sizeof(SmoothBeam) % 4 == 0, "the table is copied as words");
     __shared__ SmoothBeam sm;
     __shared__ float s_dc[6], s_ds[6];
-    if (threadIdx.x < 6) smooth_dir_dev(threadIdx.x, s_dc[threadIdx.x], s_ds[threadIdx.x]);
     const BatchWet &W = items[find_wet_item(items, n_items, blockIdx.x)];
+    const long long block = blockIdx.x - W.brick_start;
+    if (block >= W.smooth_blocks) return;   // the whole block
+    if (threadIdx.x < 6) smooth_dir_dev(threadIdx.x, s_dc[threadIdx.x], s_ds[threadIdx.x]);
     // the block's sample table into shared memory (one item per block)
     const int *src = reinterpret_cast<const int *>(&W.sm);
     int *dst = reinterpret_cast<int *>(&sm);
     for (int q = threadIdx.x; q < (int)(sizeof(SmoothBeam) / 4); q += blockDim.x)
         dst[q] = __ldg(src + q);
     __syncthreads();
-    int i, j, k;
-    if (!brick_voxel(W, blockIdx.x, i, j, k)) return;
-    float *out = W.wet + i + (int64_t)W.g.nx * (j + (int64_t)W.g.ny * k);
-    *out = sm.pow2 ? smooth_voxel<true>(W.raw, W.g, W.geom, sm, s_dc, s_ds, i, j, k)
-                   : smooth_voxel<false>(W.raw, W.g, W.geom, sm, s_dc, s_ds, i, j, k);
+    if (sm.pow2)
+        smooth_block<true>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
+    else
+        smooth_block<false>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
 }
 
 __device__ float g_smooth_dirs[12];
@@ -1019,10 +1222,7 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
     for (int b = 0; b < n_beams; ++b) bs.b[b] = beams[b];
     SmoothSet ss;
     smooth_set(g, beams, n_beams, ss);
-    const int zb = (g.nz + 3) / 4;
-    dim3 block(8, 4, 4);
-    dim3 grid((g.nx + 7) / 8, (g.ny + 3) / 4, zb * n_beams);
-    const int64_t bricks = (int64_t)grid.x * grid.y * grid.z;
+    const int64_t bricks = (int64_t)((g.nx + 7) / 8) * ((g.ny + 3) / 4) * ((g.nz + 3) / 4) * n_beams;
     if (bricks > INT32_MAX) return set_error(PB_ERR_INVALID, "grid too large");
     const int64_t some = (bricks + kBricksPerBlock - 1) / kBricksPerBlock;
     const unsigned rg = (unsigned)(bricks < 148 * 512 ? bricks : some);
@@ -1040,10 +1240,20 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
     }
     PbStatus s = check_launch("k_raytrace");
     if (s != PB_OK) return s;
+    SmoothStarts at;
+    at.n = n_beams;
+    long long blocks = 0;
+    for (int b = 0; b < n_beams; ++b) {
+        at.start[b] = (unsigned)blocks;
+        const SmoothBox X = smooth_box(g, ss.b[b].margin);
+        blocks += X.inner + X.shell;
+        if (blocks > INT32_MAX) return set_error(PB_ERR_INVALID, "grid too large");
+    }
+    const unsigned sg = (unsigned)blocks;
     if (ss.b[0].pow2)
-        k_smooth<true><<<grid, block, 0, st>>>(raw, g, bs, ss, zb, wet);
+        k_smooth<true><<<sg, 128, 0, st>>>(raw, g, bs, ss, at, wet);
     else
-        k_smooth<false><<<grid, block, 0, st>>>(raw, g, bs, ss, zb, wet);
+        k_smooth<false><<<sg, 128, 0, st>>>(raw, g, bs, ss, at, wet);
     return check_launch("k_smooth");
 }
 
@@ -1071,7 +1281,7 @@ long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbB
     smooth_set(g, beams, n_beams, ss);
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
     const int bx = (g.nx + 7) / 8, by = (g.ny + 3) / 4, bz = (g.nz + 3) / 4;
-    const long long per = (long long)bx * by * bz;
+    long long start = brick_start;
     for (int b = 0; b < n_beams; ++b) {
         BatchWet &w = W[b];
         w.g = g;
@@ -1086,9 +1296,13 @@ long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbB
         w.bx = bx;
         w.by = by;
         w.bz = bz;
-        w.brick_start = brick_start + per * b;
+        w.brick_start = start;
+        const SmoothBox X = smooth_box(g, w.sm.margin);
+        w.smooth_blocks = X.inner + X.shell;
+        // both launches go by these starts
+        start += std::max((long long)bx * by * bz, w.smooth_blocks);
     }
-    return per * n_beams;
+    return start - brick_start;
 }
 
 PbStatus launch_wet_batch(const void *items_dev, int n_items, long long n_bricks, int *status,
