@@ -1041,11 +1041,17 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
 // cull differently, or add a layer's spots in another order, and agree to
 // rounding.
 
-// Spots the forward evaluates side by side, both terms and halo only (up to
-// this many less one are added with weight 0 to fill the last group).  4-beam
+// Spots the forward evaluates side by side, both terms and halo only (spots of
+// weight 0 fill the last group).  4-beam
 // 256x256x160 plan / 512x512x200 plan of 59,840 spots, forward alone: 4 spots
 // 5.65 / 100.8 ms, 5 5.58 / 99.7, 6 5.55 / 98.8, 7 5.74 / 102.3, 8 5.79 / 102.7.
+// The last group of a class is filled up to half a group where that holds the
+// rest (6 spots: 1 of them unused instead of 2.5 on average; 512x512x200 100.6 ->
+// 100.05 ms, the 4-beam plan's step 11.54 -> 11.45 ms).  Tiles of 64
+// threads, the batch's, are kept to whole groups: a batch of 8 plans 8.03 ms
+// against 8.12.
 constexpr int kGroupBoth = 6, kGroupHalo = 6;
+template <int NT> constexpr int line_fill(int group) { return NT >= 128 ? group / 2 : group; }
 constexpr int kLine = 8;
 
 // Line-tile record of one surviving spot: (-x, -y, x/VSADX, -y/VSADY),
@@ -1285,7 +1291,10 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
     constexpr int kCap = NT * KCULL;
     // end of the halo-only spots: the forward's filled-up groups need the room
     constexpr int kTop = MODE == kModeDose ? kCap + 16 : kCap;
-    static_assert(kGroupBoth + kGroupHalo - 2 <= 16, "padding of both classes");
+    constexpr int kFillBoth = line_fill<NT>(kGroupBoth), kFillHalo = line_fill<NT>(kGroupHalo);
+    static_assert(kGroupBoth % 2 == 0 && kGroupHalo % 2 == 0, "half groups");
+    static_assert(kFillBoth + kFillHalo - 2 <= 16, "padding of both classes");
+    auto filled = [](int n, int part) { return (n + part - 1) / part * part; };
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
 
@@ -1630,11 +1639,9 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                         LineSpot r;
                         r.a = r.c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         r.b = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
-                        if (t < kGroupBoth - 1 &&
-                            n2 + t < (n2 + kGroupBoth - 1) / kGroupBoth * kGroupBoth)
+                        if (t < kFillBoth - 1 && n2 + t < filled(n2, kFillBoth))
                             sh.spot[n2 + t] = r;
-                        if (t < kGroupHalo - 1 &&
-                            n1 + t < (n1 + kGroupHalo - 1) / kGroupHalo * kGroupHalo)
+                        if (t < kFillHalo - 1 && n1 + t < filled(n1, kFillHalo))
                             sh.spot[kTop - 1 - n1 - t] = r;
                     }
                     __syncthreads();
@@ -1805,15 +1812,21 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                 }
                             }
                         };
-                        using Both = std::integral_constant<int, kGroupBoth>;
-                        using Halo = std::integral_constant<int, kGroupHalo>;
+                        auto groups = [&](auto two, auto size, int c, const int end) {
+                            constexpr int kGroup = decltype(size)::value;
+                            if constexpr (line_fill<NT>(kGroup) < kGroup) {
+                                if ((end - c) % kGroup) {
+                                    group(two, std::integral_constant<int, kGroup / 2>{}, c);
+                                    c += kGroup / 2;
+                                }
+                            }
 #pragma unroll 1
-                        for (int c = 0; c < n2; c += kGroupBoth)
-                            group(std::true_type{}, Both{}, c);
-#pragma unroll 1
-                        for (int c = kTop - (n1 + kGroupHalo - 1) / kGroupHalo * kGroupHalo;
-                             c < kTop; c += kGroupHalo)
-                            group(std::false_type{}, Halo{}, c);
+                            for (; c < end; c += kGroup) group(two, size, c);
+                        };
+                        groups(std::true_type{}, std::integral_constant<int, kGroupBoth>{}, 0,
+                               filled(n2, kFillBoth));
+                        groups(std::false_type{}, std::integral_constant<int, kGroupHalo>{},
+                               kTop - filled(n1, kFillHalo), kTop);
                     }
                     __syncthreads();
                 }
