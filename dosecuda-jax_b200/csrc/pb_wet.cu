@@ -5,10 +5,11 @@
 //   ray trace             DoseCUDA/dose_kernels/CudaClasses.cu:180-228
 //   smoothing             DoseCUDA/dose_kernels/IMPTClasses.cu:139-202
 //
-// Layout: every volume is x-fastest; one thread per voxel; blocks are 8x4x4
-// voxel bricks so that a warp covers an 8x4 patch whose rays have similar
+// Layout: every volume is x-fastest.  The ray trace takes one voxel per thread
+// in bricks of 8x4x4, so that a warp covers an 8x4 patch whose rays have similar
 // lengths whatever the beam direction, and each row of 8 voxels is one
-// 32-byte sector.  Several beams share one launch (grid z = z-bricks x beams).
+// 32-byte sector; the smoothing takes runs of consecutive voxels.  Several beams
+// share one launch.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
