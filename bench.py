@@ -382,7 +382,8 @@ def run_mine(args, world, rank, local):
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "call": "IMPTDoseGrid.computeIMPTPlan" if args.mode == "forward"
                 else "engine.HostGradientStep"},
-        # per forward step: HU->RLSP, [texture mode: five cell-record passes],
+        # per forward step: HU->RLSP, [texture mode: four cell-record passes and
+        # the ray trace of the other kind of volume, which ends at once],
         # ray trace, smoothing, the tile order (cost, histogram, scan,
         # scatter), pencil-beam sum; the grad step adds the objective (two)
         # and the adjoint
