@@ -1333,6 +1333,7 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
         }
     }
 
+    int round = 0;   // of the cluster's exchange, over all beams and chunks of the tile
     for (int b = 0; b < A.n_beams; ++b) {
         const PbBeam &B = A.beams[b];
         float Xc, Yc, gxc, gyc;   // the line's centre and its divergence factors
@@ -1436,7 +1437,6 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                             : 0.0f;
                 }
             }
-            int round = 0;
             for (int l1 = 0; l1 < nsel; l1 += ranks, ++round) {
               const int li = l1 + rank;
               bool live = li < nsel;
@@ -1860,9 +1860,12 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
               if constexpr (MODE == kModeDose && SPLIT > 1) {
                 if (ranks > 1) {
                     // the round's layers, in order, into the voxels this
-                    // block owns.  The next round writes the other buffer,
-                    // and the one after it starts behind the next barrier,
-                    // which every reader of this buffer has passed by then.
+                    // block owns.  The next round, be it of another chunk of
+                    // layers or of another beam, writes the other buffer, and
+                    // the one after it starts behind the next round's barrier,
+                    // which a block reaches only when it has read this buffer.
+                    // All blocks select the same layers, so they run the same
+                    // rounds and their counts agree.
                     cluster_barrier();
                     constexpr int kOwn = kLine / SPLIT;
                     const int nr = min(ranks, nsel - l1);

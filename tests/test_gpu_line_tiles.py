@@ -191,3 +191,41 @@ def test_position_gradients_against_64_bits(n_layers, per_layer, depth_step, sha
             for q, (o, r) in enumerate(zip(out, ref)):
                 if q > 0 or weight is not None:
                     assert float((o.double() - r).abs().max()) <= 1e-5 * float(r.abs().max())
+
+
+@pytest.mark.parametrize("n_beams,n_layers", [(4, 1), (3, 2), (4, 3), (3, 4), (4, 5), (3, 33)])
+def test_splits_with_uneven_layers_over_many_beams(n_beams, n_layers):
+    """The cluster's blocks out of step: a layer of many compaction rounds
+    beside layers that are left out (their spots lie outside the tiles' reach),
+    staged beside unstaged LUT rows, an odd number of rounds in a beam and more
+    layers than one selection takes.  Every launch gives the bits of split 1."""
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_impt import IMPTPlan
+    shape, s = (24, 40, 48), 3.0
+    rng = np.random.default_rng(10 * n_beams + n_layers)
+    beams = []
+    for b in range(n_beams):
+        model = copy.copy(IMPTPlan().beam_models[0])
+        model.__dict__.pop("_pb_device_tables", None)
+        if b % 2:   # rows that are not staged
+            model.lut_depths = (model.lut_depths * 0.7).astype(np.float32)
+        rows = []
+        for q in range(n_layers):
+            heavy = q == b % n_layers
+            n = (1600 if n_layers < 9 else 600) if heavy else 3
+            xy = rng.uniform(-20.0, 20.0, (n, 2))
+            if not heavy and q % 2:
+                # two corners of a box that the tiles lie in: selected, then left out
+                xy = np.array([[-160.0, -160.0], [160.0, 160.0], [160.0, -160.0]])
+            rows.append(np.column_stack([xy, rng.uniform(0.5, 1.5, n), np.full(n, 20.0 + q)]))
+        beams.append(engine.BeamSpec(360.0 / n_beams * b + 7.0, 0.0, np.zeros(3, np.float32),
+                                     np.concatenate(rows).astype(np.float32), model))
+    dp = engine.DevicePlan(shape, s, -0.5 * s * np.array(shape[::-1], np.float32), beams, DEV)
+    j = torch.arange(shape[1], device=DEV, dtype=torch.float32)[None, :, None]
+    wet = (0.2 * j + 1.0).expand(shape).reshape(1, -1).repeat(n_beams, 1)
+    dp.set_wet(wet.contiguous())
+    one = _dose(dp, 1)
+    assert float(one.max()) > 0
+    for split in (2, 4):
+        for rep in range(60):
+            assert torch.equal(_dose(dp, split, order=rep % 2 == 0), one), (split, rep)
