@@ -392,15 +392,34 @@ PbStatus pb_dose_adjoint_ordered(const PbGrid *grid, const PbBeam *beams, int n_
                           order_dev);
 }
 
+static PbStatus check_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                 const float *spot_boxes)
+{
+    PbStatus s = check_grid(grid);
+    if (s == PB_OK && (!beams || n_beams <= 0 || n_beams > PB_MAX_BEAMS || !spot_boxes))
+        s = set_error(PB_ERR_INVALID, "NULL argument or beam count");
+    return s;
+}
+
 PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                        const float *spot_boxes, int *forward_out, int *adjoint_out)
 {
-    PbStatus s = check_grid(grid);
+    PbStatus s = check_tile_split(grid, beams, n_beams, spot_boxes);
     if (s != PB_OK) return s;
-    if (!beams || n_beams <= 0 || n_beams > PB_MAX_BEAMS || !spot_boxes || !forward_out ||
-        !adjoint_out)
-        return set_error(PB_ERR_INVALID, "NULL argument or beam count");
-    tile_split(*grid, beams, n_beams, spot_boxes, forward_out, adjoint_out);
+    if (!forward_out || !adjoint_out) return set_error(PB_ERR_INVALID, "NULL argument");
+    int positions;
+    tile_split(*grid, beams, n_beams, spot_boxes, forward_out, adjoint_out, &positions);
+    return PB_OK;
+}
+
+PbStatus pb_tile_split_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                 const float *spot_boxes, int *positions_out)
+{
+    PbStatus s = check_tile_split(grid, beams, n_beams, spot_boxes);
+    if (s != PB_OK) return s;
+    if (!positions_out) return set_error(PB_ERR_INVALID, "NULL argument");
+    int forward, adjoint;
+    tile_split(*grid, beams, n_beams, spot_boxes, &forward, &adjoint, positions_out);
     return PB_OK;
 }
 
@@ -806,8 +825,8 @@ PbStatus pb_proton_spot_host(int gpu_id, double vsadx, double vsady, const float
             box[2] = std::min(box[2], spots[i].y);
             box[3] = std::max(box[3], spots[i].y);
         }
-        int split = 1, split_adj = 1;
-        tile_split(g, &B, 1, box, &split, &split_adj);
+        int split = 1, split_adj = 1, split_pos = 1;
+        tile_split(g, &B, 1, box, &split, &split_adj, &split_pos);
         // the tiles in the order of their estimated work (pb_tile_order)
         PB_TRY(launch_tile_order(g, &B, 1, static_cast<const float *>(D.buf[kBufWet].p),
                                  static_cast<const PbLayer *>(D.buf[kBufLayers].p),

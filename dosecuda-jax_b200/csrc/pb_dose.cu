@@ -34,6 +34,7 @@
 // over a thread's voxels meet across the warp with a transposed butterfly,
 // across the block in shared memory, and go to the gradient with one global
 // atomic per spot per (tile, layer).
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 #include "pb_internal.h"
@@ -2801,58 +2802,128 @@ void tile_order_tile(int *voxels)
 
 // Blocks per tile.  A tile that the beams reach keeps its block busy for tens
 // of microseconds (a warp per scheduler, one layer after the other), so a plan
-// with fewer such tiles than the GPU has places for blocks (148 SMs x 4) ends
-// on that latency while SMs idle; sharing each tile's layers among 2 or 4
-// blocks then shortens it, at the price of setting the tile up in each.  The
-// lines measured (microseconds, forward / adjoint, 1, 2 and 4 blocks):
-//     96 tiles reached   56, 40, 34 / 64, 39, 35
-//    455                417, 289, 235 / 549, 336, 229
-//    540                190, 149, 183 / 244, 157, 165
-//    561                787, 521, 504 / 951, 571, 493
-//    702                365, 345, 362 / 350, 239, 165
-//   1232                269, 284, 353 / 295, 284, 334
-//   1412                306, 324, 384 / 346, 344, 384
-// The adjoint has no exchange between the blocks and skips tiles where its
-// field is zero, so it gains up to a larger count.  The tiles reached are
-// estimated from the beams' spot boxes: a tile counts when its centre lies
-// within 60 mm (where the widest halo falls below 2^-24) and half a tile's
-// width of a beam's box of spot axes.
+// with fewer such tiles than the GPU has places for blocks ends on that latency
+// while SMs idle; sharing each tile's layers among 2 or 4 blocks then shortens
+// it.  Only the layers are shared: each block loads the depths, forms the box
+// and selects the layers of every beam, in the tiles that no spot reaches too,
+// so a beam of one or two layers gains nothing and pays that `split` times.
+// Hence an estimate of the launch's time at each split, in microseconds:
+//     base + sqrt(chain^2 + (work / 148)^2),
+// chain the layers of a mean tile one after the other (each reached beam's
+// ceil(layers / split) of them), work what the SMs do in all: a block's set-up
+// per reached tile and beam and per tile not reached, `split` times, and the
+// layers once.  The constants are fitted to the measured ratios of the three
+// splits on random plans (1 to 4 beams of 1 to 33 layers of 9 to 1,153 spots, 75
+// to 3,465 tiles reached; the forward 640 plans, the gradients 220); a larger
+// split is taken where its estimate is the smaller one (forward: by 4 %).
+// Microseconds at 1, 2 and 4 blocks, and what is taken:
+//   tiles beams layers spots   forward           weight gradient    taken
+//    120    2     1     185   50,  58,  76         74,  78,  89     1 / 1
+//    498    4     1      69   52,  68, 117         51,  54,  58     1 / 1
+//    495    2     2      37   53,  68, 102         54,  46,  55     1 / 2
+//    342    1     3      49   34,  32,  43         41,  35,  34     1 / 2
+//     90    1     3      89   42,  35,  33         59,  43,  37     4 / 4
+//    291    2     6      97   160, 107, 109        222, 127,  97    2 / 4
+//    797    3     6     101   388, 274, 337        402, 256, 180    2 / 2
+//    120    1    12      97   150,  97,  64        218, 122,  78    4 / 4
+//    728    2    16     973   4055, 2474, 2345     5017, 2783, 1876 4 / 4
+//   1326    4    16      61   673, 702, 849        757, 684, 770    1 / 1
+// Against one block per tile over those plans: forward 1.27 times as fast (the
+// best of the three would be 1.30), slower by more than 5 % in 4 of 640 (17 % at
+// most); weight gradient of a field without zeros 1.41 (1.42) and 1 of 220 (9 %);
+// position gradients 1.20 (1.21) and 2 (13 %).  A gradient skips the tiles where
+// its field is zero, which the host does not know; the fit is to fields without
+// zeros, as the gradient of an objective over the whole grid is, and a field
+// around the target alone still gains 1.65 of 1.81 and is never slower.  The tiles
+// reached are estimated from the beams' spot boxes: a tile counts for a beam when
+// its centre lies within 60 mm (where the widest halo falls below 2^-24) and half
+// a tile's width of the beam's box of spot axes.
 constexpr int kSplitMaxTiles = 4096;   // larger grids are not looked at
 
-void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
-                int *forward, int *adjoint)
+struct SplitCost {
+    float base;          // launch, ramp and the chain's set-up
+    float layer, spot;   // of the chain, per layer and per spot of a layer
+    float block;         // set-up per block of a reached tile and beam
+    float idle;          // set-up per block of a tile not reached, and beam
+    float share;         // of an SM that a layer's time occupies
+    float gain;          // estimates a larger split must win by
+};
+constexpr SplitCost kSplitForward = {15.0f, 6.0f, 0.06f, 2.9f, 0.7f, 0.15f, 1.04f};
+constexpr SplitCost kSplitAdjoint = {24.0f, 4.3f, 0.14f, 1.9f, 0.45f, 0.115f, 1.0f};
+constexpr SplitCost kSplitPositions = {28.0f, 6.4f, 0.14f, 3.1f, 1.3f, 0.265f, 1.0f};
+
+// Tiles that a plan's beams reach.
+struct SplitTiles {
+    int tiles, active;                 // all, and those that some beam reaches
+    int reached[PB_MAX_BEAMS];         // by each beam
+};
+
+static int split_of(const SplitTiles &T, const PbBeam *beams, int n_beams, const SplitCost &C)
 {
-    *forward = *adjoint = 1;
+    auto time = [&](int split) {
+        float chain = 0.0f, work = (float)(T.tiles - T.active) * n_beams * split * C.idle;
+        for (int b = 0; b < n_beams; ++b) {
+            if (T.reached[b] == 0) continue;
+            const int L = beams[b].n_layers;
+            const float one = C.layer + C.spot * (float)beams[b].n_spots / (float)L;
+            chain += (float)T.reached[b] / (float)T.active * (float)((L + split - 1) / split) * one;
+            work += (float)T.reached[b] * (split * C.block + L * one * C.share);
+        }
+        return C.base + sqrtf(chain * chain + work / 148.0f * (work / 148.0f));
+    };
+    if (T.active == 0) return 1;
+    const float t1 = time(1), t2 = time(2), t4 = time(4);
+    const bool two = C.gain * t2 < t1;
+    return C.gain * t4 < (two ? t2 : t1) ? 4 : two ? 2 : 1;
+}
+
+void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                int *forward, int *adjoint, int *positions)
+{
+    *forward = *adjoint = *positions = 1;
     const int ntx = (g.nx + kLine - 1) / kLine, nty = (g.ny + kLineTY - 1) / kLineTY;
     const int ntz = (g.nz + kLineTZ - 1) / kLineTZ;
     if ((long long)ntx * nty * ntz > kSplitMaxTiles) return;
     const float reach = 60.0f + 0.5f * kLine * g.spacing;
-    int active = 0;
-    for (int z = 0; z < ntz; ++z)
-        for (int y = 0; y < nty; ++y)
-            for (int x = 0; x < ntx; ++x) {
-                bool in = false;
-                for (int b = 0; b < n_beams && !in; ++b) {
-                    const PbBeamGeom &B = beams[b].geom;
-                    const float *q = spot_boxes + 4 * b;
-                    if (!(q[0] <= q[1] && q[2] <= q[3])) continue;   // no spots
-                    const float px = (kLine * (x + 0.5f) - 0.5f) * g.spacing - B.iso[0];
-                    const float py = (kLineTY * (y + 0.5f) - 0.5f) * g.spacing - B.iso[1];
-                    const float pz = (kLineTZ * (z + 0.5f) - 0.5f) * g.spacing - B.iso[2];
-                    const float xt = px * B.costa - pz * B.sinta;
-                    const float hy = px * B.sinta + pz * B.costa;
-                    const float hx = -(xt * B.cosga + py * B.singa);
-                    const float hz = py * B.cosga - xt * B.singa;
-                    const float gx = 1.0f - hz / B.vsadx, gy = 1.0f - hz / B.vsady;
-                    in = hx > fminf(q[0] * gx, q[1] * gx) - reach &&
-                         hx < fmaxf(q[0] * gx, q[1] * gx) + reach &&
-                         hy > fminf(q[2] * gy, q[3] * gy) - reach &&
-                         hy < fmaxf(q[2] * gy, q[3] * gy) + reach;
+    unsigned char any[kSplitMaxTiles] = {};
+    SplitTiles T = {};
+    T.tiles = ntx * nty * ntz;
+    for (int b = 0; b < n_beams; ++b) {
+        const PbBeamGeom &B = beams[b].geom;
+        const float *q = spot_boxes + 4 * b;
+        if (!(q[0] <= q[1] && q[2] <= q[3]) || beams[b].n_layers <= 0) continue;   // no spots
+        const float ivx = 1.0f / B.vsadx, ivy = 1.0f / B.vsady;
+        const float dx = kLine * g.spacing;
+        for (int z = 0; z < ntz; ++z)
+            for (int y = 0; y < nty; ++y) {
+                // the row's first tile centre, and the step to the next
+                const float px = (0.5f * kLine - 0.5f) * g.spacing - B.iso[0];
+                const float py = (kLineTY * (y + 0.5f) - 0.5f) * g.spacing - B.iso[1];
+                const float pz = (kLineTZ * (z + 0.5f) - 0.5f) * g.spacing - B.iso[2];
+                const float xt = px * B.costa - pz * B.sinta;
+                const float hx = -(xt * B.cosga + py * B.singa);
+                const float hy = px * B.sinta + pz * B.costa;
+                const float hz = py * B.cosga - xt * B.singa;
+                const float sx = -dx * B.costa * B.cosga, sy = dx * B.sinta;
+                const float sz = -dx * B.costa * B.singa;
+                unsigned char *row = any + ntx * (y + nty * z);
+                int n = 0;
+                for (int x = 0; x < ntx; ++x) {
+                    const float X = hx + sx * x, Y = hy + sy * x, Z = hz + sz * x;
+                    const float gx = 1.0f - Z * ivx, gy = 1.0f - Z * ivy;
+                    const float xa = q[0] * gx, xb = q[1] * gx, ya = q[2] * gy, yb = q[3] * gy;
+                    const int in = (X > std::min(xa, xb) - reach) & (X < std::max(xa, xb) + reach) &
+                                   (Y > std::min(ya, yb) - reach) & (Y < std::max(ya, yb) + reach);
+                    row[x] |= (unsigned char)in;
+                    n += in;
                 }
-                active += in;
+                T.reached[b] += n;
             }
-    *forward = active < 500 ? 4 : active < 900 ? 2 : 1;
-    *adjoint = active < 900 ? 4 : active < 1500 ? 2 : 1;
+    }
+    for (int t = 0; t < T.tiles; ++t) T.active += any[t];
+    *forward = split_of(T, beams, n_beams, kSplitForward);
+    *adjoint = split_of(T, beams, n_beams, kSplitAdjoint);
+    *positions = split_of(T, beams, n_beams, kSplitPositions);
 }
 
 size_t tile_order_work_size(const PbGrid &g)

@@ -104,9 +104,10 @@ PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
 long long tile_order_count(const PbGrid &g);
 void tile_order_tile(int *voxels);
 size_t tile_order_work_size(const PbGrid &g);
-// Blocks per tile for the forward and the adjoint (pb_tile_split).
+// Blocks per tile for the forward, the weight gradient and the position
+// gradients (pb_tile_split, pb_tile_split_positions).
 void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
-                int *forward, int *adjoint);
+                int *forward, int *adjoint, int *positions);
 PbStatus launch_tile_order(const PbGrid &g, const PbBeam *beams, int n_beams, const float *wet,
                            const PbLayer *layers, void *work, int *order, cudaStream_t st);
 

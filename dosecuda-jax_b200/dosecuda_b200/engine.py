@@ -272,6 +272,11 @@ class DevicePlan:
         boxes = np.array([(g[:, 0].min(), g[:, 0].max(), g[:, 1].min(), g[:, 1].max()) if len(g)
                           else (1.0, -1.0, 1.0, -1.0) for g in geo_blocks], np.float32)
         self._split, self._split_adjoint = self._tile_split(0, self.n_beams, boxes)
+        positions = ctypes.c_int(1)
+        check(_lib.lib.pb_tile_split_positions(ctypes.byref(self.grid), self._beam_ptr(0),
+                                               self.n_beams, ptr(boxes), ctypes.byref(positions)),
+              "pb_tile_split_positions")
+        self._split_positions = positions.value
         self._beam_split = [self._tile_split(b, 1, boxes)[0] for b in range(self.n_beams)]
         # per-layer culling bounds (spot box, halo and MCS sigma bounds) on the device
         if self.layer_offsets[-1]:
@@ -532,7 +537,7 @@ class DevicePlan:
         check(_lib.lib.pb_dose_adjoint_positions_split(
             ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
             ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu), ptr(w), float(scale),
-            ptr(g), ptr(gx), ptr(gy), ptr(order), self._split_adjoint, _stream(self.device)),
+            ptr(g), ptr(gx), ptr(gy), ptr(order), self._split_positions, _stream(self.device)),
             "pb_dose_adjoint_positions_split")
         return g[: self.n_spots], gx[: self.n_spots], gy[: self.n_spots]
 

@@ -255,7 +255,7 @@ PbStatus pb_dose_adjoint_positions(const PbGrid *grid, const PbBeam *beams, int 
                                    const float *dobj_dose_dev, float scale, float *grad_dev,
                                    float *grad_x_dev, float *grad_y_dev, void *stream);
 /* The same in a given tile order (pb_tile_order; NULL: none), each tile shared
- * by `split` blocks (1, 2 or 4: pb_tile_split's for the adjoint). */
+ * by `split` blocks (1, 2 or 4: pb_tile_split_positions). */
 PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                                          const float *wet_dev, const PbLayer *layers_dev,
                                          const float *spot_geo_dev, const float *mu_dev,
@@ -402,13 +402,17 @@ PbStatus pb_dose_adjoint_ordered(const PbGrid *grid, const PbBeam *beams, int n_
                                  void *stream);
 
 /* Blocks per tile for pb_dose_split and pb_dose_adjoint_split (1, 2 or 4),
- * from how many tiles the beams reach: where those are fewer than the GPU
- * has places for blocks, sharing a tile's layers among several blocks
- * shortens the launch.  Host only.  spot_boxes: per beam the least and
+ * from how many tiles the beams reach and their layers and spots: where the
+ * tiles are fewer than the GPU has places for blocks and have layers to share,
+ * several blocks a tile shorten the launch.  Host only.  Of `beams` the
+ * geometry and the counts are read; spot_boxes: per beam the least and
  * greatest spot x, then y, at the isocentre plane (mm; least > greatest for
  * a beam without spots).  No counterpart in the reference. */
 PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                        const float *spot_boxes, int *forward_out, int *adjoint_out);
+/* The same for pb_dose_adjoint_positions_split. */
+PbStatus pb_tile_split_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                 const float *spot_boxes, int *positions_out);
 /* pb_dose_ordered (without per-beam doses) and pb_dose_adjoint_ordered with
  * each tile of the default shape shared by `split` blocks (1, 2 or 4).  The
  * dose is the same bits for every split, the gradient the same to float

@@ -268,3 +268,47 @@ def test_tile_order_split_by_z_slabs(dims, n_parts):
         seen.append(listed)
     allt = torch.cat(seen).sort().values
     assert torch.equal(allt, torch.arange(n, dtype=torch.int32))
+
+
+def _split(shape, spacing, beams):
+    """pb_tile_split of beams at gantry angles, (angle, layers, spots a layer,
+    half width of the spots' box), aimed at the grid's centre."""
+    from dosecuda_b200 import _lib
+    nx, ny, nz = shape
+    g = _lib.PbGrid(nx, ny, nz, spacing)
+    B = (_lib.PbBeam * len(beams))()
+    box = np.empty((len(beams), 4), np.float32)
+    for b, (angle, layers, spots, half) in enumerate(beams):
+        B[b].geom = _lib.beam_setup(angle, 0.0, 1340.0, 1930.0,
+                                    0.5 * spacing * np.array(shape, np.float32), [0, 0, 0])
+        B[b].n_layers, B[b].n_spots = layers, layers * spots
+        box[b] = (-half, half, -half, half)
+    f, a = ctypes.c_int(-1), ctypes.c_int(-1)
+    _lib.check(_lib.lib.pb_tile_split(ctypes.byref(g), ctypes.cast(B, ctypes.c_void_p), len(beams),
+                                      _lib.ptr(box), ctypes.byref(f), ctypes.byref(a)))
+    return f.value, a.value
+
+
+@pytest.mark.parametrize("n", [40, 64, 96, 150])
+@pytest.mark.parametrize("n_beams", [1, 4])
+@pytest.mark.parametrize("spots", [1, 20, 500])
+def test_tile_split_needs_layers_to_share(n, n_beams, spots):
+    """A beam of one layer has nothing to share among a tile's blocks, one of
+    two layers nothing for a third; a small plan of many layers has."""
+    def at(layers, half=20.0):
+        return _split((n, n, n), 3.0, [(90.0 * b, layers, spots, half) for b in range(n_beams)])
+    assert at(1) == (1, 1)
+    assert max(at(2)) <= 2
+    assert at(0) == (1, 1) and at(12, -1.0) == (1, 1)      # no layer, no spot box
+    if n == 40:
+        assert at(12) == (4, 4)
+
+
+def test_tile_split_counts_work_and_grid():
+    many = [(0.0, 12, 500, 60.0)]
+    assert _split((264, 256, 256), 1.0, many) == (1, 1)    # more than 4096 tiles
+    assert _split((256, 256, 64), 3.0, [(90.0 * b, 16, 30, 110.0) for b in range(4)])[0] == 1
+    # uneven beams: a beam of one layer beside one of twelve
+    assert _split((40, 40, 40), 3.0, [(0.0, 12, 100, 20.0), (90.0, 1, 100, 20.0)]) == (4, 4)
+    # the reached tiles alone: a small target in a wide grid
+    assert _split((160, 160, 24), 3.0, [(0.0, 12, 100, 20.0)])[1] == 4
