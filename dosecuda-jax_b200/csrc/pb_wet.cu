@@ -175,9 +175,9 @@ __device__ __forceinline__ float ray_sample(const float *__restrict__ rho,
 // flight per thread.
 //
 // Volumes are of two kinds (cells_dense, counted when the records are made).
-// Where most cells are flat (phantoms, a CT without noise) a ray is a chain of
-// record loads with a few fetches between, and the kernel lives on occupancy.
-// Where a quarter or more are not (a CT with image noise) nearly every sample
+// Where rays meet flat cells (phantoms, a CT whose air is clean) a ray is a chain
+// of record loads with fetches between, and the kernel lives on occupancy.
+// Where hardly any cell is flat (image noise everywhere) nearly every sample
 // is fetched, and the texture unit's rate bounds it: there some samples come
 // from the records (cell_sample2).  Each kind has its own kernel, and the
 // launch of the other one ends at once: the host does not wait for the count.
@@ -357,11 +357,20 @@ __device__ __forceinline__ float2 cell_sample2(const RayCells &C, const CellInde
     return make_float2(out[0], out[1]);
 }
 
-// Whether the volume's cells are dense: a quarter of them or more not flat.
+// Whether the volume's cells are dense: 85 % of them or more not flat.  Below
+// that the rays that leave through flat cells make the sparse kernel the faster
+// one: us of the ray trace, sparse / dense, of volumes whose body has noise and
+// whose air has none, by the share of cells that are not flat:
+//     96 x  87 x  68, 2 beams   0.27 164 / 239, 0.56 241 / 317, 0.83  280 /  252
+//    130 x 121 x  85, 2 beams   0.25 378 / 587, 0.54 652 / 874, 0.83  891 / 1021,
+//                               0.87 898 / 823
+//    220 x 211 x 130, 3 beams   0.52 5360 / 5505, 0.81 7353 / 6804, 0.91 7796 / 6420
+// and of phantoms without noise, where surfaces alone are not flat (0.09 to 0.28):
+// the dense kernel takes 1.6 to 2.3 times as long.
 __device__ __forceinline__ bool cells_dense(const unsigned int *odd, const PbGrid &g)
 {
     const long long n = (long long)(g.nx + 1) * (g.ny + 1) * (g.nz + 1);
-    return 4ll * (long long)__ldg(odd + 1) >= n;
+    return 20ll * (long long)__ldg(odd + 1) >= 17ll * n;
 }
 
 // Samples of a burst, fetched together.
