@@ -387,9 +387,15 @@ constexpr int kThick = 3, kByCells = 2, kMaxBursts = 8;
 // phantom), dense 7 (72; 5, 6 and 8 took 7.93, 7.82 and 8.08 ms on the CT above
 // against 7.62), exact weights 6 (80).
 constexpr int kSparseBlocks = 12, kDenseBlocks = 7, kExactBlocks = 6;
-// Bricks a block takes in turn where there are many (75,776 or more): the launch
-// that finds the volume of the other kind then ends in a few us.
+// Bricks a block takes in turn where there are many: the launch that finds the
+// volume of the other kind then ends in a few us (0.55 ns a block).  Up to
+// kEachBricks the sparse kernel has a block per brick: us, a loop over bricks
+// against a block each, 50x111x55, 4 beams 187 / 183; 96x87x68, 2 beams, noise in
+// the body 241 / 239; 180x171x110, 3 beams (83,000 bricks) 2587 / 2511;
+// 256x256x160, 4 beams, phantom 3640 / 3729.  (One brick index in a row, divided by
+// the three extents in the kernel, cost 8 % of a small volume's ray trace.)
 constexpr int kBricksPerBlock = 8;
+constexpr int64_t kEachBricks = 148 * 1024;
 
 template <bool TEX, bool DENSE>
 __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
@@ -584,26 +590,31 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
     return __double2float_rn(fma(0.1, acc, -0.05));
 }
 
-template <bool TEX, bool DENSE>
+// EACH: a block per brick.  Otherwise a block takes the bricks of its row and
+// column in every gridDim.z-th plane (and, past the grid's limit, row).
+template <bool TEX, bool DENSE, bool EACH>
 __global__ void __launch_bounds__(128, !DENSE ? kSparseBlocks : TEX ? kDenseBlocks : kExactBlocks)
 k_raytrace(const float *__restrict__ rho, cudaTextureObject_t tex, const RayCells rec,
            PbGrid g, const __grid_constant__ BeamGeomSet bs, int n_beams, int cap,
            float *__restrict__ raw, int *status)
 {
     if (TEX && rec.quad && cells_dense(rec.odd, g) != DENSE) return;   // the other launch's
-    const int bx = (g.nx + 7) / 8, by = (g.ny + 3) / 4, bz = (g.nz + 3) / 4;
+    const unsigned by = (g.ny + 3) / 4, bz = (g.nz + 3) / 4;
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
-    const int n = bx * by * bz * n_beams;
-    for (int q = blockIdx.x; q < n; q += gridDim.x) {
-        int r = q;
-        const int i = r % bx * 8 + (threadIdx.x & 7);
-        r /= bx;
-        const int j = r % by * 4 + ((threadIdx.x >> 3) & 3);
-        r /= by;
-        const int k = r % bz * 4 + (threadIdx.x >> 5), b = r / bz;
-        if (i >= g.nx || j >= g.ny || k >= g.nz) continue;
+    const int i = blockIdx.x * 8 + (threadIdx.x & 7);
+    if (i >= g.nx) return;
+    auto brick = [&](unsigned y, unsigned z) {
+        const int j = y * 4 + ((threadIdx.x >> 3) & 3);
+        const int b = z / bz, k = (z - b * bz) * 4 + (threadIdx.x >> 5);
+        if (j >= g.ny || k >= g.nz) return;
         const int64_t v = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
         raw[b * V + v] = raytrace_voxel<TEX, DENSE>(rho, tex, rec, g, bs.b[b], i, j, k, cap, status);
+    };
+    if constexpr (EACH) {
+        brick(blockIdx.y, blockIdx.z);
+    } else {
+        for (unsigned y = blockIdx.y; y < by; y += gridDim.y)
+            for (unsigned z = blockIdx.z; z < bz * n_beams; z += gridDim.z) brick(y, z);
     }
 }
 
@@ -1232,21 +1243,34 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
     for (int b = 0; b < n_beams; ++b) bs.b[b] = beams[b];
     SmoothSet ss;
     smooth_set(g, beams, n_beams, ss);
-    const int64_t bricks = (int64_t)((g.nx + 7) / 8) * ((g.ny + 3) / 4) * ((g.nz + 3) / 4) * n_beams;
+    const int64_t bx = (g.nx + 7) / 8, by = (g.ny + 3) / 4;
+    const int64_t planes = (int64_t)((g.nz + 3) / 4) * n_beams, bricks = bx * by * planes;
     if (bricks > INT32_MAX) return set_error(PB_ERR_INVALID, "grid too large");
-    const int64_t some = (bricks + kBricksPerBlock - 1) / kBricksPerBlock;
-    const unsigned rg = (unsigned)(bricks < 148 * 512 ? bricks : some);
-    // small dense volumes: enough blocks that each SM takes several in turn
-    const unsigned dg = (unsigned)std::min(bricks, std::max<int64_t>(148 * 8 * kDenseBlocks, some));
+    const int64_t limit = 65535;   // of a launch's y and z
+    // about `blocks` blocks: all of a plane's bricks, every so many planes
+    auto some = [&](int64_t blocks) {
+        const int64_t z = std::min(std::max<int64_t>((blocks + bx * by - 1) / (bx * by), 1), planes);
+        return dim3((unsigned)bx, (unsigned)std::min(by, limit), (unsigned)std::min(z, limit));
+    };
+    const int64_t eighth = (bricks + kBricksPerBlock - 1) / kBricksPerBlock;
+    const bool each = bricks <= kEachBricks && by <= limit && planes <= limit;
+    const dim3 all((unsigned)bx, (unsigned)by, (unsigned)planes);
     const int cap = ray_step_cap(g);
     if (tex) {
-        k_raytrace<true, false><<<rg, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
+        if (each)
+            k_raytrace<true, false, true><<<all, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap,
+                                                               raw, status);
+        else
+            k_raytrace<true, false, false><<<some(eighth), 128, 0, st>>>(rlsp, tex, rec, g, bs,
+                                                                         n_beams, cap, raw, status);
         if (rec.quad)
-            k_raytrace<true, true><<<dg, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap, raw,
-                                                       status);
+            // small volumes: enough blocks that each SM takes several in turn
+            k_raytrace<true, true, false>
+                <<<some(std::max<int64_t>(148 * 8 * kDenseBlocks, eighth)), 128, 0, st>>>(
+                    rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
     } else {
-        k_raytrace<false, true><<<rg, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap, raw,
-                                                    status);
+        k_raytrace<false, true, false><<<some(each ? bricks : eighth), 128, 0, st>>>(
+            rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
     }
     PbStatus s = check_launch("k_raytrace");
     if (s != PB_OK) return s;

@@ -194,3 +194,23 @@ def test_refilling_a_handle_with_the_other_kind():
     for vol in vols:
         got = _raw(dp, vol)
         assert torch.equal(got, _raw(_texture_plan(shape, 2.0, 21.0), vol))
+
+
+@pytest.mark.parametrize("planes", [0, 30, 128])
+@pytest.mark.parametrize("mode", ["texture", "exact"])
+def test_many_bricks_give_each_beams_depths(planes, mode):
+    """A launch with more bricks than get a block each (16 beams), one with a
+    block each (a beam alone), sparse and dense: the same bits."""
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_impt import IMPTPlan
+    shape = (121, 126, 123)
+    vol = torch.as_tensor(_half_noisy(shape, min(planes, shape[0])), device=DEV).reshape(-1)
+    iso = np.array(shape[::-1], np.float32)
+    spots = np.array([[0.0, 0.0, 1.0, 30.0]], np.float32)
+    model = IMPTPlan().beam_models[0]
+    beams = [engine.BeamSpec(22.5 * b, 7.0 * (b % 3), iso, spots, model) for b in range(16)]
+    dp = engine.DevicePlan(shape, 2.0, np.zeros(3, np.float32), beams, DEV)
+    wet = dp.compute_wet(vol, wet_mode=mode)
+    for b in (0, 5, 15):
+        one = engine.DevicePlan(shape, 2.0, np.zeros(3, np.float32), [beams[b]], DEV)
+        assert torch.equal(one.compute_wet(vol, wet_mode=mode)[0], wet[b])
