@@ -868,15 +868,19 @@ __device__ __forceinline__ float smooth_voxel(const float *__restrict__ R, const
 
 // The voxels whose every sample lies in the grid (the table's margins) and the
 // shell around them are different blocks of the launch.  Inside, a thread takes
-// kSmoothPer voxels 32 apart in memory, a warp 32 * kSmoothPer consecutive ones: a
+// PER voxels 32 apart in memory, a warp 32 * PER consecutive ones: a
 // sample's table entry, its test for a flagged axis and its address are formed
-// once for the four, whose loads differ by a constant, and a warp's load is one
+// once for them, whose loads differ by a constant, and a warp's load is one
 // run of 128 bytes.  One voxel a thread in 8x4x4 bricks, interior or not, spent
 // some 20 instructions on a sample that is not flagged (issue slots 87 % used) and
 // four L1 wavefronts on each load.  256x256x160, 4 beams along the axes (18 of 54
 // samples flagged): 2.28 -> 1.7 ms; 200x188x160, 3 oblique beams: 0.93 -> 0.46 ms.
-constexpr int kSmoothPer = 4;   // (smooth_block names the four)
-constexpr int kSmoothBlock = 128 * kSmoothPer;   // voxels of a block inside
+//
+// PER is 4, or 2 where fours would fill the GPU less than twice (kSmoothFew): then
+// the chain of a thread's samples is the launch's length.  us, one voxel a thread /
+// 2 / 4: 96x88x72, 1 beam 42 / 26 / 35; 322,000 voxels, 1 beam 36 / 27 / 46;
+// 421,000, 2 beams 62 / 36 / 50; 305,000, 4 beams 93 / 82 / 91; 572,000, 2 beams
+// 87 / 48 / 49; 1,351,000, 2 beams 178 / 157 / 129.
 
 // The inner box of a grid: voxels m[a] .. n[a] - 1 - m[a] of each axis, or none;
 // the blocks of the inside (over the whole volume) and of the shell.
@@ -885,6 +889,7 @@ struct SmoothBox {
     long long inner, shell;        // blocks
 };
 
+template <int PER>
 __host__ __device__ __forceinline__ SmoothBox smooth_box(const PbGrid &g, const int *margin)
 {
     SmoothBox X;
@@ -897,7 +902,7 @@ __host__ __device__ __forceinline__ SmoothBox smooth_box(const PbGrid &g, const 
     X.mz = some ? margin[2] : g.nz;
     const long long in = some ? (long long)(g.nx - 2 * X.mx) * (g.ny - 2 * X.my) *
                                     (g.nz - 2 * X.mz) : 0;
-    X.inner = some ? (V + kSmoothBlock - 1) / kSmoothBlock : 0;
+    X.inner = some ? (V + 128 * PER - 1) / (128 * PER) : 0;
     X.shell = (V - in + 127) / 128;
     return X;
 }
@@ -943,14 +948,14 @@ __device__ __forceinline__ bool shell_voxel(const PbGrid &g, const SmoothBox &X,
     return true;
 }
 
-template <bool POW2>
+template <bool POW2, int PER>
 __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const PbGrid &g,
                                              const PbBeamGeom &Bp, const SmoothBeam &T,
                                              const float *dc, const float *ds, long long block,
                                              float *__restrict__ out)
 {
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
-    const SmoothBox X = smooth_box(g, T.margin);
+    const SmoothBox X = smooth_box<PER>(g, T.margin);
     const PbBeamGeom B = Bp;   // the rotation and isocentre in registers
     const float s = g.spacing;
     int i, j, k;
@@ -962,7 +967,7 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
                                             : c;
         return;
     }
-    const int v0 = (int)block * kSmoothBlock + (threadIdx.x >> 5) * (32 * kSmoothPer) +
+    const int v0 = (int)block * (128 * PER) + (threadIdx.x >> 5) * (32 * PER) +
                    (threadIdx.x & 31);
     if (v0 >= V) return;
     {
@@ -971,17 +976,17 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
         k = (int)(row / (unsigned)g.ny);
         j = (int)(row - (unsigned)k * (unsigned)g.ny);
     }
-    // Whether every sample of the four, at either candidate, lies in the
+    // Whether every sample of the PER, at either candidate, lies in the
     // volume's memory: then the loads need no tests.  What a voxel of the shell
     // reads so is not used.
     const int64_t reach = X.mx + (int64_t)g.nx * (X.my + (int64_t)g.ny * X.mz);
-    const bool whole = v0 >= reach && v0 + 32 * (kSmoothPer - 1) + reach < V;
-    float center[kSmoothPer], sum[kSmoothPer], hx[kSmoothPer], hy[kSmoothPer], hz[kSmoothPer];
-    float fi[kSmoothPer], fj[kSmoothPer], fk[kSmoothPer];
-    int nr[kSmoothPer];        // radii of each voxel, -1: not inside
+    const bool whole = v0 >= reach && v0 + 32 * (PER - 1) + reach < V;
+    float center[PER], sum[PER], hx[PER], hy[PER], hz[PER];
+    float fi[PER], fj[PER], fk[PER];
+    int nr[PER];        // radii of each voxel, -1: not inside
     bool inner = false;
 #pragma unroll
-    for (int m = 0; m < kSmoothPer; ++m) {
+    for (int m = 0; m < PER; ++m) {
         if (m > 0) {
             i += 32;
             while (i >= g.nx) {
@@ -1016,7 +1021,7 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
                 for (int r = 0; r < 9; ++r) {
                     const float *q = at + T.off[dd][r];
 #pragma unroll
-                    for (int m = 0; m < kSmoothPer; ++m) {
+                    for (int m = 0; m < PER; ++m) {
                         const float x = __ldg(q + 32 * m);
                         sum[m] = r < nr[m] ? __fadd_rn(sum[m], x) : sum[m];
                     }
@@ -1028,7 +1033,7 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
             for (int r = 0; r < 9; ++r) {
                 const int axes = (tm >> (3 * r)) & 7u;
                 const float *q = at + T.off[dd][r];
-                float x[kSmoothPer] = {};
+                float x[PER] = {};
                 // One flagged axis, the usual case (beams along the image
                 // axes): exact_steps' operations for it alone, with what does
                 // not change over the samples in registers.  The candidate is
@@ -1037,7 +1042,7 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
                     constexpr int A = decltype(a)::value;
                     const float hh = T.hh[dd][r][A], dr = (float)(r + 1);
 #pragma unroll
-                    for (int m = 0; m < kSmoothPer; ++m) {
+                    for (int m = 0; m < PER; ++m) {
                         const float xz = -__fmaf_rn(dr, c, hx[m]);
                         float p;
                         if constexpr (A == 1) {
@@ -1062,29 +1067,32 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
                     one_axis(std::integral_constant<int, 2>{}, sz);
                 } else if (axes) {
 #pragma unroll 1
-                    for (int m = 0; m < kSmoothPer; ++m) {
+                    for (int m = 0; m < PER; ++m) {
                         int ui = 0, uj = 0, uk = 0;
                         auto of = [&](const float *v) {   // no indexed registers
-                            return m == 0 ? v[0] : m == 1 ? v[1] : m == 2 ? v[2] : v[3];
+                            float r = v[0];
+#pragma unroll
+                            for (int l = 1; l < PER; ++l) r = l == m ? v[l] : r;
+                            return r;
                         };
                         exact_steps<POW2>(B, T, s, dc, ds, of(hx), of(hy), of(hz), of(fi), of(fj),
                                           of(fk), dd, r, axes, ui, uj, uk);
                         const float w = __ldg(q + 32 * m + (ui + sy * uj + sz * uk));
 #pragma unroll
-                        for (int l = 0; l < kSmoothPer; ++l) x[l] = l == m ? w : x[l];
+                        for (int l = 0; l < PER; ++l) x[l] = l == m ? w : x[l];
                     }
                 } else {
 #pragma unroll
-                    for (int m = 0; m < kSmoothPer; ++m) x[m] = __ldg(q + 32 * m);
+                    for (int m = 0; m < PER; ++m) x[m] = __ldg(q + 32 * m);
                 }
 #pragma unroll
-                for (int m = 0; m < kSmoothPer; ++m)
+                for (int m = 0; m < PER; ++m)
                     sum[m] = r < nr[m] ? __fadd_rn(sum[m], x[m]) : sum[m];
             }
         }
     }
 #pragma unroll
-    for (int m = 0; m < kSmoothPer; ++m) {
+    for (int m = 0; m < PER; ++m) {
         if (nr[m] < 0) continue;
         float r = nr[m] > 0 ? __fdiv_rn(sum[m], (float)(6 * nr[m] + 1)) : center[m];
         if (!whole && nr[m] > 0)   // the first and last rows inside
@@ -1099,13 +1107,14 @@ __device__ __forceinline__ void smooth_block(const float *__restrict__ R, const 
 // For the batch, whose table is in shared memory, 10: 8.03 ms for a batch of 8 plans
 // against 8.18 (6) and 8.08 (8).
 constexpr int kSmoothBlocks = 9, kSmoothBatchBlocks = 10;
+constexpr int64_t kSmoothFew = 2ll * 148 * kSmoothBlocks * 128 * 4;   // voxels x beams
 // First block of each beam.
 struct SmoothStarts {
     int n;
     unsigned start[PB_MAX_BEAMS];
 };
 
-template <bool POW2>
+template <bool POW2, int PER>
 __global__ void __launch_bounds__(128, kSmoothBlocks)
 k_smooth(const float *__restrict__ raw, PbGrid g, const __grid_constant__ BeamGeomSet bs,
          const __grid_constant__ SmoothSet st,
@@ -1117,7 +1126,7 @@ k_smooth(const float *__restrict__ raw, PbGrid g, const __grid_constant__ BeamGe
     int b = 0;
     while (b + 1 < at.n && blockIdx.x >= at.start[b + 1]) ++b;
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
-    smooth_block<POW2>(raw + b * V, g, bs.b[b], st.b[b], s_dc, s_ds, blockIdx.x - at.start[b],
+    smooth_block<POW2, PER>(raw + b * V, g, bs.b[b], st.b[b], s_dc, s_ds, blockIdx.x - at.start[b],
                        wet + b * V);
 }
 
@@ -1199,9 +1208,9 @@ k_smooth_batch(const BatchWet *__restrict__ items, int n_items)
         dst[q] = __ldg(src + q);
     __syncthreads();
     if (sm.pow2)
-        smooth_block<true>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
+        smooth_block<true, 4>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
     else
-        smooth_block<false>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
+        smooth_block<false, 4>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
 }
 
 __device__ float g_smooth_dirs[12];
@@ -1276,18 +1285,17 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
     if (s != PB_OK) return s;
     SmoothStarts at;
     at.n = n_beams;
+    const bool few = (int64_t)g.nx * g.ny * g.nz * n_beams < kSmoothFew;
     long long blocks = 0;
     for (int b = 0; b < n_beams; ++b) {
         at.start[b] = (unsigned)blocks;
-        const SmoothBox X = smooth_box(g, ss.b[b].margin);
+        const SmoothBox X = few ? smooth_box<2>(g, ss.b[b].margin) : smooth_box<4>(g, ss.b[b].margin);
         blocks += X.inner + X.shell;
         if (blocks > INT32_MAX) return set_error(PB_ERR_INVALID, "grid too large");
     }
-    const unsigned sg = (unsigned)blocks;
-    if (ss.b[0].pow2)
-        k_smooth<true><<<sg, 128, 0, st>>>(raw, g, bs, ss, at, wet);
-    else
-        k_smooth<false><<<sg, 128, 0, st>>>(raw, g, bs, ss, at, wet);
+    auto kernel = ss.b[0].pow2 ? (few ? k_smooth<true, 2> : k_smooth<true, 4>)
+                               : (few ? k_smooth<false, 2> : k_smooth<false, 4>);
+    kernel<<<(unsigned)blocks, 128, 0, st>>>(raw, g, bs, ss, at, wet);
     return check_launch("k_smooth");
 }
 
@@ -1331,7 +1339,7 @@ long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbB
         w.by = by;
         w.bz = bz;
         w.brick_start = start;
-        const SmoothBox X = smooth_box(g, w.sm.margin);
+        const SmoothBox X = smooth_box<4>(g, w.sm.margin);
         w.smooth_blocks = X.inner + X.shell;
         // both launches go by these starts
         start += std::max((long long)bx * by * bz, w.smooth_blocks);

@@ -73,3 +73,19 @@ def test_batch_of_uneven_volumes(oracle):
     for dp, (model, iso, angles, shape, spacing, alone) in zip(plans, more):
         _check(oracle, dp, model, iso, angles, shape, spacing)
         assert torch.equal(dp.wet, alone)
+
+
+@pytest.mark.parametrize("shape,spacing", [((31, 57, 49), 1.0), ((70, 9, 141), 2.5),
+                                           ((24, 240, 15), 2.0)])
+def test_many_beams_as_each_alone(oracle, shape, spacing):
+    """A launch large enough for four voxels a thread (16 beams) and ones that
+    take two (a beam alone)."""
+    angles = [(22.5 * b, 9.0 * (b % 4)) for b in range(16)]
+    assert 16 * int(np.prod(shape)) > 2 * 148 * 9 * 512 / 1.1
+    dp, model, iso = _plan(shape, spacing, angles)
+    dp.compute_wet(_rlsp(shape, 3), wet_mode="exact")
+    _check(oracle, dp, model, iso, angles, shape, spacing)
+    for b in (0, 4, 11):
+        one, _, _ = _plan(shape, spacing, angles[b:b + 1])
+        one.compute_wet(_rlsp(shape, 3), wet_mode="exact")
+        assert torch.equal(one.wet[0], dp.wet[b])
