@@ -906,16 +906,26 @@ PbStatus pb_batch_setup(const PbBatchPlan *plans, int n_plans, void *work_dev,
     }
     // WET records in plan order
     std::vector<unsigned char> wet_items(batch_wet_size() * (size_t)n_plans * PB_MAX_BEAMS);
-    long long bricks = 0;
+    long long bricks = 0, voxel_beams = 0;
+    for (int p = 0; p < n_plans; ++p)
+        voxel_beams += (long long)plans[p].grid.nx * plans[p].grid.ny * plans[p].grid.nz *
+                       plans[p].n_beams;
     int n_wet = 0;
-    for (int p = 0; p < n_plans; ++p) {
-        const PbBatchPlan &P = plans[p];
-        PbBeamGeom geoms[PB_MAX_BEAMS];
-        for (int b = 0; b < P.n_beams; ++b) geoms[b] = P.beams[b].geom;
-        bricks += fill_batch_wet(wet_items.data(), n_wet, P.grid, geoms, P.n_beams, P.rlsp_dev,
-                                 texture_object(P.tex), texture_cells(P.tex), P.raw_work_dev,
-                                 P.wet_dev, bricks);
-        n_wet += P.n_beams;
+    for (bool few : {true, false}) {
+        if (few && voxel_beams / 128 >= batch_wet_few()) continue;
+        bricks = n_wet = 0;
+        for (int p = 0; p < n_plans; ++p) {
+            const PbBatchPlan &P = plans[p];
+            PbBeamGeom geoms[PB_MAX_BEAMS];
+            for (int b = 0; b < P.n_beams; ++b) geoms[b] = P.beams[b].geom;
+            bricks += fill_batch_wet(wet_items.data(), n_wet, P.grid, geoms, P.n_beams,
+                                     P.rlsp_dev, texture_object(P.tex), texture_cells(P.tex),
+                                     P.raw_work_dev, P.wet_dev, bricks, few);
+            n_wet += P.n_beams;
+        }
+        // not a small batch: its count says so, if need be by blocks without work
+        if (!few) bricks = std::max(bricks, batch_wet_few());
+        if (bricks < batch_wet_few()) break;
     }
     // dose records, most expensive tiles first (spots over all beams)
     std::vector<int> order((size_t)n_plans);

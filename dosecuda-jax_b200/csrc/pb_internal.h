@@ -59,7 +59,11 @@ void smooth_table_host(const PbGrid &g, const PbBeamGeom *beams, int n_beams, in
 size_t batch_wet_size();
 long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbBeamGeom *beams,
                          int n_beams, const float *rlsp, cudaTextureObject_t tex,
-                         const RayCells &rec, float *raw, float *wet, long long brick_start);
+                         const RayCells &rec, float *raw, float *wet, long long brick_start,
+                         bool few);
+// A batch of fewer bricks than this is smoothed with two voxels a thread
+// (fill_batch_wet's few); its launch goes by the count.
+long long batch_wet_few();
 PbStatus launch_wet_batch(const void *items_dev, int n_items, long long n_bricks, int *status,
                           cudaStream_t st);
 

@@ -1191,6 +1191,7 @@ k_raytrace_batch(const BatchWet *__restrict__ items, int n_items, int *status)
     W.raw[i + (int64_t)W.g.nx * (j + (int64_t)W.g.ny * k)] = r;
 }
 
+template <int PER>
 __global__ void __launch_bounds__(128, kSmoothBatchBlocks)
 k_smooth_batch(const BatchWet *__restrict__ items, int n_items)
 {
@@ -1208,9 +1209,9 @@ k_smooth_batch(const BatchWet *__restrict__ items, int n_items)
         dst[q] = __ldg(src + q);
     __syncthreads();
     if (sm.pow2)
-        smooth_block<true, 4>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
+        smooth_block<true, PER>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
     else
-        smooth_block<false, 4>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
+        smooth_block<false, PER>(W.raw, W.g, W.geom, sm, s_dc, s_ds, block, W.wet);
 }
 
 __device__ float g_smooth_dirs[12];
@@ -1313,10 +1314,15 @@ void smooth_table_host(const PbGrid &g, const PbBeamGeom *beams, int n_beams, in
 
 size_t batch_wet_size() { return sizeof(BatchWet); }
 
+// Bricks below which a batch's smoothing takes two voxels a thread.
+long long batch_wet_few() { return kSmoothFew / 128; }
+
 // Fills the batch records of one plan's beams; returns the bricks they use.
+// few: for the smoothing with two voxels a thread.
 long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbBeamGeom *beams,
                          int n_beams, const float *rlsp, cudaTextureObject_t tex,
-                         const RayCells &rec, float *raw, float *wet, long long brick_start)
+                         const RayCells &rec, float *raw, float *wet, long long brick_start,
+                         bool few)
 {
     BatchWet *W = static_cast<BatchWet *>(items_host) + first;
     SmoothSet ss;
@@ -1339,7 +1345,7 @@ long long fill_batch_wet(void *items_host, int first, const PbGrid &g, const PbB
         w.by = by;
         w.bz = bz;
         w.brick_start = start;
-        const SmoothBox X = smooth_box<4>(g, w.sm.margin);
+        const SmoothBox X = few ? smooth_box<2>(g, w.sm.margin) : smooth_box<4>(g, w.sm.margin);
         w.smooth_blocks = X.inner + X.shell;
         // both launches go by these starts
         start += std::max((long long)bx * by * bz, w.smooth_blocks);
@@ -1357,7 +1363,10 @@ PbStatus launch_wet_batch(const void *items_dev, int n_items, long long n_bricks
     k_raytrace_batch<true><<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items, status);
     PbStatus s = check_launch("k_raytrace_batch");
     if (s != PB_OK) return s;
-    k_smooth_batch<<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items);
+    if (n_bricks < batch_wet_few())
+        k_smooth_batch<2><<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items);
+    else
+        k_smooth_batch<4><<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items);
     return check_launch("k_smooth_batch");
 }
 

@@ -338,7 +338,7 @@ typedef struct {
 
 /* Sizes of a prepared batch, filled by pb_batch_setup. */
 typedef struct {
-    long long n_bricks;     /* WET work: 8x4x4-voxel bricks over all (plan, beam) */
+    long long n_bricks;     /* WET work: 8x4x4-voxel bricks over all (plan, beam), or more */
     long long n_tiles;      /* dose work: 8x8x8 tiles over all plans              */
     int n_wet_items;        /* (plan, beam) records                              */
     int n_plans;

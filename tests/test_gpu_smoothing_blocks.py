@@ -89,3 +89,28 @@ def test_many_beams_as_each_alone(oracle, shape, spacing):
         one, _, _ = _plan(shape, spacing, angles[b:b + 1])
         one.compute_wet(_rlsp(shape, 3), wet_mode="exact")
         assert torch.equal(one.wet[0], dp.wet[b])
+
+
+@pytest.mark.parametrize("n_plans", [5, 6, 7])
+def test_batches_around_the_two_voxel_line(oracle, n_plans):
+    """Batches of some 1.2 to 1.5 million voxels times beams, smoothed with two
+    and with four voxels a thread: each plan's depths alone."""
+    from dosecuda_b200 import batch
+    angles = [(33.0, 0.0), (90.0, 5.0)]
+    plans, rlsps, alone = [], [], []
+    for q in range(n_plans):
+        shape = (41 + q, 53, 47)
+        dp, model, iso = _plan(shape, 2.0, angles)
+        rlsp = _rlsp(shape, q)
+        dp.compute_wet(rlsp, wet_mode="texture" if q % 2 else "exact")
+        alone.append(dp.wet.clone())
+        plans.append(dp)
+        rlsps.append(rlsp)
+        if q == 0:
+            _check(oracle, dp, model, iso, angles, shape, 2.0)
+    for dp in plans:
+        dp.wet.fill_(float("nan"))
+    batch.BatchPlans(plans, rlsps).run()
+    torch.cuda.synchronize()
+    for dp, wet in zip(plans, alone):
+        assert torch.equal(dp.wet, wet)
