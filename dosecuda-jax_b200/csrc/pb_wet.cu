@@ -387,6 +387,11 @@ constexpr int kThick = 3, kByCells = 2, kMaxBursts = 8;
 // phantom), dense 7 (72; 5, 6 and 8 took 7.93, 7.82 and 8.08 ms on the CT above
 // against 7.62), exact weights 6 (80).
 constexpr int kSparseBlocks = 12, kDenseBlocks = 7, kExactBlocks = 6;
+// The batch's sparse kernel keeps its item too and spills at 12: two plans of
+// 48x52x45, 1 beam 56 us at 12 blocks, 50 at 10, 47 at 9, 46 at 8; eight of 64x68x61,
+// 2 beams 220, 210, 210, 210; four of up to 1.6 million voxels, 1 beam 650, 630, 638,
+// 635.
+constexpr int kSparseBatchBlocks = 9;
 // Bricks a block takes in turn where there are many: the launch that finds the
 // volume of the other kind then ends in a few us (0.55 ns a block).  Up to
 // kEachBricks the sparse kernel has a block per brick: us, a loop over bricks
@@ -1175,7 +1180,7 @@ __device__ __forceinline__ bool brick_voxel(const BatchWet &W, long long brick, 
 // The items whose volume is the launch's kind, as k_raytrace (exact sampling
 // goes with the dense ones).
 template <bool DENSE>
-__global__ void __launch_bounds__(128, DENSE ? kDenseBlocks : kSparseBlocks)
+__global__ void __launch_bounds__(128, DENSE ? kDenseBlocks : kSparseBatchBlocks)
 k_raytrace_batch(const BatchWet *__restrict__ items, int n_items, int *status)
 {
     const BatchWet &W = items[find_wet_item(items, n_items, blockIdx.x)];
