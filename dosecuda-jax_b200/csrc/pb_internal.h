@@ -46,9 +46,8 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
                     const PbGrid &g, const PbBeamGeom *beams, int n_beams, float *raw,
                     float *wet, int *status, cudaStream_t st);
 
-PbStatus launch_texture_sample(cudaTextureObject_t tex, const RayCells &rec, const PbGrid &g,
-                               const float *at, int64_t pairs, float *unit, float *cells,
-                               cudaStream_t st);
+PbStatus launch_texture_sample(cudaTextureObject_t tex, const PbGrid &g, const float *at,
+                               int64_t pairs, float *unit, float *cells, cudaStream_t st);
 
 // Batched WET pass (pb_wet.cu): one record per (plan, beam).
 // The smoothing sample table of one beam (pb_wet.cu), as the WET launch

@@ -216,7 +216,7 @@ __host__ __device__ __forceinline__ int cell_row(int nx) { return (nx + 1 + 3) &
 //         cell_row(nx) bytes
 //   odd   not 0 where a texel is infinite or not a number: the unit leaves out
 //         texels of weight 0, which the products below do not, so it samples
-//         such a volume itself
+//         such a volume itself; nor where an axis has kFixLimit voxels or more
 struct CellIndex {
     int cx, cxy;      // quad strides per row and per plane
     unsigned off;     // takes the biased integers of the float adders out
@@ -239,9 +239,11 @@ __device__ __forceinline__ float flat_run(const RayCells &C, const CellIndex &I,
 {
     const int i = floor_small(__fsub_rn(x, 0.5f)) + 1, j = floor_small(__fsub_rn(y, 0.5f)) + 1,
               k = floor_small(__fsub_rn(z, 0.5f)) + 1;
-    const int d = __ldg(C.dist + (unsigned)(i + drow * (j + cy * k)));
+    // (up to 2^32 - 1 entries, twice the cells that a handle takes)
+    const unsigned ui = i, uj = j, uk = k;
+    const int d = __ldg(C.dist + (ui + (unsigned)drow * (uj + (unsigned)cy * uk)));
     if (d < 3) return 0.0f;
-    at = C.quad + (unsigned)(i + I.cx * j + I.cxy * k);
+    at = C.quad + (ui + (unsigned)I.cx * uj + (unsigned)I.cxy * uk);
     // floor((r - 3) / dmax) + 1, every rounding downward so that the run
     // never exceeds the bound
     return floor_small_f(__fmul_rd((float)(d - 3), inv_dmax)) + 1.0f;
@@ -274,6 +276,7 @@ __device__ __forceinline__ float sparse_run(const float2 *__restrict__ rec, int 
 // rounding.  Otherwise exact trilinear weights, in trilinear's operation order
 // bit for bit.
 constexpr float kFixMagic = 6291328.5f;    // 1.5 * 2^22 - 128 + 0.5: an ulp of 0.5
+constexpr int kFixLimit = 8192;            // coordinates that hold in it are below this
 constexpr float kIntMagic = 12582912.0f;   // 1.5 * 2^23: an ulp of 1
 
 template <bool FILTER>
@@ -626,6 +629,21 @@ k_raytrace(const float *__restrict__ rho, cudaTextureObject_t tex, const RayCell
 // Samples at the coordinates of `at` (x, y, z; two per thread), through the
 // texture unit and from the cell records with its filter; only those the
 // records take (inside the grid by the ray trace's margin), the others 0.
+__global__ void k_texture_quads(cudaTextureObject_t tex, PbGrid g, int64_t n,
+                                float4 *__restrict__ quad)
+{
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int cx = g.nx + 1, rows = g.ny + 2;
+    const int i = (int)(q % cx), j = (int)(q / cx % rows), k = (int)(q / cx / rows);
+    // a texel's centre: weight 1 for it, border 0 outside
+    auto texel = [&](int a, int c) {
+        return tex3D<float>(tex, (float)(i - 1 + a) + 0.5f, (float)(j - 1) + 0.5f,
+                            (float)(k - 1 + c) + 0.5f);
+    };
+    quad[q] = make_float4(texel(0, 0), texel(0, 1), texel(1, 0), texel(1, 1));
+}
+
 __global__ void k_texture_sample(cudaTextureObject_t tex, const RayCells rec, PbGrid g,
                                  const float *__restrict__ at, int64_t pairs,
                                  float *__restrict__ unit, float *__restrict__ cells)
@@ -653,14 +671,23 @@ __global__ void k_texture_sample(cudaTextureObject_t tex, const RayCells rec, Pb
     }
 }
 
-PbStatus launch_texture_sample(cudaTextureObject_t tex, const RayCells &rec, const PbGrid &g,
-                               const float *at, int64_t pairs, float *unit, float *cells,
-                               cudaStream_t st)
+// A sparse volume's handle holds no quads (its cells lie there), so they are
+// made here from the texture, for the length of the call.
+PbStatus launch_texture_sample(cudaTextureObject_t tex, const PbGrid &g, const float *at,
+                               int64_t pairs, float *unit, float *cells, cudaStream_t st)
 {
     if (pairs == 0) return PB_OK;
-    k_texture_sample<<<(unsigned)((pairs + 127) / 128), 128, 0, st>>>(tex, rec, g, at, pairs, unit,
-                                                                     cells);
-    return check_launch("k_texture_sample");
+    const int64_t n = (int64_t)(g.nx + 1) * (g.ny + 2) * (g.nz + 1);
+    float4 *quad = nullptr;
+    PbStatus s = check_cuda(cudaMalloc(&quad, sizeof(float4) * n), "cudaMalloc");
+    if (s != PB_OK) return s;
+    k_texture_quads<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(tex, g, n, quad);
+    k_texture_sample<<<(unsigned)((pairs + 127) / 128), 128, 0, st>>>(
+        tex, RayCells{quad, nullptr, nullptr, nullptr}, g, at, pairs, unit, cells);
+    s = check_launch("k_texture_sample");
+    const PbStatus w = check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    cudaFree(quad);
+    return s != PB_OK ? s : w;
 }
 
 // Per-beam table of the smoothing samples.  Sample (direction dd, radius
@@ -1436,7 +1463,7 @@ k_cell_flat(const float *__restrict__ rho, PbGrid g, float4 *__restrict__ quad,
         rough += !f;
         a = b;
     }
-    if (sum != sum) odd[0] = 1;
+    if (sum != sum || max(g.nx, max(g.ny, g.nz)) >= kFixLimit) odd[0] = 1;
     rough = __reduce_add_sync(0xffffffffu, rough);
     if ((threadIdx.x & 31) == 0 && rough) atomicAdd(odd + 1, (unsigned)rough);
 }
@@ -1563,12 +1590,15 @@ k_cell_dist4(PbGrid g, const unsigned int *__restrict__ din, unsigned int *__res
 struct RlspTexture {
     cudaArray_t arr = nullptr;
     cudaTextureObject_t tex = 0;
-    float4 *quad = nullptr;           // cell records (RayCells), or none: no memory for them
-    float2 *cell = nullptr;           // with a texture: value and distance per cell, where the
-                                      // volume is sparse
+    // The cell records (RayCells) and the passes' work arrays, in one allocation,
+    // or none of them: no memory.  The quads of a sparse volume with a texture
+    // are overwritten by its cells, which are all that its ray trace reads.
+    unsigned char *block = nullptr;
+    float4 *quad = nullptr;
+    float2 *cell = nullptr;           // with a texture
     unsigned char *d0 = nullptr, *d1 = nullptr;  // distances, and the passes' other buffer
     unsigned char *flag = nullptr;    // work: flat flags (zero-padded rows)
-    unsigned int *odd = nullptr;      // whether a texel is infinite or not a number
+    unsigned int *odd = nullptr;      // RayCells::odd, and the count of cells not flat
     int nx = 0, ny = 0, nz = 0;
 };
 
@@ -1610,12 +1640,7 @@ static void texture_free(RlspTexture *t)
 {
     if (t->tex) cudaDestroyTextureObject(t->tex);
     if (t->arr) cudaFreeArray(t->arr);
-    cudaFree(t->quad);
-    cudaFree(t->cell);
-    cudaFree(t->d0);
-    cudaFree(t->d1);
-    cudaFree(t->flag);
-    cudaFree(t->odd);
+    cudaFree(t->block);
     delete t;
 }
 
@@ -1640,26 +1665,33 @@ PbStatus texture_create(const float *rlsp, const PbGrid &g, uint64_t *out, cudaS
     // the records of a grid that leaves no memory for them are left out: the
     // ray trace then takes every sample from the texture or the volume
     const size_t nquad = (size_t)(g.nx + 1) * (g.ny + 2) * (g.nz + 1);
-    // (cell_sample2's fixed point holds coordinates below 8192)
-    const bool fits = nquad <= (size_t)INT32_MAX && std::max(g.nx, std::max(g.ny, g.nz)) < 8192;
-    if (s == PB_OK && fits &&
-        (cudaMalloc(&t->quad, sizeof(float4) * nquad) != cudaSuccess ||
-         (with_texture && cudaMalloc(&t->cell, sizeof(float2) * ncell) != cudaSuccess))) {
-        cudaFree(t->quad);
-        t->quad = nullptr;
-        t->cell = nullptr;
-        cudaGetLastError();
-    }
     // distance passes: rows padded to 4 cells (32-bit words)
     const size_t npad = (size_t)cell_row(g.nx) * (g.ny + 1) * (g.nz + 1);
-    if (s == PB_OK) s = check_cuda(cudaMalloc(&t->d0, npad), "cudaMalloc");
-    if (s == PB_OK) s = check_cuda(cudaMalloc(&t->d1, npad), "cudaMalloc");
-    if (s == PB_OK) s = check_cuda(cudaMalloc(&t->odd, 2 * sizeof(*t->odd)), "cudaMalloc");
-    // flat flags: the padding bytes stay zero, the cells are rewritten by
-    // every fill
     const size_t nflag = (size_t)flag_row(g.nx) * (g.ny + 1) * (g.nz + 1);
-    if (s == PB_OK) s = check_cuda(cudaMalloc(&t->flag, nflag), "cudaMalloc");
-    if (s == PB_OK) s = check_cuda(cudaMemset(t->flag, 0, nflag), "cudaMemset");
+    size_t bytes = 0;
+    auto part = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    static_assert(sizeof(float2) <= sizeof(float4), "the cells fit where the quads are");
+    const size_t at_quad = part(sizeof(float4) * nquad), at_d0 = part(npad), at_d1 = part(npad);
+    const size_t at_flag = part(nflag), at_odd = part(2 * sizeof(unsigned int));
+    if (s == PB_OK && cudaMalloc(&t->block, bytes) != cudaSuccess) {
+        t->block = nullptr;
+        cudaGetLastError();
+    }
+    if (s == PB_OK && t->block) {
+        t->quad = reinterpret_cast<float4 *>(t->block + at_quad);
+        if (with_texture) t->cell = reinterpret_cast<float2 *>(t->block + at_quad);
+        t->d0 = t->block + at_d0;
+        t->d1 = t->block + at_d1;
+        t->flag = t->block + at_flag;
+        t->odd = reinterpret_cast<unsigned int *>(t->block + at_odd);
+        // flat flags: the padding bytes stay zero, the cells are rewritten by
+        // every fill
+        s = check_cuda(cudaMemsetAsync(t->flag, 0, nflag, st), "cudaMemsetAsync");
+    }
     if (s == PB_OK && with_texture) {
         cudaResourceDesc rd{};
         rd.resType = cudaResourceTypeArray;

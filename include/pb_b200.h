@@ -147,9 +147,10 @@ PbStatus pb_rlsp_from_hu(const float *hu_dev, int64_t n, const double *curve_hu,
  * holds per-cell records (the texels of each 2x2x2 block, and how far the
  * nearest block is whose texels differ) from which pb_wet adds whole runs of
  * samples through flat regions at once and forms the other samples with the
- * unit's filter (pb_texture_sample compares the two).  They take 27 bytes per
- * voxel (19 without a texture); a grid that leaves no memory for them, or with
- * more than 8191 voxels along an axis, is sampled through the unit alone. */
+ * unit's filter (pb_texture_sample compares the two).  They take 19 bytes per
+ * voxel, in one allocation; a grid that leaves no memory for it is sampled
+ * through the unit alone, and one with more than 8191 voxels along an axis takes
+ * its runs from them and its samples through the unit. */
 typedef uint64_t PbTexture;
 
 PbStatus pb_texture_create(const float *rlsp_dev, const PbGrid *grid,
@@ -166,6 +167,7 @@ PbStatus pb_texture_destroy(PbTexture tex);
  * 2 x pairs coordinates (x, y, z each, unnormalised), through the unit into
  * unit_dev and from the records, as pb_wet takes them, into cells_dev; 0
  * where a coordinate is nearer than 0.003 to the grid's faces or outside.
+ * Synchronous; it allocates the records anew for the length of the call.
  * No counterpart in the reference. */
 PbStatus pb_texture_sample(PbTexture tex, const PbGrid *grid, const float *at_dev, int64_t pairs,
                            float *unit_dev, float *cells_dev, void *stream);

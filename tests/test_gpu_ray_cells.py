@@ -214,3 +214,62 @@ def test_many_bricks_give_each_beams_depths(planes, mode):
     for b in (0, 5, 15):
         one = engine.DevicePlan(shape, 2.0, np.zeros(3, np.float32), [beams[b]], DEV)
         assert torch.equal(one.compute_wet(vol, wet_mode=mode)[0], wet[b])
+
+
+@pytest.mark.parametrize("left", [25.7, 13.0, 2.0])
+def test_grids_that_leave_little_memory(left):
+    """A handle made where only `left` bytes a voxel are free beside its texture:
+    with the records, or without any (pb_texture_create has to succeed), the
+    depths of a handle with records.  Runs of samples and samples one by one
+    add up in FP32 groups of 8 at most: 1e-6 of the largest depth."""
+    shape = (300, 320, 320)
+    v = int(np.prod(shape))
+    vol = np.ones(shape, np.float32)
+    vol[:, 100:180, 60:200] = 1.5
+    dp = _texture_plan(shape, 2.0, 0.0)
+    ref = _raw(dp, vol)
+    rlsp = torch.as_tensor(vol, device=DEV).reshape(-1)
+    del dp
+    dp = _texture_plan(shape, 2.0, 0.0)
+    torch.cuda.synchronize()
+    # the depths' buffers come from torch's cache, the handle from what is left
+    free = torch.cuda.mem_get_info(DEV)[0]
+    hog = torch.empty(int(free - (4.3 + left) * v), dtype=torch.uint8, device=DEV)
+    try:
+        dp.compute_wet(rlsp)
+        torch.cuda.synchronize()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert float((dp.raw_wet.reshape(shape) - ref).abs().max()) <= 1e-6 * float(ref.max())
+
+
+@pytest.mark.parametrize("noise", [0.0, 0.02])
+def test_axis_past_the_filters_fixed_point(noise):
+    """More than 8191 voxels along an axis: exact depths with and without records
+    as above; texture depths within the unit's weights of them, which are off
+    by 1/512 at most on each axis."""
+    from dosecuda_b200 import _lib
+    shape = (6, 7, 8200)
+    rng = np.random.default_rng(3)
+    rho = np.ones(shape, np.float32)
+    rho[:, :, 3000:5000] = 0.25
+    rho += (noise * rng.standard_normal(shape)).astype(np.float32)
+    dp = _texture_plan(shape, 2.0, 0.0)
+    v = torch.as_tensor(rho, device=DEV).reshape(-1).contiguous()
+    dp.compute_wet(v)
+    tex = dp.raw_wet.clone()
+    at, out = torch.zeros(6, device=DEV), torch.zeros(2, device=DEV)
+    stream = ctypes.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)
+    assert _lib.lib.pb_texture_sample(dp._tex, ctypes.byref(dp.grid), _lib.ptr(at), 1,
+                                      _lib.ptr(out), _lib.ptr(out), stream) == _lib.PB_ERR_INVALID
+    dp.compute_wet(v, wet_mode="exact")
+    exact = dp.raw_wet.clone()
+    raw, wet = torch.empty_like(exact), torch.empty_like(exact)
+    _lib.check(_lib.lib.pb_wet(_lib.ptr(v), 0, ctypes.byref(dp.grid),
+                               ctypes.cast(dp.geoms, ctypes.c_void_p), 1, _lib.ptr(raw),
+                               _lib.ptr(wet), None, stream))
+    top = float(raw.max())
+    assert top > 0.5
+    assert float((raw - exact).abs().max()) <= 1e-6 * top
+    assert float((tex - exact).abs().max()) <= 3.0 / 512.0 * float(rho.max()) / 0.2 * top
