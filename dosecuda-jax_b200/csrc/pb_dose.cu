@@ -1108,6 +1108,7 @@ struct LineShared {
     TileBounds tb;                   // the tile's box and depth range for the beam
     float4 step;                     // head-frame step per voxel along x: x, y, and of the
                                      // divergence factors
+    float4 inv;                      // positions: 1/VSADX, 1/VSADY and their difference
     float red[kWarps][kRedSlots];
     int wcount[KCULL][kWarps];
     int wcount_h[KCULL][kWarps];
@@ -1238,14 +1239,13 @@ __device__ __forceinline__ TileBounds corner_bounds(const PbGrid &g, const PbBea
 // quadratic, so each bracket is a quadratic too: a line needs only the moments
 // m0, m1, m2 of its voxels' factors with 1, q', q'^2, and a spot's two
 // derivatives are three products each (out by 2 it2 mu ln2, which the tile's
-// sum is multiplied with).
+// sum is multiplied with).  inv: 1/VSADX, 1/VSADY, k.
 __device__ __forceinline__ void line_position(const LineSpot &r, float Xc, float Yc, float gxc,
                                               float gyc, float S0, float B1, const float4 &step,
-                                              const PbBeamGeom &G, float m0, float m1, float m2,
+                                              const float4 &inv, float m0, float m1, float m2,
                                               float &vx, float &vy)
 {
-    const float ivx = __fdividef(1.0f, G.vsadx), ivy = __fdividef(1.0f, G.vsady);
-    const float kap = __fsub_rn(ivx, ivy);
+    const float ivx = inv.x, ivy = inv.y, kap = inv.z;
     const float kx2 = r.a.x * (ivx * ivx), ky2 = r.a.y * (ivy * ivy);   // -xs/VSADX^2, ...
     // the components at the line's centre and their steps along it
     const float ax = __fmaf_rn(r.a.x, gxc, Xc), ay = __fmaf_rn(r.a.y, gyc, Yc);
@@ -1392,6 +1392,12 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                 if (lane == 0) {
                     sh.tb = tb;
                     sh.step = step;
+                    if constexpr (POS) {
+                        // the reciprocals nearly cancel in their difference
+                        const float ivx = __fdiv_rn(1.0f, B.geom.vsadx);
+                        const float ivy = __fdiv_rn(1.0f, B.geom.vsady);
+                        sh.inv = make_float4(ivx, ivy, __fsub_rn(ivx, ivy), 0.0f);
+                    }
                 }
                 LineLayer Y;
                 bool keep = false;
@@ -1680,7 +1686,7 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                     m2 = __ffma2_rn(__fmul2_rn(o, o), g, m2);
                                 }
                                 v[u] = acc.x + acc.y;
-                                line_position(r, Xc, Yc, gxc, gyc, S0, B1, sh.step, B.geom,
+                                line_position(r, Xc, Yc, gxc, gyc, S0, B1, sh.step, sh.inv,
                                               m0.x + m0.y, m1.x + m1.y, m2.x + m2.y, vx[u], vy[u]);
                             }
                             int slot;
