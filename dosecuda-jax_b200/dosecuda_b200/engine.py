@@ -268,16 +268,11 @@ class DevicePlan:
             B.n_energies = t.n_energies
             B.lut_len = t.lut_len
             B.dvp_len = t.dvp_len
-        # blocks per tile of the plan's launches and of each beam's own
-        boxes = np.array([(g[:, 0].min(), g[:, 0].max(), g[:, 1].min(), g[:, 1].max()) if len(g)
-                          else (1.0, -1.0, 1.0, -1.0) for g in geo_blocks], np.float32)
-        self._split, self._split_adjoint = self._tile_split(0, self.n_beams, boxes)
-        positions = ctypes.c_int(1)
-        check(_lib.lib.pb_tile_split_positions(ctypes.byref(self.grid), self._beam_ptr(0),
-                                               self.n_beams, ptr(boxes), ctypes.byref(positions)),
-              "pb_tile_split_positions")
-        self._split_positions = positions.value
-        self._beam_split = [self._tile_split(b, 1, boxes)[0] for b in range(self.n_beams)]
+        # each beam's spot box, for the blocks per tile of a launch
+        self._spot_boxes = np.array([(g[:, 0].min(), g[:, 0].max(), g[:, 1].min(), g[:, 1].max())
+                                     if len(g) else (1.0, -1.0, 1.0, -1.0) for g in geo_blocks],
+                                    np.float32)
+        self._splits = {}
         # per-layer culling bounds (spot box, halo and MCS sigma bounds) on the device
         if self.layer_offsets[-1]:
             check(_lib.lib.pb_layer_bounds(ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
@@ -285,14 +280,25 @@ class DevicePlan:
                                            _stream(self.device)), "pb_layer_bounds")
         self.spots_loaded = True
 
-    def _tile_split(self, b0: int, n: int, boxes: np.ndarray):
-        """(forward, adjoint) blocks per tile of a launch over beams
-        b0 .. b0 + n - 1 (pb_tile_split); boxes: each beam's spot box."""
-        fwd, adj = ctypes.c_int(1), ctypes.c_int(1)
-        q = np.ascontiguousarray(boxes[b0:b0 + n])
-        check(_lib.lib.pb_tile_split(ctypes.byref(self.grid), self._beam_ptr(b0), n, ptr(q),
-                                     ctypes.byref(fwd), ctypes.byref(adj)), "pb_tile_split")
-        return fwd.value, adj.value
+    def _tile_split(self, kind: str, b0: int = 0, n: Optional[int] = None) -> int:
+        """Blocks per tile of a launch over beams b0 .. b0 + n - 1 (all), of
+        kind "forward", "adjoint" or "positions" (pb_tile_split)."""
+        n = self.n_beams if n is None else n
+        split = self._splits.get((kind, b0, n))
+        if split is None:
+            args = (ctypes.byref(self.grid), self._beam_ptr(b0), n, ptr(self._spot_boxes[b0:b0 + n]))
+            f, a = ctypes.c_int(1), ctypes.c_int(1)
+            if kind == "positions":
+                check(_lib.lib.pb_tile_split_positions(*args, ctypes.byref(f)),
+                      "pb_tile_split_positions")
+                self._splits[("positions", b0, n)] = f.value
+            else:
+                check(_lib.lib.pb_tile_split(*args, ctypes.byref(f), ctypes.byref(a)),
+                      "pb_tile_split")
+                self._splits[("forward", b0, n)] = f.value
+                self._splits[("adjoint", b0, n)] = a.value
+            split = self._splits[(kind, b0, n)]
+        return split
 
     def __del__(self):
         if not getattr(self, "_owns_textures", True):
@@ -437,7 +443,8 @@ class DevicePlan:
             return dose, bd
         check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), beams, self.n_beams, ptr(self.wet),
                                      ptr(self.layers), ptr(self.spot_geo), ptr(mu), float(scale),
-                                     ptr(dose), ptr(order), self._split, _stream(self.device)),
+                                     ptr(dose), ptr(order), self._tile_split("forward"),
+                                     _stream(self.device)),
               "pb_dose_split")
         return dose
 
@@ -478,7 +485,7 @@ class DevicePlan:
         check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), self._beam_ptr(b), 1,
                                      ptr(self.wet[b]), ptr(self.layers), ptr(self.spot_geo),
                                      ptr(mu), float(scale), ptr(dose), ptr(order),
-                                     self._beam_split[b], _stream(self.device)),
+                                     self._tile_split("forward", b, 1), _stream(self.device)),
               "pb_dose_split")
         return dose
 
@@ -513,7 +520,7 @@ class DevicePlan:
             check(_lib.lib.pb_dose_adjoint_split(
                 ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
                 ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(w), float(scale),
-                ptr(grad), ptr(order), self._split_adjoint, _stream(self.device)),
+                ptr(grad), ptr(order), self._tile_split("adjoint"), _stream(self.device)),
                 "pb_dose_adjoint_split")
         else:
             check(_lib.lib.pb_dose_adjoint_variant(
@@ -537,7 +544,8 @@ class DevicePlan:
         check(_lib.lib.pb_dose_adjoint_positions_split(
             ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
             ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu), ptr(w), float(scale),
-            ptr(g), ptr(gx), ptr(gy), ptr(order), self._split_positions, _stream(self.device)),
+            ptr(g), ptr(gx), ptr(gy), ptr(order), self._tile_split("positions"),
+            _stream(self.device)),
             "pb_dose_adjoint_positions_split")
         return g[: self.n_spots], gx[: self.n_spots], gy[: self.n_spots]
 
