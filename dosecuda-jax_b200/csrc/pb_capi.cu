@@ -408,19 +408,17 @@ PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
     PbStatus s = check_tile_split(grid, beams, n_beams, spot_boxes);
     if (s != PB_OK) return s;
     if (!forward_out || !adjoint_out) return set_error(PB_ERR_INVALID, "NULL argument");
-    int positions;
-    tile_split(*grid, beams, n_beams, spot_boxes, forward_out, adjoint_out, &positions);
+    tile_split(*grid, beams, n_beams, spot_boxes, forward_out, adjoint_out);
     return PB_OK;
 }
 
-PbStatus pb_tile_split_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
-                                 const float *spot_boxes, int *positions_out)
+PbStatus pb_tile_split_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                             const float *spot_boxes, int positions, int *limits_out)
 {
     PbStatus s = check_tile_split(grid, beams, n_beams, spot_boxes);
     if (s != PB_OK) return s;
-    if (!positions_out) return set_error(PB_ERR_INVALID, "NULL argument");
-    int forward, adjoint;
-    tile_split(*grid, beams, n_beams, spot_boxes, &forward, &adjoint, positions_out);
+    if (!limits_out) return set_error(PB_ERR_INVALID, "NULL argument");
+    tile_split_field(*grid, beams, n_beams, spot_boxes, positions != 0, limits_out, limits_out + 1);
     return PB_OK;
 }
 
@@ -463,6 +461,30 @@ PbStatus pb_dose_adjoint_split(const PbGrid *grid, const PbBeam *beams, int n_be
     return launch_adjoint(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev,
                           dobj_dose_dev, scale, grad_dev, static_cast<cudaStream_t>(stream), -1,
                           order_dev, split);
+}
+
+static PbStatus check_limits(const PbGrid &g, const int *limits, const int *count_dev)
+{
+    if (!limits || !count_dev) return set_error(PB_ERR_INVALID, "NULL argument");
+    if (limits[0] < 0 || limits[1] < limits[0])
+        return set_error(PB_ERR_INVALID, "limits must be ascending from 0");
+    return limits[1] > 0 ? check_split(g, 4) : PB_OK;
+}
+
+PbStatus pb_dose_adjoint_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                               const float *wet_dev, const PbLayer *layers_dev,
+                               const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
+                               float *grad_dev, const int *order_dev, const int *limits,
+                               int *count_dev, void *stream)
+{
+    PbStatus s = check_beams(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev);
+    if (s == PB_OK) s = check_limits(*grid, limits, count_dev);
+    if (s != PB_OK) return s;
+    if (!dobj_dose_dev || !grad_dev) return set_error(PB_ERR_INVALID, "NULL argument");
+    const FieldSplit field{limits[0], limits[1], count_dev};
+    return launch_adjoint(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev,
+                          dobj_dose_dev, scale, grad_dev, static_cast<cudaStream_t>(stream), -1,
+                          order_dev, 1, &field);
 }
 
 PbStatus pb_dose_adjoint(const PbGrid *grid, const PbBeam *beams, int n_beams,
@@ -517,6 +539,21 @@ PbStatus pb_count_pairs(const PbGrid *grid, const PbBeam *beams, int n_beams,
                               static_cast<cudaStream_t>(stream));
 }
 
+static PbStatus check_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                const float *wet_dev, const PbLayer *layers_dev,
+                                const float *spot_geo_dev, const float *mu_dev,
+                                const float *dobj_dose_dev, const float *grad_x_dev,
+                                const float *grad_y_dev)
+{
+    PbStatus s = check_beams(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev);
+    if (s != PB_OK) return s;
+    if (!dobj_dose_dev || !grad_x_dev || !grad_y_dev)
+        return set_error(PB_ERR_INVALID, "NULL argument");
+    for (int b = 0; b < n_beams; ++b)
+        if (beams[b].n_layers && !mu_dev) return set_error(PB_ERR_INVALID, "mu is NULL");
+    return PB_OK;
+}
+
 PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                                          const float *wet_dev, const PbLayer *layers_dev,
                                          const float *spot_geo_dev, const float *mu_dev,
@@ -524,17 +561,33 @@ PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams
                                          float *grad_dev, float *grad_x_dev, float *grad_y_dev,
                                          const int *order_dev, int split, void *stream)
 {
-    PbStatus s = check_beams(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev);
+    PbStatus s = check_positions(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev, mu_dev,
+                                 dobj_dose_dev, grad_x_dev, grad_y_dev);
     if (s == PB_OK) s = check_split(*grid, split);
     if (s != PB_OK) return s;
-    if (!dobj_dose_dev || !grad_x_dev || !grad_y_dev)
-        return set_error(PB_ERR_INVALID, "NULL argument");
-    for (int b = 0; b < n_beams; ++b)
-        if (beams[b].n_layers && !mu_dev) return set_error(PB_ERR_INVALID, "mu is NULL");
     return launch_adjoint_positions(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev,
                                     mu_dev, dobj_dose_dev, scale, grad_dev, grad_x_dev,
                                     grad_y_dev, static_cast<cudaStream_t>(stream), order_dev,
                                     split);
+}
+
+PbStatus pb_dose_adjoint_positions_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                         const float *wet_dev, const PbLayer *layers_dev,
+                                         const float *spot_geo_dev, const float *mu_dev,
+                                         const float *dobj_dose_dev, float scale,
+                                         float *grad_dev, float *grad_x_dev, float *grad_y_dev,
+                                         const int *order_dev, const int *limits, int *count_dev,
+                                         void *stream)
+{
+    PbStatus s = check_positions(grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev, mu_dev,
+                                 dobj_dose_dev, grad_x_dev, grad_y_dev);
+    if (s == PB_OK) s = check_limits(*grid, limits, count_dev);
+    if (s != PB_OK) return s;
+    const FieldSplit field{limits[0], limits[1], count_dev};
+    return launch_adjoint_positions(*grid, beams, n_beams, wet_dev, layers_dev, spot_geo_dev,
+                                    mu_dev, dobj_dose_dev, scale, grad_dev, grad_x_dev,
+                                    grad_y_dev, static_cast<cudaStream_t>(stream), order_dev, 1,
+                                    &field);
 }
 
 PbStatus pb_dose_adjoint_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
@@ -826,8 +879,8 @@ PbStatus pb_proton_spot_host(int gpu_id, double vsadx, double vsady, const float
             box[2] = std::min(box[2], spots[i].y);
             box[3] = std::max(box[3], spots[i].y);
         }
-        int split = 1, split_adj = 1, split_pos = 1;
-        tile_split(g, &B, 1, box, &split, &split_adj, &split_pos);
+        int split = 1, split_adj = 1;
+        tile_split(g, &B, 1, box, &split, &split_adj);
         // the tiles in the order of their estimated work (pb_tile_order)
         PB_TRY(launch_tile_order(g, &B, 1, static_cast<const float *>(D.buf[kBufWet].p),
                                  static_cast<const PbLayer *>(D.buf[kBufLayers].p),

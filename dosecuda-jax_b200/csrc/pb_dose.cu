@@ -1096,6 +1096,7 @@ struct LineShared {
         float2 lut_at[kLine][NT];    // or IDD and sigma per voxel, from rows not staged
     };
     int lut_bad;                     // the layer whose staged row is not uniform
+    int2 share;                      // adjoint: the block's rank and the tile's blocks
     // adjoint: per-slot gradient partials (weight; with positions also x, y)
     float gsum[POS ? 3 : 1][DOSE ? 1 : NT * KCULL + 8];
     float w[kLine][NT];              // the beam's 10*WET per voxel (INF: not valid)
@@ -1305,7 +1306,10 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
     const int64_t vbase = i0 + (int64_t)A.g.nx * (j + (int64_t)A.g.ny * k);
     const int64_t V = (int64_t)A.g.nx * A.g.ny * A.g.nz;
     unsigned long long n_ex2 = 0, n_eval = 0;
-    if (t == 0) sh.lut_bad = 0;   // before the first barrier
+    if (t == 0) {   // before the first barrier
+        sh.lut_bad = 0;
+        if constexpr (ADJ) sh.share = make_int2(rank, ranks);   // not in registers
+    }
 
     if constexpr (MODE == kModeDose) {
 #pragma unroll
@@ -1444,8 +1448,8 @@ __device__ __forceinline__ void line_tile(const PlanArgs &A, int tx, int ty, int
                                             : 0.0f;
                 }
             }
-            for (int l1 = 0; l1 < nsel; l1 += ranks, ++round) {
-              const int li = l1 + rank;
+            for (int l1 = 0; l1 < nsel; l1 += ADJ ? sh.share.y : ranks, ++round) {
+              const int li = l1 + (ADJ ? sh.share.x : rank);
               bool live = li < nsel;
               const int layer_id = (b << 20) + l0 + li + 1;   // not 0
               const LineLayer &Y = sh.layer[live ? li : 0];
@@ -2068,18 +2072,51 @@ k_dose_count_line(const __grid_constant__ PlanArgs A, const float *__restrict__ 
                                                               count, wfield);
 }
 
+// Tiles in which scale * the field is not zero anywhere: those that a gradient
+// launch does not skip.  One block per tile; *count is 0 before.
+__global__ void __launch_bounds__(kLineTY * kLineTZ)
+k_field_tiles(PbGrid g, const float *__restrict__ wfield, float scale, int *__restrict__ count)
+{
+    const int nx8 = (g.nx + kLine - 1) / kLine, nty = (g.ny + kLineTY - 1) / kLineTY;
+    const int i0 = (int)(blockIdx.x % nx8) * kLine;
+    const int j = (int)(blockIdx.x / nx8 % nty) * kLineTY + (int)(threadIdx.x % kLineTY);
+    const int k = (int)(blockIdx.x / nx8 / nty) * kLineTZ + (int)(threadIdx.x / kLineTY);
+    bool any = false;
+    if (j < g.ny && k < g.nz) {
+        const float *p = wfield + i0 + (int64_t)g.nx * (j + (int64_t)g.ny * k);
+#pragma unroll
+        for (int q = 0; q < kLine; ++q) any |= i0 + q < g.nx && __ldg(p + q) * scale != 0.0f;
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) atomicAdd(count, 1);
+}
+
+// Blocks that share a tile in this launch of `split` blocks a tile: all of them,
+// or as many as the count of the field's tiles asks for.  The same in every block.
+// The blocks without work are the launch's last: every fourth block with work would
+// leave the most expensive tiles to every fourth SM (1,122 tiles, 4 beams of 3
+// layers, one block a tile of four launched: 534 us against 427).
+__device__ __forceinline__ unsigned field_ranks(const FieldSplit &f, unsigned split)
+{
+    if (f.count == nullptr) return split;
+    const int n = __ldg(f.count);
+    return min(split, n <= f.four ? 4u : n <= f.two ? 2u : 1u);
+}
+
 __global__ void __launch_bounds__(kLineTY * kLineTZ, line_min_blocks<kLineTY * kLineTZ>())
 k_adjoint_line(const __grid_constant__ PlanArgs A, const float *__restrict__ wet,
                const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
-               const float *__restrict__ wfield, float *__restrict__ grad, int split)
+               const float *__restrict__ wfield, float *__restrict__ grad, unsigned split,
+               const FieldSplit field)
 {
     __shared__ LineShared<kLineTY * kLineTZ, kLineCull, false, false> sh;
-    // each tile by `split` blocks, block r taking every split-th kept layer
+    // each tile by `ranks` blocks, block r taking every ranks-th kept layer
+    const unsigned ranks = field_ranks(field, split);
     int tx, ty, tz;
-    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / split, tx, ty, tz)) return;
+    if (blockIdx.x >= gridDim.x / split * ranks) return;
+    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / ranks, tx, ty, tz)) return;
     line_tile<kLineTY, kLineTZ, kLineCull, false, kModeAdjoint>(
         A, tx, ty, tz, wet, layers, geo, nullptr, nullptr, nullptr, sh, nullptr, wfield, grad,
-        (int)(blockIdx.x % split), split);
+        (int)(blockIdx.x % ranks), (int)ranks);
 }
 
 // Spot-weight and spot-position gradients (grad may be NULL).  A line's eight
@@ -2094,14 +2131,16 @@ k_adjoint_pos_line(const __grid_constant__ PlanArgs A, const float *__restrict__
                    const PbLayer *__restrict__ layers, const float4 *__restrict__ geo,
                    const float *__restrict__ mu, const float *__restrict__ wfield,
                    float *__restrict__ grad, float *__restrict__ grad_x,
-                   float *__restrict__ grad_y, int split)
+                   float *__restrict__ grad_y, unsigned split, const FieldSplit field)
 {
     __shared__ LineShared<kLineTY * kLineTZ, kLineCull, false, false, 1, true> sh;
+    const unsigned ranks = field_ranks(field, split);
     int tx, ty, tz;
-    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / split, tx, ty, tz)) return;
+    if (blockIdx.x >= gridDim.x / split * ranks) return;
+    if (!line_tile_coords<kLineTY, kLineTZ>(A, blockIdx.x / ranks, tx, ty, tz)) return;
     line_tile<kLineTY, kLineTZ, kLineCull, false, kModeAdjointPos>(
         A, tx, ty, tz, wet, layers, geo, mu, nullptr, nullptr, sh, nullptr, wfield, grad,
-        (int)(blockIdx.x % split), split, grad_x, grad_y);
+        (int)(blockIdx.x % ranks), (int)ranks, grad_x, grad_y);
 }
 
 // ------------------------------------------------------------ tile order
@@ -2716,10 +2755,32 @@ int dose_variant_threads(int variant)
     return (variant >= 0 && variant < kNumDoseVariants) ? kDoseVariants[variant].nt : 128;
 }
 
+// How a gradient launch under `limits` goes: `split` blocks a tile, and with a
+// count those of them that it asks for.  Without one where every count gives the
+// same.
+static FieldSplit field_split(const PbGrid &g, const FieldSplit &limits, int &split)
+{
+    const long long tiles = line_tiles(g, kLineTY, kLineTZ);
+    split = limits.four > 0 ? 4 : limits.two > 0 ? 2 : 1;
+    if (split == 1 || limits.four >= tiles || (split == 2 && limits.two >= tiles))
+        return FieldSplit{};
+    return limits;
+}
+
+static PbStatus launch_field_tiles(const PbGrid &g, const float *w, float scale, int *count,
+                                   bool zero, cudaStream_t st)
+{
+    const PbStatus s = zero ? check_cuda(cudaMemsetAsync(count, 0, sizeof(int), st),
+                                         "cudaMemsetAsync(count)") : PB_OK;
+    if (s != PB_OK) return s;
+    k_field_tiles<<<line_tiles(g, kLineTY, kLineTZ), kLineTY * kLineTZ, 0, st>>>(g, w, scale, count);
+    return check_launch("k_field_tiles");
+}
+
 PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
                         const float *wet, const PbLayer *layers, const float *geo,
                         const float *w, float scale, float *grad, cudaStream_t st,
-                        int variant, const int *order, int split)
+                        int variant, const int *order, int split, const FieldSplit *limits)
 {
     PlanArgs A;
     fill_args(A, g, beams, n_beams, scale);
@@ -2729,14 +2790,19 @@ PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
         const int e = beams[b].spot_start + beams[b].n_spots;
         if (e > total_spots) total_spots = e;
     }
-    PbStatus s = check_cuda(cudaMemsetAsync(grad, 0, sizeof(float) * (size_t)total_spots, st),
-                            "cudaMemsetAsync(grad)");
+    const bool line = variant_line(variant);
+    const FieldSplit field = line && limits ? field_split(g, *limits, split) : FieldSplit{};
+    // the count after the last gradient is zeroed with them
+    const bool with = field.count && (void *)field.count == (void *)(grad + total_spots);
+    PbStatus s = check_cuda(cudaMemsetAsync(grad, 0, sizeof(float) * ((size_t)total_spots + with),
+                                            st), "cudaMemsetAsync(grad)");
+    if (s == PB_OK && field.count) s = launch_field_tiles(g, w, scale, field.count, !with, st);
     if (s != PB_OK) return s;
     const int64_t tiles = (int64_t)A.tiles_x * A.tiles_y * A.tiles_z;
     const float4 *g4 = reinterpret_cast<const float4 *>(geo);
-    if (variant_line(variant)) {
+    if (line) {
         k_adjoint_line<<<line_tiles(g, kLineTY, kLineTZ) * split, kLineTY * kLineTZ, 0, st>>>(
-            A, wet, layers, g4, w, grad, split);
+            A, wet, layers, g4, w, grad, split, field);
         return check_launch("k_adjoint_line");
     }
     k_adjoint_tile<<<(unsigned)tiles, 128, 0, st>>>(A, wet, layers, g4, w, grad);
@@ -2747,7 +2813,7 @@ PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_be
                                   const float *wet, const PbLayer *layers, const float *geo,
                                   const float *mu, const float *w, float scale, float *grad,
                                   float *grad_x, float *grad_y, cudaStream_t st, const int *order,
-                                  int split)
+                                  int split, const FieldSplit *limits)
 {
     PlanArgs A;
     fill_args(A, g, beams, n_beams, scale);
@@ -2757,13 +2823,22 @@ PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_be
         const int e = beams[b].spot_start + beams[b].n_spots;
         if (e > total_spots) total_spots = e;
     }
+    const FieldSplit field = limits ? field_split(g, *limits, split) : FieldSplit{};
     const size_t bytes = sizeof(float) * (size_t)total_spots;
     PbStatus s = PB_OK;
-    for (float *o : {grad, grad_x, grad_y})
-        if (o && s == PB_OK) s = check_cuda(cudaMemsetAsync(o, 0, bytes, st), "cudaMemsetAsync");
+    bool with = false;   // the count after an array's last entry is zeroed with it
+    for (float *o : {grad, grad_x, grad_y}) {
+        if (!o || s != PB_OK) continue;
+        const bool here = field.count && (void *)field.count == (void *)(o + total_spots);
+        s = check_cuda(cudaMemsetAsync(o, 0, bytes + (here ? sizeof(int) : 0), st),
+                       "cudaMemsetAsync");
+        with |= here;
+    }
+    if (s == PB_OK && field.count) s = launch_field_tiles(g, w, scale, field.count, !with, st);
     if (s != PB_OK) return s;
     k_adjoint_pos_line<<<line_tiles(g, kLineTY, kLineTZ) * split, kLineTY * kLineTZ, 0, st>>>(
-        A, wet, layers, reinterpret_cast<const float4 *>(geo), mu, w, grad, grad_x, grad_y, split);
+        A, wet, layers, reinterpret_cast<const float4 *>(geo), mu, w, grad, grad_x, grad_y, split,
+        field);
     return check_launch("k_adjoint_pos_line");
 }
 
@@ -2818,33 +2893,34 @@ void tile_order_tile(int *voxels)
 // chain the layers of a mean tile one after the other (each reached beam's
 // ceil(layers / split) of them), work what the SMs do in all: a block's set-up
 // per reached tile and beam and per tile not reached, `split` times, and the
-// layers once.  The constants are fitted to the measured ratios of the three
-// splits on random plans (1 to 4 beams of 1 to 33 layers of 9 to 1,153 spots, 75
-// to 3,465 tiles reached; the forward 640 plans, the gradients 220); a larger
-// split is taken where its estimate is the smaller one (forward: by 4 %).
-// Microseconds at 1, 2 and 4 blocks, and what is taken:
-//   tiles beams layers spots   forward           weight gradient    taken
-//    120    2     1     185   50,  58,  76         74,  78,  89     1 / 1
-//    498    4     1      69   52,  68, 117         51,  54,  58     1 / 1
-//    495    2     2      37   53,  68, 102         54,  46,  55     1 / 2
-//    342    1     3      49   34,  32,  43         41,  35,  34     1 / 2
-//     90    1     3      89   42,  35,  33         59,  43,  37     4 / 4
-//    291    2     6      97   160, 107, 109        222, 127,  97    2 / 4
-//    797    3     6     101   388, 274, 337        402, 256, 180    2 / 2
-//    120    1    12      97   150,  97,  64        218, 122,  78    4 / 4
-//    728    2    16     973   4055, 2474, 2345     5017, 2783, 1876 4 / 4
-//   1326    4    16      61   673, 702, 849        757, 684, 770    1 / 1
-// Against one block per tile over those plans: forward 1.27 times as fast (the
-// best of the three would be 1.30), slower by more than 5 % in 4 of 640 (17 % at
-// most); weight gradient of a field without zeros 1.41 (1.42) and 1 of 220 (9 %);
-// position gradients 1.20 (1.21) and 2 (13 %).  A gradient skips the tiles where
-// its field is zero, which the host does not know; the fit is to fields without
-// zeros, as the gradient of an objective over the whole grid is, and a field
-// around the target alone still gains 1.65 of 1.81 and is never slower.  The tiles
-// reached are estimated from the beams' spot boxes: a tile counts for a beam when
-// its centre lies within 60 mm (where the widest halo falls below 2^-24) and half
-// a tile's width of the beam's box of spot axes.
+// layers once.  A gradient skips the tiles where its field is zero, and there are
+// as many of the others as k_field_tiles counts: the host gives the counts up to
+// which 4 and 2 blocks are taken (tile_split_field).  Where every count gives the
+// same, nothing is counted.  The constants are fitted to the measured ratios of
+// the three splits on random plans (1 to 4 beams of 1 to 33 layers of 9 to 1,153
+// spots, 75 to 3,465 tiles reached; the forward 640 plans, the gradients 240, each
+// with a field around the target and with one without zeros); a larger split is
+// taken where its estimate is smaller by 4 %.  Microseconds at 1, 2 and 4 blocks:
+//   tiles beams layers spots   forward           weight gradient (around the target)
+//    120    2     1     185   50,  58,  76         74,  78,  89
+//    498    4     1      69   52,  68, 117         51,  54,  58
+//    495    2     2      37   53,  68, 102         54,  46,  55
+//    342    1     3      49   34,  32,  43         41,  35,  34
+//     90    1     3      89   42,  35,  33         59,  43,  37
+//    291    2     6      97   160, 107, 109        222, 127,  97
+//    797    3     6     101   388, 274, 337        402, 256, 180
+//    120    1    12      97   150,  97,  64        218, 122,  78
+//    728    2    16     973   4055, 2474, 2345     5017, 2783, 1876
+//   1326    4    16      61   673, 702, 849        757, 684, 770
+// Against one block per tile over those plans (in brackets the best of the three),
+// and the plans slower by more than 5 %: forward 1.27 (1.30), 4 of 640, 17 % at
+// most; weight gradient 1.82 (1.82), 0 of 240, of a field without zeros 1.41
+// (1.42), 0; position gradients 1.59 (1.60), 3 (15 %), without zeros 1.17 (1.19), 1
+// (7 %).  The tiles reached are estimated from the beams' spot boxes: a tile
+// counts for a beam when its centre lies within 60 mm (where the widest halo falls
+// below 2^-24) and half a tile's width of the beam's box of spot axes.
 constexpr int kSplitMaxTiles = 4096;   // larger grids are not looked at
+constexpr float kSplitGain = 1.04f;    // what a larger split's estimate must win by
 
 struct SplitCost {
     float base;          // launch, ramp and the chain's set-up
@@ -2852,11 +2928,10 @@ struct SplitCost {
     float block;         // set-up per block of a reached tile and beam
     float idle;          // set-up per block of a tile not reached, and beam
     float share;         // of an SM that a layer's time occupies
-    float gain;          // estimates a larger split must win by
 };
-constexpr SplitCost kSplitForward = {15.0f, 6.0f, 0.06f, 2.9f, 0.7f, 0.15f, 1.04f};
-constexpr SplitCost kSplitAdjoint = {24.0f, 4.3f, 0.14f, 1.9f, 0.45f, 0.115f, 1.0f};
-constexpr SplitCost kSplitPositions = {28.0f, 6.4f, 0.14f, 3.1f, 1.3f, 0.265f, 1.0f};
+constexpr SplitCost kSplitForward = {15.0f, 6.0f, 0.06f, 2.9f, 0.7f, 0.15f};
+constexpr SplitCost kSplitAdjoint = {30.0f, 4.7f, 0.13f, 2.1f, 0.23f, 0.13f};
+constexpr SplitCost kSplitPositions = {29.0f, 6.5f, 0.135f, 3.5f, 1.0f, 0.32f};
 
 // Tiles that a plan's beams reach.
 struct SplitTiles {
@@ -2864,35 +2939,39 @@ struct SplitTiles {
     int reached[PB_MAX_BEAMS];         // by each beam
 };
 
-static int split_of(const SplitTiles &T, const PbBeam *beams, int n_beams, const SplitCost &C)
+// Blocks per tile where `live` tiles are not skipped (reached ones first).
+static int split_of(const SplitTiles &T, const PbBeam *beams, int n_beams, const SplitCost &C,
+                    int live)
 {
+    if (T.active == 0) return 1;
+    const float busy = (float)std::min(live, T.active), rest = (float)std::max(live - T.active, 0);
     auto time = [&](int split) {
-        float chain = 0.0f, work = (float)(T.tiles - T.active) * n_beams * split * C.idle;
+        float chain = 0.0f, work = rest * n_beams * split * C.idle;
         for (int b = 0; b < n_beams; ++b) {
             if (T.reached[b] == 0) continue;
             const int L = beams[b].n_layers;
             const float one = C.layer + C.spot * (float)beams[b].n_spots / (float)L;
-            chain += (float)T.reached[b] / (float)T.active * (float)((L + split - 1) / split) * one;
-            work += (float)T.reached[b] * (split * C.block + L * one * C.share);
+            const float part = (float)T.reached[b] / (float)T.active;   // of the reached tiles
+            chain += part * (float)((L + split - 1) / split) * one;
+            work += busy * part * (split * C.block + L * one * C.share);
         }
         return C.base + sqrtf(chain * chain + work / 148.0f * (work / 148.0f));
     };
-    if (T.active == 0) return 1;
     const float t1 = time(1), t2 = time(2), t4 = time(4);
-    const bool two = C.gain * t2 < t1;
-    return C.gain * t4 < (two ? t2 : t1) ? 4 : two ? 2 : 1;
+    const bool two = kSplitGain * t2 < t1;
+    return kSplitGain * t4 < (two ? t2 : t1) ? 4 : two ? 2 : 1;
 }
 
-void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
-                int *forward, int *adjoint, int *positions)
+// False for a grid that is not looked at.
+static bool split_tiles(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                        SplitTiles &T)
 {
-    *forward = *adjoint = *positions = 1;
     const int ntx = (g.nx + kLine - 1) / kLine, nty = (g.ny + kLineTY - 1) / kLineTY;
     const int ntz = (g.nz + kLineTZ - 1) / kLineTZ;
-    if ((long long)ntx * nty * ntz > kSplitMaxTiles) return;
+    if ((long long)ntx * nty * ntz > kSplitMaxTiles) return false;
     const float reach = 60.0f + 0.5f * kLine * g.spacing;
     unsigned char any[kSplitMaxTiles] = {};
-    SplitTiles T = {};
+    T = SplitTiles{};
     T.tiles = ntx * nty * ntz;
     for (int b = 0; b < n_beams; ++b) {
         const PbBeamGeom &B = beams[b].geom;
@@ -2927,9 +3006,38 @@ void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *
             }
     }
     for (int t = 0; t < T.tiles; ++t) T.active += any[t];
-    *forward = split_of(T, beams, n_beams, kSplitForward);
-    *adjoint = split_of(T, beams, n_beams, kSplitAdjoint);
-    *positions = split_of(T, beams, n_beams, kSplitPositions);
+    return true;
+}
+
+void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                int *forward, int *adjoint)
+{
+    SplitTiles T;
+    *forward = *adjoint = 1;
+    if (!split_tiles(g, beams, n_beams, spot_boxes, T)) return;
+    *forward = split_of(T, beams, n_beams, kSplitForward, T.tiles);
+    *adjoint = split_of(T, beams, n_beams, kSplitAdjoint, T.tiles);
+}
+
+void tile_split_field(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                      bool positions, int *four, int *two)
+{
+    SplitTiles T;
+    *four = *two = 0;
+    if (!split_tiles(g, beams, n_beams, spot_boxes, T)) return;
+    const SplitCost &C = positions ? kSplitPositions : kSplitAdjoint;
+    // the largest count of tiles at which at least `want` blocks are taken
+    auto up_to = [&](int want) {
+        int lo = 0, hi = T.tiles;
+        while (lo < hi) {
+            const int m = (lo + hi + 1) / 2;
+            if (split_of(T, beams, n_beams, C, m) >= want) lo = m;
+            else hi = m - 1;
+        }
+        return lo;
+    };
+    *four = up_to(4);
+    *two = std::max(*four, up_to(2));
 }
 
 size_t tile_order_work_size(const PbGrid &g)

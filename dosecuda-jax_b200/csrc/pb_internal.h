@@ -99,18 +99,29 @@ PbStatus launch_dose_batch(const void *plans_dev, int n_plans, long long n_items
                            unsigned long long *counter, int variant, int blocks,
                            cudaStream_t st);
 
+// A gradient launch whose blocks per tile go by the tiles in which the field is not
+// zero: up to `four` of them 4 blocks a tile, up to `two` 2, counted on the device.
+struct FieldSplit {
+    int four, two;
+    int *count;
+};
+
 PbStatus launch_adjoint(const PbGrid &g, const PbBeam *beams, int n_beams,
                         const float *wet, const PbLayer *layers,
                         const float *geo, const float *w, float scale,
                         float *grad, cudaStream_t st, int variant = -1,
-                        const int *order = nullptr, int split = 1);
+                        const int *order = nullptr, int split = 1,
+                        const FieldSplit *limits = nullptr);
 long long tile_order_count(const PbGrid &g);
 void tile_order_tile(int *voxels);
 size_t tile_order_work_size(const PbGrid &g);
-// Blocks per tile for the forward, the weight gradient and the position
-// gradients (pb_tile_split, pb_tile_split_positions).
+// Blocks per tile for the forward and for the weight gradient of a field without
+// zeros (pb_tile_split).
 void tile_split(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
-                int *forward, int *adjoint, int *positions);
+                int *forward, int *adjoint);
+// The gradients' limits (pb_tile_split_field).
+void tile_split_field(const PbGrid &g, const PbBeam *beams, int n_beams, const float *spot_boxes,
+                      bool positions, int *four, int *two);
 PbStatus launch_tile_order(const PbGrid &g, const PbBeam *beams, int n_beams, const float *wet,
                            const PbLayer *layers, void *work, int *order, cudaStream_t st);
 
@@ -123,7 +134,8 @@ PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_be
                                   const float *wet, const PbLayer *layers, const float *geo,
                                   const float *mu, const float *w, float scale, float *grad,
                                   float *grad_x, float *grad_y, cudaStream_t st,
-                                  const int *order = nullptr, int split = 1);
+                                  const int *order = nullptr, int split = 1,
+                                  const FieldSplit *limits = nullptr);
 PbStatus launch_layer_bounds(const PbBeam *beams, int n_beams, PbLayer *layers,
                             const float *geo, cudaStream_t st);
 PbStatus launch_count_evaluated(const PbGrid &g, const PbBeam *beams, int n_beams,

@@ -153,7 +153,12 @@ _SIGS = {
                                      ctypes.c_float, _VP, _VP, _VP]),
     "pb_tile_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, ctypes.POINTER(_I),
                            ctypes.POINTER(_I)]),
-    "pb_tile_split_positions": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, ctypes.POINTER(_I)]),
+    "pb_tile_split_field": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _I, ctypes.POINTER(_I)]),
+    "pb_dose_adjoint_field": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _F, _VP,
+                                   _VP, ctypes.POINTER(_I), _VP, _VP]),
+    "pb_dose_adjoint_positions_field": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP,
+                                             _VP, _F, _VP, _VP, _VP, _VP, ctypes.POINTER(_I), _VP,
+                                             _VP]),
     "pb_dose_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _F, _VP, _VP, _I,
                            _VP]),
     "pb_dose_adjoint_split": (_I, [ctypes.POINTER(PbGrid), _VP, _I, _VP, _VP, _VP, _VP, _F, _VP,

@@ -280,25 +280,29 @@ class DevicePlan:
                                            _stream(self.device)), "pb_layer_bounds")
         self.spots_loaded = True
 
-    def _tile_split(self, kind: str, b0: int = 0, n: Optional[int] = None) -> int:
-        """Blocks per tile of a launch over beams b0 .. b0 + n - 1 (all), of
-        kind "forward", "adjoint" or "positions" (pb_tile_split)."""
+    def _forward_split(self, b0: int = 0, n: Optional[int] = None) -> int:
+        """Blocks per tile of a forward launch over beams b0 .. b0 + n - 1
+        (all; pb_tile_split)."""
         n = self.n_beams if n is None else n
-        split = self._splits.get((kind, b0, n))
+        split = self._splits.get((b0, n))
         if split is None:
-            args = (ctypes.byref(self.grid), self._beam_ptr(b0), n, ptr(self._spot_boxes[b0:b0 + n]))
             f, a = ctypes.c_int(1), ctypes.c_int(1)
-            if kind == "positions":
-                check(_lib.lib.pb_tile_split_positions(*args, ctypes.byref(f)),
-                      "pb_tile_split_positions")
-                self._splits[("positions", b0, n)] = f.value
-            else:
-                check(_lib.lib.pb_tile_split(*args, ctypes.byref(f), ctypes.byref(a)),
-                      "pb_tile_split")
-                self._splits[("forward", b0, n)] = f.value
-                self._splits[("adjoint", b0, n)] = a.value
-            split = self._splits[(kind, b0, n)]
+            check(_lib.lib.pb_tile_split(ctypes.byref(self.grid), self._beam_ptr(b0), n,
+                                         ptr(self._spot_boxes[b0:b0 + n]), ctypes.byref(f),
+                                         ctypes.byref(a)), "pb_tile_split")
+            split = self._splits[(b0, n)] = f.value
         return split
+
+    def _field_limits(self, positions: bool):
+        """The gradients' limits for their field's tiles (pb_tile_split_field)."""
+        key = "positions" if positions else "weights"
+        limits = self._splits.get(key)
+        if limits is None:
+            limits = self._splits[key] = (ctypes.c_int * 2)()
+            check(_lib.lib.pb_tile_split_field(ctypes.byref(self.grid), self._beam_ptr(0),
+                                               self.n_beams, ptr(self._spot_boxes),
+                                               int(positions), limits), "pb_tile_split_field")
+        return limits
 
     def __del__(self):
         if not getattr(self, "_owns_textures", True):
@@ -443,7 +447,7 @@ class DevicePlan:
             return dose, bd
         check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), beams, self.n_beams, ptr(self.wet),
                                      ptr(self.layers), ptr(self.spot_geo), ptr(mu), float(scale),
-                                     ptr(dose), ptr(order), self._tile_split("forward"),
+                                     ptr(dose), ptr(order), self._forward_split(),
                                      _stream(self.device)),
               "pb_dose_split")
         return dose
@@ -485,7 +489,7 @@ class DevicePlan:
         check(_lib.lib.pb_dose_split(ctypes.byref(self.grid), self._beam_ptr(b), 1,
                                      ptr(self.wet[b]), ptr(self.layers), ptr(self.spot_geo),
                                      ptr(mu), float(scale), ptr(dose), ptr(order),
-                                     self._tile_split("forward", b, 1), _stream(self.device)),
+                                     self._forward_split(b, 1), _stream(self.device)),
               "pb_dose_split")
         return dose
 
@@ -513,15 +517,17 @@ class DevicePlan:
         if dobj_ddose.dtype != torch.float32 or dobj_ddose.numel() != self.n_vox:
             raise ValueError("dobj_ddose must be float32 with one entry per voxel")
         w = dobj_ddose.contiguous()
-        grad = out if out is not None else torch.empty(max(self.n_spots, 1), dtype=torch.float32,
-                                                       device=self.device)
+        # one entry more: the launch's count of the field's tiles
+        work = torch.empty(self.n_spots + 1 if out is None else 1, dtype=torch.float32,
+                           device=self.device)
+        grad = work if out is None else out
         if variant is None:
             order = self.tile_order()
-            check(_lib.lib.pb_dose_adjoint_split(
+            check(_lib.lib.pb_dose_adjoint_field(
                 ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
                 ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(w), float(scale),
-                ptr(grad), ptr(order), self._tile_split("adjoint"), _stream(self.device)),
-                "pb_dose_adjoint_split")
+                ptr(grad), ptr(order), self._field_limits(False), ptr(work[-1:]),
+                _stream(self.device)), "pb_dose_adjoint_field")
         else:
             check(_lib.lib.pb_dose_adjoint_variant(
                 ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
@@ -538,15 +544,15 @@ class DevicePlan:
         if dobj_ddose.dtype != torch.float32 or dobj_ddose.numel() != self.n_vox:
             raise ValueError("dobj_ddose must be float32 with one entry per voxel")
         mu = self.mu_sorted if mu_sorted is None else mu_sorted
-        n = max(self.n_spots, 1)
+        # one entry more: the launch's count of the field's tiles
+        n = self.n_spots + 1
         g, gx, gy = (torch.empty(n, dtype=torch.float32, device=self.device) for _ in range(3))
         mu, w, order = mu.contiguous(), dobj_ddose.contiguous(), self.tile_order()
-        check(_lib.lib.pb_dose_adjoint_positions_split(
+        check(_lib.lib.pb_dose_adjoint_positions_field(
             ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
             ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu), ptr(w), float(scale),
-            ptr(g), ptr(gx), ptr(gy), ptr(order), self._tile_split("positions"),
-            _stream(self.device)),
-            "pb_dose_adjoint_positions_split")
+            ptr(g), ptr(gx), ptr(gy), ptr(order), self._field_limits(True), ptr(gy[-1:]),
+            _stream(self.device)), "pb_dose_adjoint_positions_field")
         return g[: self.n_spots], gx[: self.n_spots], gy[: self.n_spots]
 
     def count_pairs(self) -> int:

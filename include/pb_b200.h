@@ -257,7 +257,7 @@ PbStatus pb_dose_adjoint_positions(const PbGrid *grid, const PbBeam *beams, int 
                                    const float *dobj_dose_dev, float scale, float *grad_dev,
                                    float *grad_x_dev, float *grad_y_dev, void *stream);
 /* The same in a given tile order (pb_tile_order; NULL: none), each tile shared
- * by `split` blocks (1, 2 or 4: pb_tile_split_positions). */
+ * by `split` blocks (1, 2 or 4). */
 PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                                          const float *wet_dev, const PbLayer *layers_dev,
                                          const float *spot_geo_dev, const float *mu_dev,
@@ -409,12 +409,16 @@ PbStatus pb_dose_adjoint_ordered(const PbGrid *grid, const PbBeam *beams, int n_
  * several blocks a tile shorten the launch.  Host only.  Of `beams` the
  * geometry and the counts are read; spot_boxes: per beam the least and
  * greatest spot x, then y, at the isocentre plane (mm; least > greatest for
- * a beam without spots).  No counterpart in the reference. */
+ * a beam without spots).  adjoint_out is for a field without zeros.  No
+ * counterpart in the reference. */
 PbStatus pb_tile_split(const PbGrid *grid, const PbBeam *beams, int n_beams,
                        const float *spot_boxes, int *forward_out, int *adjoint_out);
-/* The same for pb_dose_adjoint_positions_split. */
-PbStatus pb_tile_split_positions(const PbGrid *grid, const PbBeam *beams, int n_beams,
-                                 const float *spot_boxes, int *positions_out);
+/* The same for the gradients, which skip the tiles where their field is zero:
+ * limits_out[0] the count of other tiles up to which 4 blocks share a tile,
+ * limits_out[1] that of 2 (or 4), for the weight gradient or (positions not 0)
+ * the position gradients.  No counterpart in the reference. */
+PbStatus pb_tile_split_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                             const float *spot_boxes, int positions, int *limits_out);
 /* pb_dose_ordered (without per-beam doses) and pb_dose_adjoint_ordered with
  * each tile of the default shape shared by `split` blocks (1, 2 or 4).  The
  * dose is the same bits for every split, the gradient the same to float
@@ -427,6 +431,24 @@ PbStatus pb_dose_adjoint_split(const PbGrid *grid, const PbBeam *beams, int n_be
                                const float *wet_dev, const PbLayer *layers_dev,
                                const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
                                float *grad_dev, const int *order_dev, int split, void *stream);
+
+/* pb_dose_adjoint_split and pb_dose_adjoint_positions_split with the blocks per
+ * tile from the field: its tiles that are not zero everywhere are counted into
+ * count_dev (one device int, overwritten; zeroed with the gradients where it
+ * follows the last entry of one of them) and held against limits
+ * (pb_tile_split_field, or ascending from 0), all in the stream. */
+PbStatus pb_dose_adjoint_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                               const float *wet_dev, const PbLayer *layers_dev,
+                               const float *spot_geo_dev, const float *dobj_dose_dev, float scale,
+                               float *grad_dev, const int *order_dev, const int *limits,
+                               int *count_dev, void *stream);
+PbStatus pb_dose_adjoint_positions_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
+                                         const float *wet_dev, const PbLayer *layers_dev,
+                                         const float *spot_geo_dev, const float *mu_dev,
+                                         const float *dobj_dose_dev, float scale,
+                                         float *grad_dev, float *grad_x_dev, float *grad_y_dev,
+                                         const int *order_dev, const int *limits, int *count_dev,
+                                         void *stream);
 
 /* Adjoint of pb_dose: grad_dev[s] = scale * sum_v dobj_dose_dev[v] * K(v,s)
  * for every spot s, where K(v,s) is the dose per unit weight of spot s at

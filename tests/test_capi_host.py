@@ -312,3 +312,55 @@ def test_tile_split_counts_work_and_grid():
     assert _split((40, 40, 40), 3.0, [(0.0, 12, 100, 20.0), (90.0, 1, 100, 20.0)]) == (4, 4)
     # the reached tiles alone: a small target in a wide grid
     assert _split((160, 160, 24), 3.0, [(0.0, 12, 100, 20.0)])[1] == 4
+
+
+def _limits(shape, spacing, beams, positions):
+    from dosecuda_b200 import _lib
+    nx, ny, nz = shape
+    g = _lib.PbGrid(nx, ny, nz, spacing)
+    B = (_lib.PbBeam * len(beams))()
+    box = np.empty((len(beams), 4), np.float32)
+    for b, (angle, layers, spots, half) in enumerate(beams):
+        B[b].geom = _lib.beam_setup(angle, 0.0, 1340.0, 1930.0,
+                                    0.5 * spacing * np.array(shape, np.float32), [0, 0, 0])
+        B[b].n_layers, B[b].n_spots = layers, layers * spots
+        box[b] = (-half, half, -half, half)
+    lim = (ctypes.c_int * 2)(-1, -1)
+    _lib.check(_lib.lib.pb_tile_split_field(ctypes.byref(g), ctypes.cast(B, ctypes.c_void_p),
+                                            len(beams), _lib.ptr(box), positions, lim))
+    return tuple(lim)
+
+
+@pytest.mark.parametrize("n,layers,spots", [(40, 1, 50), (40, 2, 50), (40, 12, 100),
+                                            (120, 3, 50), (120, 12, 100), (180, 6, 100)])
+@pytest.mark.parametrize("positions", [0, 1])
+def test_tile_split_field_limits(n, layers, spots, positions):
+    """Ascending counts within the grid's tiles; nothing to share in one layer,
+    no third block for two; at the grid's tiles, pb_tile_split's answer for a
+    field without zeros."""
+    shape, beams = (n, n, n), [(90.0 * b, layers, spots, 20.0) for b in range(2)]
+    tiles = -(-n // 8) * -(-n // 16) * -(-n // 8)
+    four, two = _limits(shape, 3.0, beams, positions)
+    assert 0 <= four <= two <= tiles
+    if layers == 1:
+        assert two == 0
+    if layers == 2:
+        assert four == 0
+    if n == 40 and layers == 12:
+        assert four == tiles
+    if not positions:
+        assert _split(shape, 3.0, beams)[1] == (4 if four == tiles else 2 if two == tiles else 1)
+
+
+def test_adjoint_field_refuses_bad_limits():
+    from dosecuda_b200 import _lib
+    g = _lib.PbGrid(16, 16, 16, 2.0)
+    B = (_lib.PbBeam * 1)()
+    one = ctypes.c_void_p(16)
+    for limits in ((-1, 3), (4, 3)):
+        lim = (ctypes.c_int * 2)(*limits)
+        assert _lib.lib.pb_dose_adjoint_field(
+            ctypes.byref(g), ctypes.cast(B, ctypes.c_void_p), 1, one, one, one, one, 1.0, one,
+            None, lim, one, None) == _lib.PB_ERR_INVALID
+    assert _lib.lib.pb_tile_split_field(ctypes.byref(g), ctypes.cast(B, ctypes.c_void_p), 1, None,
+                                        0, (ctypes.c_int * 2)()) == _lib.PB_ERR_INVALID

@@ -229,3 +229,76 @@ def test_splits_with_uneven_layers_over_many_beams(n_beams, n_layers):
     for split in (2, 4):
         for rep in range(60):
             assert torch.equal(_dose(dp, split, order=rep % 2 == 0), one), (split, rep)
+
+
+def _field(dp, kind):
+    w = torch.randn(dp.n_vox, device=DEV, generator=torch.Generator(DEV).manual_seed(3)) + 0.5
+    at = torch.arange(dp.n_vox, device=DEV)
+    if kind == "none":
+        w.zero_()
+    elif kind == "one":
+        w[at != dp.n_vox // 2] = 0.0
+    elif kind == "part":
+        w[at % (dp.grid.nx * dp.grid.ny) < dp.grid.nx * dp.grid.ny // 2] = 0.0
+    return w
+
+
+def _live_tiles(dp, w):
+    g = dp.grid
+    v = torch.nn.functional.pad((w.reshape(1, 1, g.nz, g.ny, g.nx) != 0).float(),
+                                (0, -g.nx % 8, 0, -g.ny % 16, 0, -g.nz % 8))
+    return int(torch.nn.functional.max_pool3d(v, (8, 16, 8)).sum())
+
+
+@pytest.mark.parametrize("kind", ["none", "one", "part", "full"])
+@pytest.mark.parametrize("n_layers,per_layer,shape", [(5, 20, (21, 37, 43)), (3, 300, (8, 16, 8)),
+                                                      (7, 2, (9, 17, 9))])
+def test_gradients_by_the_fields_tiles(kind, n_layers, per_layer, shape):
+    """Every number of blocks that the count of the field's tiles can ask for, at
+    the limits themselves, against one block per tile (atomic sums in another
+    order: 1e-5 of the largest), with the count after a gradient's last entry
+    and in a buffer of its own."""
+    from dosecuda_b200 import _lib
+    dp = _plan(n_layers, per_layer, shape=shape)
+    w = _field(dp, kind)
+    live = _live_tiles(dp, w)
+    n = dp.n_spots
+    stream = ctypes.c_void_p(torch.cuda.current_stream(DEV).cuda_stream)
+    head = (ctypes.byref(dp.grid), ctypes.cast(dp.beams, ctypes.c_void_p), dp.n_beams,
+            _lib.ptr(dp.wet), _lib.ptr(dp.layers), _lib.ptr(dp.spot_geo))
+    order = _lib.ptr(dp.tile_order())
+    ref = [torch.empty(n, device=DEV) for _ in range(3)]
+    _lib.check(_lib.lib.pb_dose_adjoint_positions_split(
+        *head, _lib.ptr(dp.mu_sorted), _lib.ptr(w), 1.0, *(_lib.ptr(r) for r in ref), order, 1,
+        stream))
+    assert (kind == "none") == (float(ref[0].abs().max()) == 0.0)
+
+    def close(got):
+        for a, b in zip(got, ref):
+            assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+    many = 1 << 20
+    for limits in ((0, 0), (live, live), (live - 1, live), (live - 1, live - 1), (0, live),
+                   (0, live - 1), (0, many), (live - 1, many), (many, many)):
+        if limits[0] < 0 or limits[1] < limits[0]:
+            continue
+        lim = (ctypes.c_int * 2)(*limits)
+        for apart in (False, True):
+            out = [torch.full((n + 1,), float("nan"), device=DEV) for _ in range(3)]
+            count = torch.full((1,), -5, dtype=torch.int32, device=DEV)
+            at = count if apart else out[0][n:]
+            _lib.check(_lib.lib.pb_dose_adjoint_field(
+                *head, _lib.ptr(w), 1.0, _lib.ptr(out[0]), order, lim, _lib.ptr(at), stream))
+            close([out[0][:n]])
+            if apart and limits[0] == live - 1 and limits[1] == live and live > 1:
+                assert int(count) == live
+            at = count if apart else out[2][n:]
+            for o in out:
+                o.fill_(float("nan"))
+            _lib.check(_lib.lib.pb_dose_adjoint_positions_field(
+                *head, _lib.ptr(dp.mu_sorted), _lib.ptr(w), 1.0, *(_lib.ptr(o) for o in out),
+                order, lim, _lib.ptr(at), stream))
+            close([o[:n] for o in out])
+    close([dp.adjoint(w)])
+    close([dp.adjoint(w, out=torch.empty(n, device=DEV))])
+    close(dp.adjoint_positions(w))
