@@ -62,12 +62,12 @@ METRIC = "IMPT dose+grad ms/plan (20k spots, 256²×160) vs plain fwd; spot-voxe
 UNIT = "spot-voxel evals/s"
 L2_FLUSH_BYTES = 256 << 20
 L2_NOTE = "flushed (256 MiB write) between timed iterations"
-# dram__bytes_read.sum + dram__bytes_write.sum per launch, from ncu captures of
+# dram__bytes_read.sum + dram__bytes_write.sum per launch, from an ncu capture of
 # this workload (seed 3, texture WET); the command and the figures are in
 # profiles/pencil_beam_kernels_heterogeneous_256x256x160_4beams.md.  Reported only
-# for that workload.  The depths' kernels have changed since that capture, so
-# they have no figure here.
-NCU_TRAFFIC = {"k_dose_line": 208_208_128, "k_adjoint_line": 129_612_544}
+# for that workload ("wet": the cell passes, k_raytrace and k_smooth).
+NCU_TRAFFIC = {"k_dose_line": 204_658_432, "k_adjoint_line": 126_976_000,
+               "wet": 825_198_592}
 NCU_TRAFFIC_WORKLOAD = {"seed": 3, "wet_mode": "texture"}
 
 

@@ -1031,6 +1031,14 @@ __device__ __forceinline__ void dose_tile(const PlanArgs &A, int tile,
 //   - the LUT intervals of the tile's depths are staged in shared memory with
 //     their differences, one interval per thread, so a voxel takes two shared
 //     loads instead of six global ones and a search.
+// A row that does not run from 0 in steps of a power of two (the machines' own do)
+// is not staged: its voxels read and search it in global memory.  Forward of the
+// 4-beam plan below: own rows 5.52 ms, steps of 0.999 mm 5.83, uneven steps 9.4;
+// with every row read so and five blocks an SM these took 5.65, 5.66 and 8.2.
+// Small plans gain with such rows too (120^3 cube: 231 -> 151 us, uneven 333 ->
+// 236).  Staged with a search in shared memory they take 6.0 and 7.3 ms, but that
+// code costs the machines' rows 1.2 % (step of forward and adjoint), in every form
+// measured; unrolling the voxels' loop by 2, 4 or 8 gains nothing.
 // Measured, launches with no spot in reach: 413 -> 281 us on the 4-beam
 // 256x256x160 plan; forward 5.65 -> 5.55 ms, adjoint 6.26 -> 6.05 ms; on the
 // 120^3 cube with 1,210 spots the forward 228 -> 193 us (141 us with each tile
@@ -2824,16 +2832,29 @@ PbStatus launch_adjoint_positions(const PbGrid &g, const PbBeam *beams, int n_be
         if (e > total_spots) total_spots = e;
     }
     const FieldSplit field = limits ? field_split(g, *limits, split) : FieldSplit{};
-    const size_t bytes = sizeof(float) * (size_t)total_spots;
+    // arrays one after the other, and the count after the last entry of one, are
+    // zeroed together
     PbStatus s = PB_OK;
-    bool with = false;   // the count after an array's last entry is zeroed with it
+    bool with = false;
+    float *from = nullptr, *to = nullptr;
+    auto flush = [&]() {
+        if (from != to)
+            s = check_cuda(cudaMemsetAsync(from, 0, sizeof(float) * (size_t)(to - from), st),
+                           "cudaMemsetAsync");
+    };
     for (float *o : {grad, grad_x, grad_y}) {
         if (!o || s != PB_OK) continue;
-        const bool here = field.count && (void *)field.count == (void *)(o + total_spots);
-        s = check_cuda(cudaMemsetAsync(o, 0, bytes + (here ? sizeof(int) : 0), st),
-                       "cudaMemsetAsync");
-        with |= here;
+        if (o != to) {
+            flush();
+            from = to = o;
+        }
+        to += total_spots;
     }
+    if (s == PB_OK && field.count && (void *)field.count == (void *)to) {
+        with = true;
+        ++to;
+    }
+    if (s == PB_OK) flush();
     if (s == PB_OK && field.count) s = launch_field_tiles(g, w, scale, field.count, !with, st);
     if (s != PB_OK) return s;
     k_adjoint_pos_line<<<line_tiles(g, kLineTY, kLineTZ) * split, kLineTY * kLineTZ, 0, st>>>(

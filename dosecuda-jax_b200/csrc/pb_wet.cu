@@ -265,7 +265,8 @@ __device__ __forceinline__ float sparse_run(const float2 *__restrict__ rec, int 
 // texture-unit ray trace of a CT with image noise is the unit itself: a linear
 // 3-D FP32 fetch of a warp takes 16 cycles of the L1's data stage (ncu: 93 %
 // of its peak, issue slots 34 %), whatever it hits.  A sample from the records
-// is two 16-byte loads, about 9 cycles of that stage.
+// is two 16-byte loads of 4.9 cycles each (exact ray trace of a 165x150x121 CT:
+// 332 million wavefronts for 68 million loads of a warp).
 //
 // FILTER: the texture unit's own filter, from its fixed-point rule: the
 // coordinate to the nearest 1/256 (halves up), the cell and three 8-bit
@@ -462,7 +463,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                         // not added, so the sum is the loop's, bit for bit
                         // (measured 7.50 -> 7.24 ms for the whole WET)
                         float sv[kBurst - 1];
-    #pragma unroll
+#pragma unroll
                         for (int q = 1; q < kBurst; ++q) {
                             const float tq = __fadd_rn(t, (float)q);
                             const float x = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(ux, tq, px), ix), 0.5f);
@@ -470,7 +471,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                             const float z = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(uz, tq, pz), iz), 0.5f);
                             sv[q - 1] = fmaxf(tex3D<float>(tex, x, y, z), 0.0f);
                         }
-    #pragma unroll
+#pragma unroll
                         for (int q = 1; q < kBurst; ++q)
                             part = __fadd_rn(t, (float)q) < e ? __fadd_rn(part, sv[q - 1]) : part;
                         t = fmaxf(__fadd_rn(t, 1.0f), e);
@@ -529,7 +530,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                     constexpr int kCells = decltype(by_cells)::value;
                     float sv[kBurst];
                     if (!first) at2(t, X, Y, Z);
-    #pragma unroll
+#pragma unroll
                     for (int m = 0; m < kBurst; m += 2) {
                         if (m > 0) at2(t + (float)m, X, Y, Z);
                         if (m < kCells) {
@@ -542,7 +543,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                         }
                     }
                     float part = fmaxf(sv[0], 0.0f);
-    #pragma unroll
+#pragma unroll
                     for (int m = 1; m < kBurst; ++m) part = __fadd_rn(part, fmaxf(sv[m], 0.0f));
                     acc += (double)part;
                     t += (float)kBurst;
@@ -554,7 +555,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                     burst(None{}, true);
                 } else {
                     burst(Some{}, true);
-    #pragma unroll 1
+#pragma unroll 1
                     for (int q = 1; q < min(TEX ? 2 * thick : thick, kMaxBursts) && t + (float)kBurst <= nsf; ++q)
                         burst(Some{}, false);
                 }

@@ -544,16 +544,17 @@ class DevicePlan:
         if dobj_ddose.dtype != torch.float32 or dobj_ddose.numel() != self.n_vox:
             raise ValueError("dobj_ddose must be float32 with one entry per voxel")
         mu = self.mu_sorted if mu_sorted is None else mu_sorted
-        # one entry more: the launch's count of the field's tiles
-        n = self.n_spots + 1
-        g, gx, gy = (torch.empty(n, dtype=torch.float32, device=self.device) for _ in range(3))
+        # in one buffer, zeroed at once, with the launch's count of the field's tiles
+        n = self.n_spots
+        work = torch.empty(3 * n + 1, dtype=torch.float32, device=self.device)
+        g, gx, gy = work, work[n:], work[2 * n:]
         mu, w, order = mu.contiguous(), dobj_ddose.contiguous(), self.tile_order()
         check(_lib.lib.pb_dose_adjoint_positions_field(
             ctypes.byref(self.grid), ctypes.cast(self.beams, ctypes.c_void_p), self.n_beams,
             ptr(self.wet), ptr(self.layers), ptr(self.spot_geo), ptr(mu), ptr(w), float(scale),
-            ptr(g), ptr(gx), ptr(gy), ptr(order), self._field_limits(True), ptr(gy[-1:]),
+            ptr(g), ptr(gx), ptr(gy), ptr(order), self._field_limits(True), ptr(work[-1:]),
             _stream(self.device)), "pb_dose_adjoint_positions_field")
-        return g[: self.n_spots], gx[: self.n_spots], gy[: self.n_spots]
+        return g[:n], gx[:n], gy[:n]
 
     def count_pairs(self) -> int:
         """Dense spot-voxel pair count E of the reference kernel."""

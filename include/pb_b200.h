@@ -269,8 +269,9 @@ PbStatus pb_dose_adjoint_positions_split(const PbGrid *grid, const PbBeam *beams
 
 /* What the forward pencil-beam sum issues, counted with its own culling
  * decisions (no dose is computed): count_dev[0] = SFU exp2 operations,
- * count_dev[1] = spot-voxel evaluations (each surviving spot against the
- * 512 voxel slots of a tile).  With a time, count_dev[0] gives the SFU
+ * count_dev[1] = spot-voxel evaluations (each surviving spot against every
+ * voxel slot of its tile).  The spots of weight 0 that fill the forward's last
+ * groups are not counted.  With a time, count_dev[0] gives the SFU
  * roofline fraction of pb_dose.  No counterpart in the reference. */
 PbStatus pb_count_evaluated(const PbGrid *grid, const PbBeam *beams, int n_beams,
                             const float *wet_dev, const PbLayer *layers_dev,
@@ -435,7 +436,7 @@ PbStatus pb_dose_adjoint_split(const PbGrid *grid, const PbBeam *beams, int n_be
 /* pb_dose_adjoint_split and pb_dose_adjoint_positions_split with the blocks per
  * tile from the field: its tiles that are not zero everywhere are counted into
  * count_dev (one device int, overwritten; zeroed with the gradients where it
- * follows the last entry of one of them) and held against limits
+ * follows the last entry of the last of them) and held against limits
  * (pb_tile_split_field, or ascending from 0), all in the stream. */
 PbStatus pb_dose_adjoint_field(const PbGrid *grid, const PbBeam *beams, int n_beams,
                                const float *wet_dev, const PbLayer *layers_dev,
