@@ -382,13 +382,11 @@ def run_mine(args, world, rank, local):
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "call": "IMPTDoseGrid.computeIMPTPlan" if args.mode == "forward"
                 else "engine.HostGradientStep"},
-        # per forward step: HU->RLSP, [texture mode: four cell-record passes and
-        # the ray trace of the other kind of volume, which ends at once],
-        # ray trace, smoothing, the tile order (cost, histogram, scan,
-        # scatter), pencil-beam sum; the grad step adds the objective (two)
-        # and the adjoint
-        "gpu_launches": ((13 if args.wet_mode == "texture" else 8) +
-                         (3 if args.mode == "grad" else 0)) * args.steps,
+        # per forward step: HU->RLSP, four cell-record passes, ray trace,
+        # smoothing, the tile order (cost, histogram, scan, scatter),
+        # pencil-beam sum; the grad step adds the objective (two) and the
+        # adjoint
+        "gpu_launches": (12 + (3 if args.mode == "grad" else 0)) * args.steps,
         "clocks": clk.summary(),
     }
     same = args.seed == NCU_TRAFFIC_WORKLOAD["seed"] and \
@@ -541,7 +539,7 @@ def run_batch(args, world, rank, local):
                    "variant": autotune.variants()[variant], "blocks_per_sm": bps,
                    "plans_per_s": bp.n_plans * world / (ms * 1e-3),
                    "l2": L2_NOTE},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": 3 * args.steps,    # ray trace, smoothing, pencil-beam sum
         "clocks": clk.summary(),
     }
     if rank == 0:

@@ -271,7 +271,7 @@ PbStatus pb_texture_sample(PbTexture tex, const PbGrid *grid, const float *at_de
     if (s != PB_OK) return s;
     if (!tex || !at_dev || !unit_dev || !cells_dev || pairs < 0 || pairs > INT_MAX)
         return set_error(PB_ERR_INVALID, "NULL argument or count");
-    if (!texture_matches(tex, *grid) || !texture_samples(tex) || !texture_cells(tex).quad ||
+    if (!texture_matches(tex, *grid) || !texture_samples(tex) || !texture_cells(tex).cell ||
         std::max(grid->nx, std::max(grid->ny, grid->nz)) > 8191)
         return set_error(PB_ERR_INVALID, "not a texture with cell records of this grid");
     return launch_texture_sample(texture_object(tex), *grid, at_dev, pairs, unit_dev, cells_dev,

@@ -34,11 +34,11 @@ PbStatus launch_rlsp(const float *hu, int64_t n, const double *xh,
 PbStatus check_wet_args(const float *rlsp_dev, uint64_t tex, const PbGrid *grid,
                         const PbBeamGeom *beams, int n_beams, const float *wet_dev);
 
-// Cell records of an RLSP volume (pb_wet.cu); null: none.
+// Cell records of an RLSP volume (pb_wet.cu); null: none.  A texture's handle has
+// cell, one without quad and dist.
 struct RayCells {
     const float4 *quad;
     const unsigned char *dist;
-    const unsigned int *odd;
     const float2 *cell;
 };
 

@@ -170,26 +170,27 @@ __device__ __forceinline__ float ray_sample(const float *__restrict__ rho,
 // samples).  A ray that exceeds the grid-diagonal step cap stops and raises
 // PB_ERR_RAY_CAP in *status.  The leading samples that are certainly inside
 // the grid (safe_steps) go without the in-grid test: with cell records, as
-// runs through flat cells (flat_run) and bursts of kBurst samples elsewhere;
-// without them, 8 fetches at a time.  Either way several fetches are in
-// flight per thread.
-//
-// Volumes are of two kinds (cells_dense, counted when the records are made).
-// Where rays meet flat cells (phantoms, a CT whose air is clean) a ray is a chain
-// of record loads with fetches between, and the kernel lives on occupancy.
-// Where hardly any cell is flat (image noise everywhere) nearly every sample
-// is fetched, and the texture unit's rate bounds it: there some samples come
-// from the records (cell_sample2).  Each kind has its own kernel, and the
-// launch of the other one ends at once: the host does not wait for the count.
-// 200x188x160 CT with noise, 3 beams: 8.70 -> 6.4 ms; exact weights, 165x150x121,
-// 2 beams: 3.41 -> 1.8 ms.
+// runs through flat cells and bursts of samples elsewhere; without them, 8
+// fetches at a time.  Either way several fetches are in flight per thread.
 //
 // TEX = true samples RLSP through a border-0, linearly filtered 3-D texture
 // and forms the ray direction with rnorm3df, as the reference does
 // (CudaClasses.cuh:41-52, TextureClasses.cu:14-41), so the samples are the
-// reference's own.  TEX = false interpolates with exact FP32 trilinear
-// weights from global memory and forms the direction in FP64, the CPU
-// oracle's arithmetic.
+// reference's own.  A ray is a chain of record loads (cell_run) with fetches
+// between, and the kernel lives on occupancy; where hardly any cell is flat (image
+// noise everywhere) the texture unit's rate bounds it.  There half of the samples
+// can come from records of the texels with the unit's filter in FP32
+// (200x188x160 CT with noise, 3 beams: 8.7 -> 6.5 ms), but they are off by a
+// rounding in a third of the samples, and that decided a radius of the smoothing
+// otherwise in some voxel of every tenth noisy volume.  The unit's own sum, exact
+// and rounded once, makes it the slower one: 11.9 ms in FP64, 10.5 as two FP32
+// sums of split texels.  So every sample is the unit's.
+//
+// TEX = false takes exact FP32 trilinear weights, from the records (flat_run,
+// cell_sample2) or from global memory, and forms the direction in FP64, the CPU
+// oracle's arithmetic.  Each sample by its eight texels from the volume is bound
+// by the loads: 165x150x121, 2 beams, noise: 3.41 -> 1.8 ms by the records.
+
 // floor(a) for -2^22 <= a < 2^22 on the FP32 adder: adding 1.5 * 2^23 with
 // rounding toward -infinity leaves floor(a) in the low mantissa bits.
 __device__ __forceinline__ int floor_small(float a)
@@ -206,17 +207,16 @@ __device__ __forceinline__ float floor_small_f(float a)
 // multiple of 4.
 __host__ __device__ __forceinline__ int cell_row(int nx) { return (nx + 1 + 3) & ~3; }
 
-// A handle's records as the ray trace reads them (build_cells below).  Cell
+// A handle's records as the ray trace reads them (texture_create below).  Cell
 // (ci, cj, ck) holds the 2x2x2 texels with base (ci-1, cj-1, ck-1), with zeros
 // outside the grid.
-//   quad  (nx+1) x (ny+2) x (nz+1), x fastest: the texels (ci-1, r-1, ck-1),
+//   cell  with a texture: value and distance (of quad and dist below) of the cell,
+//         (nx+1) x (ny+1) x (nz+1), x fastest
+//   quad  without: (nx+1) x (ny+2) x (nz+1), x fastest: the texels (ci-1, r-1, ck-1),
 //         (ci-1, r-1, ck), (ci, r-1, ck-1), (ci, r-1, ck); a cell's eight are
 //         its entries at rows cj and cj + 1
-//   dist  distance in cells to the nearest cell that is not flat, rows of
+//   dist  without: distance in cells to the nearest cell that is not flat, rows of
 //         cell_row(nx) bytes
-//   odd   not 0 where a texel is infinite or not a number: the unit leaves out
-//         texels of weight 0, which the products below do not, so it samples
-//         such a volume itself; nor where an axis has kFixLimit voxels or more
 struct CellIndex {
     int cx, cxy;      // quad strides per row and per plane
     unsigned off;     // takes the biased integers of the float adders out
@@ -249,8 +249,8 @@ __device__ __forceinline__ float flat_run(const RayCells &C, const CellIndex &I,
     return floor_small_f(__fmul_rd((float)(d - 3), inv_dmax)) + 1.0f;
 }
 
-// The same from the sparse volumes' records: value and distance in one load.
-__device__ __forceinline__ float sparse_run(const float2 *__restrict__ rec, int cx, int cy,
+// The same from a texture's records: value and distance in one load.
+__device__ __forceinline__ float cell_run(const float2 *__restrict__ rec, int cx, int cy,
                                             float x, float y, float z, float inv_dmax, float &v)
 {
     const int i = floor_small(__fsub_rn(x, 0.5f)) + 1, j = floor_small(__fsub_rn(y, 0.5f)) + 1,
@@ -261,14 +261,11 @@ __device__ __forceinline__ float sparse_run(const float2 *__restrict__ rec, int 
     return floor_small_f(__fmul_rd(r.y - 3.0f, inv_dmax)) + 1.0f;
 }
 
-// Samples from the cell records instead of the texture unit.  What bounds a
-// texture-unit ray trace of a CT with image noise is the unit itself: a linear
-// 3-D FP32 fetch of a warp takes 16 cycles of the L1's data stage (ncu: 93 %
-// of its peak, issue slots 34 %), whatever it hits.  A sample from the records
-// is two 16-byte loads of 4.9 cycles each (exact ray trace of a 165x150x121 CT:
-// 332 million wavefronts for 68 million loads of a warp).
+// Samples from the quads: two 16-byte loads of 4.9 cycles each of the L1's data
+// stage (exact ray trace of a 165x150x121 CT: 332 million wavefronts for 68 million
+// loads of a warp); a linear 3-D FP32 fetch of a warp takes the unit 16.
 //
-// FILTER: the texture unit's own filter, from its fixed-point rule: the
+// FILTER (pb_texture_sample): the texture unit's own filter, from its fixed-point rule: the
 // coordinate to the nearest 1/256 (halves up), the cell and three 8-bit
 // fractions from it, and the eight weights as whole 256ths that sum to 256,
 // divided among z, then x, then y, each product to the nearest whole (halves
@@ -276,8 +273,8 @@ __device__ __forceinline__ float sparse_run(const float2 *__restrict__ rec, int 
 // The sum is the FP32 products', so a sample agrees with the unit's to FP32
 // rounding.  Otherwise exact trilinear weights, in trilinear's operation order
 // bit for bit.
-constexpr float kFixMagic = 6291328.5f;    // 1.5 * 2^22 - 128 + 0.5: an ulp of 0.5
-constexpr int kFixLimit = 8192;            // coordinates that hold in it are below this
+constexpr float kFixMagic = 6291328.5f;    // 1.5 * 2^22 - 128 + 0.5: an ulp of 0.5,
+                                           // coordinates below 8192
 constexpr float kIntMagic = 12582912.0f;   // 1.5 * 2^23: an ulp of 1
 
 template <bool FILTER>
@@ -361,52 +358,30 @@ __device__ __forceinline__ float2 cell_sample2(const RayCells &C, const CellInde
     return make_float2(out[0], out[1]);
 }
 
-// Whether the volume's cells are dense: 85 % of them or more not flat.  Below
-// that the rays that leave through flat cells make the sparse kernel the faster
-// one: us of the ray trace, sparse / dense, of volumes whose body has noise and
-// whose air has none, by the share of cells that are not flat:
-//     96 x  87 x  68, 2 beams   0.27 164 / 239, 0.56 241 / 317, 0.83  280 /  252
-//    130 x 121 x  85, 2 beams   0.25 378 / 587, 0.54 652 / 874, 0.83  891 / 1021,
-//                               0.87 898 / 823
-//    220 x 211 x 130, 3 beams   0.52 5360 / 5505, 0.81 7353 / 6804, 0.91 7796 / 6420
-// and of phantoms without noise, where surfaces alone are not flat (0.09 to 0.28):
-// the dense kernel takes 1.6 to 2.3 times as long.
-__device__ __forceinline__ bool cells_dense(const unsigned int *odd, const PbGrid &g)
-{
-    const long long n = (long long)(g.nx + 1) * (g.ny + 1) * (g.nz + 1);
-    return 20ll * (long long)__ldg(odd + 1) >= 17ll * n;
-}
-
 // Samples of a burst, fetched together.
 constexpr int kBurst = 4;
-// Dense volumes: from the kThick-th look at the records without a run, kByCells
-// samples of a burst come from the cell records, the others from the unit, so
-// that the unit's wavefronts and the instructions of the records' filter
-// overlap; and up to kMaxBursts bursts go by until the next look.  200x188x160
-// CT with noise, 3 beams, whole WET: none by the records 9.78 ms, all four
-// 11.7, two 7.62; kThick 2 instead of 3 8.26, at most 4 bursts 7.8.
-constexpr int kThick = 3, kByCells = 2, kMaxBursts = 8;
-// Resident blocks per SM (registers): sparse 12 (40; they cover the latency of
+// Exact weights: after the n-th look at the records without a run, n bursts, at most
+// kMaxBursts, go by until the next.
+constexpr int kMaxBursts = 8;
+// Resident blocks per SM (registers): texture 12 (40; they cover the latency of
 // the dependent record loads: 10 took 6.77 ms against 6.52 on the 256x256x160
-// phantom), dense 7 (72; 5, 6 and 8 took 7.93, 7.82 and 8.08 ms on the CT above
-// against 7.62), exact weights 6 (80).
-constexpr int kSparseBlocks = 12, kDenseBlocks = 7, kExactBlocks = 6;
-// The batch's sparse kernel keeps its item too and spills at 12: two plans of
+// phantom), exact weights 6 (80).
+constexpr int kTextureBlocks = 12, kExactBlocks = 6;
+// The batch's texture kernel keeps its item too and spills at 12: two plans of
 // 48x52x45, 1 beam 56 us at 12 blocks, 50 at 10, 47 at 9, 46 at 8; eight of 64x68x61,
 // 2 beams 220, 210, 210, 210; four of up to 1.6 million voxels, 1 beam 650, 630, 638,
 // 635.
-constexpr int kSparseBatchBlocks = 9;
-// Bricks a block takes in turn where there are many: the launch that finds the
-// volume of the other kind then ends in a few us (0.55 ns a block).  Up to
-// kEachBricks the sparse kernel has a block per brick: us, a loop over bricks
-// against a block each, 50x111x55, 4 beams 187 / 183; 96x87x68, 2 beams, noise in
-// the body 241 / 239; 180x171x110, 3 beams (83,000 bricks) 2587 / 2511;
-// 256x256x160, 4 beams, phantom 3640 / 3729.  (One brick index in a row, divided by
-// the three extents in the kernel, cost 8 % of a small volume's ray trace.)
+constexpr int kTextureBatchBlocks = 9;
+// Up to kEachBricks a block per brick, above them kBricksPerBlock bricks a block in
+// turn: us, a loop over bricks against a block each, 50x111x55, 4 beams 187 / 183;
+// 96x87x68, 2 beams, noise in the body 241 / 239; 180x171x110, 3 beams (83,000
+// bricks) 2587 / 2511; 256x256x160, 4 beams, phantom 3640 / 3729.  (One brick index
+// in a row, divided by the three extents in the kernel, cost 8 % of a small volume's
+// ray trace.)
 constexpr int kBricksPerBlock = 8;
 constexpr int64_t kEachBricks = 148 * 1024;
 
-template <bool TEX, bool DENSE>
+template <bool TEX>
 __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                                                 cudaTextureObject_t tex, const RayCells &rec,
                                                 const PbGrid &g, const PbBeamGeom &B, int i, int j, int k,
@@ -431,7 +406,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
     const int nsafe = safe_steps(g, B, inv_s, px, py, pz, ux, uy, uz, cap);
     double acc = 0.0;
     int n = 0;
-    if (rec.quad) {
+    if (TEX ? rec.cell != nullptr : rec.quad != nullptr) {
         // runs through flat regions, samples elsewhere; the sample counter
         // is kept in FP32 (exact below 2^24).  Both filters on a flat cell
         // give exactly its value.
@@ -439,7 +414,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                            1e-6f;
         const float inv_dmax = __frcp_rd(dmax);
         const float nsf = (float)nsafe;
-        if constexpr (!DENSE) {
+        if constexpr (TEX) {
             const int cx = g.nx + 1, cy = g.ny + 1;
             float t = 0.0f;
             while (t < nsf) {
@@ -447,7 +422,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                 const float y = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(uy, t, py), iy), 0.5f);
                 const float z = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(uz, t, pz), iz), 0.5f);
                 float v;
-                const float run = sparse_run(rec.cell, cx, cy, x, y, z, inv_dmax, v);
+                const float run = cell_run(rec.cell, cx, cy, x, y, z, inv_dmax, v);
                 if (run > 0.0f) {
                     const float m = fminf(run, nsf - t);
                     acc += (double)(m * fmaxf(v, 0.0f));
@@ -482,8 +457,7 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
             n = (int)t;
         } else {
             const int cy = g.ny + 1, drow = cell_row(g.nx);
-            const CellIndex I = cell_index<TEX>(g);
-            const bool by_unit = TEX && __ldg(rec.odd) != 0;
+            const CellIndex I = cell_index<false>(g);
             auto at2 = [&](float t0, float2 &X, float2 &Y, float2 &Z) {
                 const float2 t2 = make_float2(t0, __fadd_rn(t0, 1.0f));
                 auto axis = [&](float u, float p, float o) {
@@ -521,26 +495,20 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                         const float x = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(ux, t, px), ix), 0.5f);
                         const float y = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(uy, t, py), iy), 0.5f);
                         const float z = __fmaf_rn(inv_s, __fadd_rn(__fmaf_rn(uz, t, pz), iz), 0.5f);
-                        part += fmaxf(ray_sample<TEX>(rho, tex, g, x, y, z), 0.0f);
+                        part += fmaxf(ray_sample<false>(rho, tex, g, x, y, z), 0.0f);
                     }
                     acc += (double)part;
                     break;
                 }
-                auto burst = [&](auto by_cells, bool first) {
-                    constexpr int kCells = decltype(by_cells)::value;
+                auto burst = [&](bool first) {
                     float sv[kBurst];
                     if (!first) at2(t, X, Y, Z);
 #pragma unroll
                     for (int m = 0; m < kBurst; m += 2) {
                         if (m > 0) at2(t + (float)m, X, Y, Z);
-                        if (m < kCells) {
-                            const float2 w = cell_sample2<TEX>(rec, I, X, Y, Z);
-                            sv[m] = w.x;
-                            sv[m + 1] = w.y;
-                        } else {
-                            sv[m] = tex3D<float>(tex, X.x, Y.x, Z.x);
-                            sv[m + 1] = tex3D<float>(tex, X.y, Y.y, Z.y);
-                        }
+                        const float2 w = cell_sample2<false>(rec, I, X, Y, Z);
+                        sv[m] = w.x;
+                        sv[m + 1] = w.y;
                     }
                     float part = fmaxf(sv[0], 0.0f);
 #pragma unroll
@@ -548,17 +516,11 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
                     acc += (double)part;
                     t += (float)kBurst;
                 };
-                using None = std::integral_constant<int, 0>;
-                using Some = std::integral_constant<int, TEX ? kByCells : kBurst>;
                 ++thick;
-                if (TEX && (by_unit || thick < kThick)) {
-                    burst(None{}, true);
-                } else {
-                    burst(Some{}, true);
+                burst(true);
 #pragma unroll 1
-                    for (int q = 1; q < min(TEX ? 2 * thick : thick, kMaxBursts) && t + (float)kBurst <= nsf; ++q)
-                        burst(Some{}, false);
-                }
+                for (int q = 1; q < min(thick, kMaxBursts) && t + (float)kBurst <= nsf; ++q)
+                    burst(false);
             }
             acc += (double)(run_m * fmaxf(run_v, 0.0f));
             n = (int)t;
@@ -601,13 +563,12 @@ __device__ __forceinline__ float raytrace_voxel(const float *__restrict__ rho,
 
 // EACH: a block per brick.  Otherwise a block takes the bricks of its row and
 // column in every gridDim.z-th plane (and, past the grid's limit, row).
-template <bool TEX, bool DENSE, bool EACH>
-__global__ void __launch_bounds__(128, !DENSE ? kSparseBlocks : TEX ? kDenseBlocks : kExactBlocks)
+template <bool TEX, bool EACH>
+__global__ void __launch_bounds__(128, TEX ? kTextureBlocks : kExactBlocks)
 k_raytrace(const float *__restrict__ rho, cudaTextureObject_t tex, const RayCells rec,
            PbGrid g, const __grid_constant__ BeamGeomSet bs, int n_beams, int cap,
            float *__restrict__ raw, int *status)
 {
-    if (TEX && rec.quad && cells_dense(rec.odd, g) != DENSE) return;   // the other launch's
     const unsigned by = (g.ny + 3) / 4, bz = (g.nz + 3) / 4;
     const int64_t V = (int64_t)g.nx * g.ny * g.nz;
     const int i = blockIdx.x * 8 + (threadIdx.x & 7);
@@ -617,7 +578,7 @@ k_raytrace(const float *__restrict__ rho, cudaTextureObject_t tex, const RayCell
         const int b = z / bz, k = (z - b * bz) * 4 + (threadIdx.x >> 5);
         if (j >= g.ny || k >= g.nz) return;
         const int64_t v = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
-        raw[b * V + v] = raytrace_voxel<TEX, DENSE>(rho, tex, rec, g, bs.b[b], i, j, k, cap, status);
+        raw[b * V + v] = raytrace_voxel<TEX>(rho, tex, rec, g, bs.b[b], i, j, k, cap, status);
     };
     if constexpr (EACH) {
         brick(blockIdx.y, blockIdx.z);
@@ -672,8 +633,7 @@ __global__ void k_texture_sample(cudaTextureObject_t tex, const RayCells rec, Pb
     }
 }
 
-// A sparse volume's handle holds no quads (its cells lie there), so they are
-// made here from the texture, for the length of the call.
+// A texture's handle holds no quads, so they are made here from the texture, for the length of the call.
 PbStatus launch_texture_sample(cudaTextureObject_t tex, const PbGrid &g, const float *at,
                                int64_t pairs, float *unit, float *cells, cudaStream_t st)
 {
@@ -684,7 +644,7 @@ PbStatus launch_texture_sample(cudaTextureObject_t tex, const PbGrid &g, const f
     if (s != PB_OK) return s;
     k_texture_quads<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(tex, g, n, quad);
     k_texture_sample<<<(unsigned)((pairs + 127) / 128), 128, 0, st>>>(
-        tex, RayCells{quad, nullptr, nullptr, nullptr}, g, at, pairs, unit, cells);
+        tex, RayCells{quad, nullptr, nullptr}, g, at, pairs, unit, cells);
     s = check_launch("k_texture_sample");
     const PbStatus w = check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     cudaFree(quad);
@@ -1205,22 +1165,17 @@ __device__ __forceinline__ bool brick_voxel(const BatchWet &W, long long brick, 
     return i < W.g.nx && j < W.g.ny && k < W.g.nz;
 }
 
-// The items whose volume is the launch's kind, as k_raytrace (exact sampling
-// goes with the dense ones).
-template <bool DENSE>
-__global__ void __launch_bounds__(128, DENSE ? kDenseBlocks : kSparseBatchBlocks)
+__global__ void __launch_bounds__(128, kTextureBatchBlocks)
 k_raytrace_batch(const BatchWet *__restrict__ items, int n_items, int *status)
 {
     const BatchWet &W = items[find_wet_item(items, n_items, blockIdx.x)];
-    const bool dense = !W.tex || (W.rec.quad && cells_dense(W.rec.odd, W.g));
-    if (dense != DENSE) return;
     int i, j, k;
     if (!brick_voxel(W, blockIdx.x, i, j, k)) return;
     float r;
-    if (!DENSE || W.tex)
-        r = raytrace_voxel<true, DENSE>(W.rlsp, W.tex, W.rec, W.g, W.geom, i, j, k, W.cap, status);
+    if (W.tex)
+        r = raytrace_voxel<true>(W.rlsp, W.tex, W.rec, W.g, W.geom, i, j, k, W.cap, status);
     else
-        r = raytrace_voxel<false, true>(W.rlsp, 0, W.rec, W.g, W.geom, i, j, k, W.cap, status);
+        r = raytrace_voxel<false>(W.rlsp, 0, W.rec, W.g, W.geom, i, j, k, W.cap, status);
     W.raw[i + (int64_t)W.g.nx * (j + (int64_t)W.g.ny * k)] = r;
 }
 
@@ -1291,30 +1246,22 @@ PbStatus launch_wet(const float *rlsp, cudaTextureObject_t tex, const RayCells &
     if (bricks > INT32_MAX) return set_error(PB_ERR_INVALID, "grid too large");
     const int64_t limit = 65535;   // of a launch's y and z
     // about `blocks` blocks: all of a plane's bricks, every so many planes
-    auto some = [&](int64_t blocks) {
+    auto many = [&](int64_t blocks) {
         const int64_t z = std::min(std::max<int64_t>((blocks + bx * by - 1) / (bx * by), 1), planes);
         return dim3((unsigned)bx, (unsigned)std::min(by, limit), (unsigned)std::min(z, limit));
     };
-    const int64_t eighth = (bricks + kBricksPerBlock - 1) / kBricksPerBlock;
     const bool each = bricks <= kEachBricks && by <= limit && planes <= limit;
     const dim3 all((unsigned)bx, (unsigned)by, (unsigned)planes);
     const int cap = ray_step_cap(g);
-    if (tex) {
-        if (each)
-            k_raytrace<true, false, true><<<all, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap,
-                                                               raw, status);
-        else
-            k_raytrace<true, false, false><<<some(eighth), 128, 0, st>>>(rlsp, tex, rec, g, bs,
-                                                                         n_beams, cap, raw, status);
-        if (rec.quad)
-            // small volumes: enough blocks that each SM takes several in turn
-            k_raytrace<true, true, false>
-                <<<some(std::max<int64_t>(148 * 8 * kDenseBlocks, eighth)), 128, 0, st>>>(
-                    rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
-    } else {
-        k_raytrace<false, true, false><<<some(each ? bricks : eighth), 128, 0, st>>>(
-            rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
-    }
+    const dim3 some = many((bricks + kBricksPerBlock - 1) / kBricksPerBlock);
+    if (tex && each)
+        k_raytrace<true, true><<<all, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap, raw, status);
+    else if (tex)
+        k_raytrace<true, false><<<some, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams, cap, raw,
+                                                      status);
+    else
+        k_raytrace<false, false><<<each ? all : some, 128, 0, st>>>(rlsp, tex, rec, g, bs, n_beams,
+                                                                    cap, raw, status);
     PbStatus s = check_launch("k_raytrace");
     if (s != PB_OK) return s;
     SmoothStarts at;
@@ -1392,8 +1339,7 @@ PbStatus launch_wet_batch(const void *items_dev, int n_items, long long n_bricks
     if (n_bricks <= 0) return PB_OK;
     if (n_bricks > 0x7fffffffLL) return set_error(PB_ERR_INVALID, "batch too large");
     const BatchWet *I = static_cast<const BatchWet *>(items_dev);
-    k_raytrace_batch<false><<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items, status);
-    k_raytrace_batch<true><<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items, status);
+    k_raytrace_batch<<<(unsigned)n_bricks, 128, 0, st>>>(I, n_items, status);
     PbStatus s = check_launch("k_raytrace_batch");
     if (s != PB_OK) return s;
     if (n_bricks < batch_wet_few())
@@ -1414,7 +1360,7 @@ constexpr int kFlagPad = 16;  // zero bytes before and after each row of flat fl
 // Row length (bytes) of the flat flags: cell_row with kFlagPad bytes on each side.
 __host__ __device__ __forceinline__ int flag_row(int nx) { return cell_row(nx) + 2 * kFlagPad; }
 
-// Pass 0: the quads of the cell records, and the x distance pass's input:
+// Pass 0: the quads (where there are any), and the x distance pass's input:
 // kRunCap where a cell is flat (its eight texels equal), else 0, in rows with
 // kFlagPad zero bytes before and after (flag_row).  A thread takes kFlatRows
 // rows of one (ci, ck) column and keeps each row's four texels for the next
@@ -1424,7 +1370,7 @@ __host__ __device__ __forceinline__ int flag_row(int nx) { return cell_row(nx) +
 constexpr int kFlatRows = 8;
 __global__ void __launch_bounds__(256)
 k_cell_flat(const float *__restrict__ rho, PbGrid g, float4 *__restrict__ quad,
-            unsigned char *__restrict__ flag, unsigned int *__restrict__ odd)
+            unsigned char *__restrict__ flag)
 {
     const int cx = g.nx + 1, cy = g.ny + 1, cz = g.nz + 1;
     const int col = blockIdx.x * 256 + threadIdx.x;   // (ci, ck)
@@ -1445,14 +1391,11 @@ k_cell_flat(const float *__restrict__ rho, PbGrid g, float4 *__restrict__ quad,
         return v;
     };
     float4 a = row(r0);
-    float sum = 0.0f;   // not a number where a texel is infinite or not one
-    int rough = 0;      // cells that are not flat
 #pragma unroll
     for (int m = 0; m < kFlatRows; ++m) {
         const int r = r0 + m;
         if (r > cy) break;                             // rows 0 .. ny + 1
-        if (live) quad[(int64_t)cx * (r + (int64_t)(cy + 1) * ck) + ci] = a;
-        sum = fmaf(a.x, 0.0f, fmaf(a.y, 0.0f, fmaf(a.z, 0.0f, fmaf(a.w, 0.0f, sum))));
+        if (live && quad) quad[(int64_t)cx * (r + (int64_t)(cy + 1) * ck) + ci] = a;
         if (r == cy) break;                            // the last row starts no cell
         const float4 b = row(r + 1);
         const float v = a.x;
@@ -1461,12 +1404,8 @@ k_cell_flat(const float *__restrict__ rho, PbGrid g, float4 *__restrict__ quad,
         if (live)
             flag[((int64_t)cy * ck + r) * flag_row(g.nx) + kFlagPad + ci] =
                 f ? (unsigned char)kRunCap : 0;
-        rough += !f;
         a = b;
     }
-    if (sum != sum || max(g.nx, max(g.ny, g.nz)) >= kFixLimit) odd[0] = 1;
-    rough = __reduce_add_sync(0xffffffffu, rough);
-    if ((threadIdx.x & 31) == 0 && rough) atomicAdd(odd + 1, (unsigned)rough);
 }
 
 // Separable L-infinity distance to the nearest non-flat cell, capped at
@@ -1479,7 +1418,7 @@ k_cell_flat(const float *__restrict__ rho, PbGrid g, float4 *__restrict__ quad,
 // byte-wise ones are a dozen; the passes were bound by them), and in y and z
 // kDistRun words along the axis, which share their taps in registers.  Measured
 // on the 257x257x161 cells of a 256x256x160 volume: x 69 -> 28 us, y 98 -> 26 us,
-// z with a sparse volume's records 108 + 32 -> 65 us.
+// z with a texture's records 108 + 32 -> 65 us.
 __device__ __forceinline__ unsigned int dist_tap(unsigned int best, int k, unsigned int below,
                                                  unsigned int above)
 {
@@ -1526,16 +1465,13 @@ k_cell_dist_x(PbGrid g, const unsigned char *__restrict__ flag, unsigned int *__
 
 constexpr int kDistRun = 8;
 
-// The z pass, the last, also writes the records of a sparse volume.
+// The z pass, the last, also writes a texture's records.
 template <int AXIS>
 __global__ void __launch_bounds__(128)
 k_cell_dist4(PbGrid g, const unsigned int *__restrict__ din, unsigned int *__restrict__ dout,
-             const float *__restrict__ rho = nullptr, const unsigned int *odd_texels = nullptr,
-             float2 *__restrict__ cell = nullptr)
+             const float *__restrict__ rho = nullptr, float2 *__restrict__ cell = nullptr)
 {
     static_assert(AXIS == 1 || AXIS == 2, "y or z");
-    bool records = false;
-    if constexpr (AXIS == 2) records = cell && !cells_dense(odd_texels, g);
     const int cy = g.ny + 1, cz = g.nz + 1, words = cell_row(g.nx) / 4;
     const int len = AXIS == 1 ? cy : cz, other = AXIS == 1 ? cz : cy;
     const int64_t stride = AXIS == 1 ? (int64_t)words : (int64_t)words * cy;
@@ -1567,7 +1503,7 @@ k_cell_dist4(PbGrid g, const unsigned int *__restrict__ din, unsigned int *__res
         }
         const unsigned int best = even | (odd << 8);
         dout[base + stride * p] = best;
-        if (AXIS == 2 && records) {
+        if (AXIS == 2 && cell) {
             // a flat cell's value from its texel inside the grid
             const int cx = g.nx + 1;
             const float *row = rho + (int64_t)g.nx * (min(o, g.ny - 1) +
@@ -1592,14 +1528,12 @@ struct RlspTexture {
     cudaArray_t arr = nullptr;
     cudaTextureObject_t tex = 0;
     // The cell records (RayCells) and the passes' work arrays, in one allocation,
-    // or none of them: no memory.  The quads of a sparse volume with a texture
-    // are overwritten by its cells, which are all that its ray trace reads.
+    // or none of them: no memory.
     unsigned char *block = nullptr;
-    float4 *quad = nullptr;
     float2 *cell = nullptr;           // with a texture
+    float4 *quad = nullptr;           // without
     unsigned char *d0 = nullptr, *d1 = nullptr;  // distances, and the passes' other buffer
     unsigned char *flag = nullptr;    // work: flat flags (zero-padded rows)
-    unsigned int *odd = nullptr;      // RayCells::odd, and the count of cells not flat
     int nx = 0, ny = 0, nz = 0;
 };
 
@@ -1616,16 +1550,13 @@ static PbStatus texture_fill(RlspTexture *t, const float *rlsp, cudaStream_t st)
         if (s != PB_OK) return s;
     }
     const PbGrid g{t->nx, t->ny, t->nz, 1.0f};
-    if (!t->quad) return PB_OK;
+    if (!t->block) return PB_OK;
     const int64_t words = cell_row(t->nx) / 4, cy = t->ny + 1, cz = t->nz + 1;
     auto blocks = [](int64_t threads, int block) { return (unsigned)((threads + block - 1) / block); };
     auto runs = [](int64_t n) { return (n + kDistRun - 1) / kDistRun; };
     const dim3 cols((unsigned)(((t->nx + 1) * (int64_t)(t->nz + 1) + 255) / 256),
                     (unsigned)((t->ny + 2 + kFlatRows - 1) / kFlatRows));
-    const PbStatus z = check_cuda(cudaMemsetAsync(t->odd, 0, 2 * sizeof(*t->odd), st),
-                                  "cudaMemsetAsync");
-    if (z != PB_OK) return z;
-    k_cell_flat<<<cols, 256, 0, st>>>(rlsp, g, t->quad, t->flag, t->odd);
+    k_cell_flat<<<cols, 256, 0, st>>>(rlsp, g, t->quad, t->flag);
     k_cell_dist_x<<<blocks(words * cy * cz, 256), 256, 0, st>>>(
         g, t->flag, reinterpret_cast<unsigned int *>(t->d0));
     k_cell_dist4<1><<<blocks(words * cz * runs(cy), 128), 128, 0, st>>>(
@@ -1633,7 +1564,7 @@ static PbStatus texture_fill(RlspTexture *t, const float *rlsp, cudaStream_t st)
         reinterpret_cast<unsigned int *>(t->d1));
     k_cell_dist4<2><<<blocks(words * cy * runs(cz), 128), 128, 0, st>>>(
         g, reinterpret_cast<const unsigned int *>(t->d1),
-        reinterpret_cast<unsigned int *>(t->d0), rlsp, t->odd, t->cell);
+        reinterpret_cast<unsigned int *>(t->d0), rlsp, t->cell);
     return check_launch("cell records");
 }
 
@@ -1675,20 +1606,18 @@ PbStatus texture_create(const float *rlsp, const PbGrid &g, uint64_t *out, cudaS
         bytes += (n + 255) / 256 * 256;
         return at;
     };
-    static_assert(sizeof(float2) <= sizeof(float4), "the cells fit where the quads are");
-    const size_t at_quad = part(sizeof(float4) * nquad), at_d0 = part(npad), at_d1 = part(npad);
-    const size_t at_flag = part(nflag), at_odd = part(2 * sizeof(unsigned int));
+    const size_t at_cells = part(with_texture ? sizeof(float2) * ncell : sizeof(float4) * nquad);
+    const size_t at_d0 = part(npad), at_d1 = part(npad), at_flag = part(nflag);
     if (s == PB_OK && cudaMalloc(&t->block, bytes) != cudaSuccess) {
         t->block = nullptr;
         cudaGetLastError();
     }
     if (s == PB_OK && t->block) {
-        t->quad = reinterpret_cast<float4 *>(t->block + at_quad);
-        if (with_texture) t->cell = reinterpret_cast<float2 *>(t->block + at_quad);
+        if (with_texture) t->cell = reinterpret_cast<float2 *>(t->block + at_cells);
+        else t->quad = reinterpret_cast<float4 *>(t->block + at_cells);
         t->d0 = t->block + at_d0;
         t->d1 = t->block + at_d1;
         t->flag = t->block + at_flag;
-        t->odd = reinterpret_cast<unsigned int *>(t->block + at_odd);
         // flat flags: the padding bytes stay zero, the cells are rewritten by
         // every fill
         s = check_cuda(cudaMemsetAsync(t->flag, 0, nflag, st), "cudaMemsetAsync");
@@ -1738,7 +1667,7 @@ cudaTextureObject_t texture_object(uint64_t h)
 RayCells texture_cells(uint64_t h)
 {
     const RlspTexture *t = reinterpret_cast<const RlspTexture *>(h);
-    return t && t->quad ? RayCells{t->quad, t->d0, t->odd, t->cell} : RayCells{};
+    return t && t->block ? RayCells{t->quad, t->d0, t->cell} : RayCells{};
 }
 
 void texture_destroy(uint64_t h)

@@ -144,30 +144,30 @@ PbStatus pb_rlsp_from_hu(const float *hu_dev, int64_t n, const double *curve_hu,
  * unit's filter weights are fixed point, so samples through it differ
  * slightly from exact trilinear interpolation; the reference's WET is
  * defined by them.  Creating one allocates a CUDA array.  The handle also
- * holds per-cell records (the texels of each 2x2x2 block, and how far the
- * nearest block is whose texels differ) from which pb_wet adds whole runs of
- * samples through flat regions at once and forms the other samples with the
- * unit's filter (pb_texture_sample compares the two).  They take 19 bytes per
+ * holds per-cell records (the value of each 2x2x2 block of equal texels, and
+ * how far the nearest block is whose texels differ) from which pb_wet adds
+ * whole runs of samples through flat regions at once.  They take 11 bytes per
  * voxel, in one allocation; a grid that leaves no memory for it is sampled
- * through the unit alone, and one with more than 8191 voxels along an axis takes
- * its runs from them and its samples through the unit. */
+ * through the unit alone. */
 typedef uint64_t PbTexture;
 
 PbStatus pb_texture_create(const float *rlsp_dev, const PbGrid *grid,
                            PbTexture *tex_out, void *stream);
 /* A handle with the cell records only (no texture, no CUDA array), for
  * exact-trilinear WET with the same runs through flat regions and its
- * samples from the records.  No counterpart in the reference. */
+ * samples from records of each block's texels (19 bytes per voxel).  No
+ * counterpart in the reference. */
 PbStatus pb_cells_create(const float *rlsp_dev, const PbGrid *grid, PbTexture *cells_out,
                          void *stream);
 /* Refill an existing handle (either kind) from a volume of the same grid. */
 PbStatus pb_texture_update(PbTexture tex, const float *rlsp_dev, void *stream);
 PbStatus pb_texture_destroy(PbTexture tex);
-/* Check of the cell records' filter against the texture unit: samples at
- * 2 x pairs coordinates (x, y, z each, unnormalised), through the unit into
- * unit_dev and from the records, as pb_wet takes them, into cells_dev; 0
- * where a coordinate is nearer than 0.003 to the grid's faces or outside.
- * Synchronous; it allocates the records anew for the length of the call.
+/* The texture unit's filter as fixed point and FP32 against the unit: samples
+ * at 2 x pairs coordinates (x, y, z each, unnormalised), through the unit into
+ * unit_dev and by that filter from the blocks' texels into cells_dev, equal to
+ * FP32 rounding; 0 where a coordinate is nearer than 0.003 to the grid's faces
+ * or outside.  A handle with records, axes of at most 8191 voxels.
+ * Synchronous; it allocates the texels' records for the length of the call.
  * No counterpart in the reference. */
 PbStatus pb_texture_sample(PbTexture tex, const PbGrid *grid, const float *at_dev, int64_t pairs,
                            float *unit_dev, float *cells_dev, void *stream);

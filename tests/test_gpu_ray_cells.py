@@ -273,3 +273,21 @@ def test_axis_past_the_filters_fixed_point(noise):
     assert top > 0.5
     assert float((raw - exact).abs().max()) <= 1e-6 * top
     assert float((tex - exact).abs().max()) <= 3.0 / 512.0 * float(rho.max()) / 0.2 * top
+
+
+@pytest.mark.parametrize("shape", [(40, 30, 33), (160, 90, 70)])
+@pytest.mark.parametrize("angle,spacing", [(0.0, 2.5), (37.0, 3.0)])
+def test_sparse_and_dense_depths_are_the_same_bits(shape, angle, spacing):
+    """As test_sparse_and_dense_volumes_agree: every sample is the unit's and the
+    sums go the same way, so the depths are the same bits, smoothed ones too (a
+    depth off by a rounding can decide a radius of the smoothing otherwise)."""
+    nz = shape[0]
+    near = int(0.8 * nz)
+    dp = _texture_plan(shape, spacing, angle)
+    first = slice(0, near // 2)
+    out = []
+    for planes in (near, nz):
+        raw = _raw(dp, _half_noisy(shape, planes))
+        out.append((raw[first], dp.wet.clone().reshape(shape)[first]))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1][:near // 2 - 12], out[1][1][:near // 2 - 12])
