@@ -882,13 +882,26 @@ struct SmoothBox {
     long long inner, shell;        // blocks
 };
 
+// Largest volume with inner blocks: the index of their last thread's last voxel,
+// past the volume's end in the last block, still is an int.  Larger volumes are all shell.
+constexpr long long smooth_inner_max(int per) { return 0x7fffffffll - 128 * per; }
+constexpr long long smooth_last_index(long long V, int per)
+{
+    return (V + 128 * per - 1) / (128 * per) * (128 * per) - 1;
+}
+static_assert(smooth_last_index(smooth_inner_max(2), 2) <= 0x7fffffffll &&
+              smooth_last_index(smooth_inner_max(2) - 255, 2) <= 0x7fffffffll &&
+              smooth_last_index(smooth_inner_max(4), 4) <= 0x7fffffffll &&
+              smooth_last_index(smooth_inner_max(4) - 511, 4) <= 0x7fffffffll,
+              "a voxel index of the smoothing's inner blocks passes INT32_MAX");
+
 template <int PER>
 __host__ __device__ __forceinline__ SmoothBox smooth_box(const PbGrid &g, const int *margin)
 {
     SmoothBox X;
     const long long V = (long long)g.nx * g.ny * g.nz;
     const bool some = 2 * margin[0] < g.nx && 2 * margin[1] < g.ny && 2 * margin[2] < g.nz &&
-                      V < (1ll << 31);
+                      V <= smooth_inner_max(PER);
     X.mx = margin[0];
     X.my = margin[1];
     // nothing inside: the shell's end planes are the whole volume
