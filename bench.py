@@ -67,7 +67,7 @@ L2_NOTE = "flushed (256 MiB write) between timed iterations"
 # profiles/pencil_beam_kernels_heterogeneous_256x256x160_4beams.md.  Reported only
 # for that workload ("wet": the cell passes, k_raytrace and k_smooth).
 NCU_TRAFFIC = {"k_dose_line": 204_658_432, "k_adjoint_line": 126_976_000,
-               "wet": 825_198_592}
+               "wet": 703_095_552}
 NCU_TRAFFIC_WORKLOAD = {"seed": 3, "wet_mode": "texture"}
 
 
